@@ -1,11 +1,9 @@
 """Build recipe of libluxgpu_backend_cuda.so (sm_100a only, in-tree).
 
-The plugin is compiled against the reference's UNCHANGED ABI header
-(include/lux/gpu/backend_plugin.h), taken where it lies in the reference tree
-(``LUX_REFERENCE_INCLUDE`` or ``LUX_REFERENCE_ROOT``, else a directory ``reference`` beside this repository or
-beside one of the directories above it); the header is not
-copied into this repository.  On a machine without the reference tree the
-prebuilt library is used as is.
+The plugin is compiled against the UNCHANGED ABI header of the Lux GPU core (include/lux/gpu/backend_plugin.h)
+where a tree of the core is found (``LUX_REFERENCE_INCLUDE`` or ``LUX_REFERENCE_ROOT``, else a directory
+``reference`` beside this repository or beside one of the directories above it), and against this repository's own
+declaration of the same layout (include/lux/gpu/) otherwise.
 """
 import os
 import subprocess
@@ -61,14 +59,7 @@ def _newer(target, deps):
 
 
 def build(verbose=False, force=False, ptxas_info=False):
-    ref_inc = reference_include()
-    if ref_inc is None:
-        if os.path.exists(LIB_PATH):
-            if verbose:
-                print(f"reference headers not present; using prebuilt {LIB_PATH}")
-            return LIB_PATH
-        raise RuntimeError("cannot build the plugin: reference ABI header (lux/gpu/backend_plugin.h) not found "
-                           "and no prebuilt library present")
+    ref_inc = reference_include() or os.path.join(ROOT, "include")
     os.makedirs(OBJ_DIR, exist_ok=True)
     headers = [os.path.join(CSRC, f) for f in os.listdir(CSRC) if f.endswith((".h", ".cuh"))] + \
               [os.path.join(ROOT, "include", "lux_cuda_quant.h"), os.path.join(ref_inc, "lux", "gpu", "backend_plugin.h")]
