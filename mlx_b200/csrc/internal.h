@@ -3,6 +3,7 @@
 // kernels.  Nothing here crosses the C ABI.
 #pragma once
 
+#include <cuda.h>
 #include <cuda_runtime.h>
 
 #include <atomic>
@@ -219,6 +220,10 @@ struct ShardPush {
 
 // decode GEMV, bf16 activations: mma.sync m16n8k16 with in-register dequant
 bool qmv_mma_supported(const QmmArgs& a, int sm_count);
+// the same without K split or peers, any K (a multiple of the group): weights through bulk copies (qmv_stream.cu);
+// n items of one shape and one side of M = 8 in one launch
+bool qmv_stream_supported(const QmmArgs& a, int sm_count);
+cudaError_t launch_qmv_stream(const QmmArgs* items, int n, int sm_count, cudaStream_t stream, bool overlap_prev, bool x_stable);
 size_t qmv_mma_workspace_bytes(const QmmArgs& a, int sm_count);
 // overlap_prev: launch as a programmatic dependent of the previous kernel in the stream (see Context);
 // x_stable: that previous kernel does not write x, which may then be read before the wait for it
@@ -237,6 +242,11 @@ int qmv_batch_max();
 // delivers its columns to the same place of every peer's
 cudaError_t launch_qmv_batch(const QmmArgs* items, int n, int sm_count, cudaStream_t stream, const char** name,
                              const ShardPush* push = nullptr);
+// cuTensorMapEncodeTiled of the driver (null if it has none)
+using EncodeTiledFn = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,
+                                   const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
+                                   CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+EncodeTiledFn encode_tiled_fn();
 // prefill GEMM, bf16 activations: TMA + tcgen05 + TMEM
 bool qmm_tc_supported(const QmmArgs& a, int sm_count);
 size_t qmm_tc_workspace_bytes(int sm_count);  // scratch of a launch (flags at its head: zero between launches)

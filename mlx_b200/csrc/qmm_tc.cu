@@ -1384,9 +1384,7 @@ qmm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_cons
 }
 
 // ---- host side -------------------------------------------------------------------
-using EncodeTiledFn = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
-                                   const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
-                                   CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+}  // namespace
 
 EncodeTiledFn encode_tiled_fn() {
     static EncodeTiledFn fn = [] {
@@ -1399,6 +1397,8 @@ EncodeTiledFn encode_tiled_fn() {
     }();
     return fn;
 }
+
+namespace {
 
 int* g_error_host = nullptr;  // pinned + mapped: written by kernels that give up on a wait, read by the host
 std::once_flag g_error_once;

@@ -1,4 +1,5 @@
-// Decode-regime quantized GEMV for bf16 activations, M <= 16:
+// Decode-regime quantized GEMV for bf16 activations, M <= 16, for launches whose K is split over CTAs (few rows of W)
+// and for column-sharded layers (the rest: qmv_stream.cu):
 //   y[M,N] = x[M,K] . dequant(Wq[N,K])^T,  w^ = RNE_bf16(s*q + b)  (one bf16 FMA)
 //
 // HBM-bound: every packed weight word, scale and bias is read from HBM exactly
@@ -17,14 +18,9 @@
 //     tasks ahead of the one being computed (2.5 KiB each) are in flight, with no
 //     registers tied up and no block-wide barrier in the streaming loop;
 //   * lane (g = lane/4, t = lane%4) copies and later reads back exactly its own
-//     pieces: rows g and g+8, the 16-byte pieces t and t+4 of the 128-byte
-//     k-block row (so each quad copies 64 contiguous bytes per instruction);
-//   * weights are dequantised in registers (dequant.cuh) and fed to
-//     mma.sync.m16n8k16 (bf16 x bf16 -> fp32): the <= 16 rows of x cost no
-//     extra instruction per weight.  The dot product is invariant under a
-//     permutation of k applied to both operands, so the weights are used in
-//     the order the mask/shift unpack yields them and the x fragments of the
-//     warp's k-block are loaded once, in that order, into registers;
+//     pieces: bytes [32t, 32t+32) of rows g and g+8 of the k-block;
+//   * weights are dequantised in registers and multiplied with mma.sync (qmv_frag.cuh);
+//     the x fragments of the warp's k-block are loaded once, into registers;
 //   * every task leaves a 16 x 8*MT fp32 partial in shared memory; at the end
 //     of a batch of tiles the partials of a tile are summed in k-block order
 //     (fixed order => the result does not depend on N, on the grid or on how
@@ -33,12 +29,10 @@
 //     per tile range: each exports its partials to a global scratch slot and
 //     bumps the tile's arrival counter; the last arriver sums all of them,
 //     again in k-block order, and resets the counter.  Nobody waits.
-#include <cuda_bf16.h>
-
 #include <algorithm>
 
-#include "dequant.cuh"
 #include "internal.h"
+#include "qmv_frag.cuh"
 
 namespace luxcuda {
 
@@ -67,14 +61,6 @@ __device__ __forceinline__ void cp_async4(uint32_t dst, const void* src) {
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;"); }
 template <int N>
 __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
-
-__device__ __forceinline__ void mma_bf16(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0,
-                                         uint32_t b1) {
-    asm volatile(
-        "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
-        : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
-        : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
-}
 
 struct Params {
     const __nv_bfloat16* x;
@@ -323,172 +309,7 @@ __device__ __noinline__ void batch_end(const Params& p, const float* part, int f
     if (more) __syncthreads();  // the partial buffer and the flags are reused by the next batch
 }
 
-// With 16 rows of x the fragments of rows 8..15 live in shared memory (one conflict-free 16-byte read per
-// use) instead of 32 more registers per lane: at the 128-register limit the kernel otherwise spills.
-constexpr bool kX1Shared = true;
-
-// One task out of the warp's ring stage: 4 x 16 bytes of packed weights per
-// lane (rows g, g+8; pieces t, t+4), their scales/biases, times the x fragments.
-// stage layout: [piece = r*2+h][lane] 16 B  |  [row 0..15 scales][row 0..15 biases] 16 B each
-template <int BITS, int MT, bool FAST>
-__device__ __forceinline__ void task_mma(const uint4 (&w)[2][2], const uint32_t (&s)[2][2], const uint32_t (&b)[2][2],
-                                         const uint4 (&xr)[MT][BITS == 4 ? 8 : 4], const uint4* xs, float (&acc)[MT][2][4]) {
-#pragma unroll
-    for (int h = 0; h < 2; h++) {
-        uint32_t sa[2], sb[2], b2[2];
-#pragma unroll
-        for (int r = 0; r < 2; r++) {
-            b2[r] = dup_bf16(b[r][h]);
-            sa[r] = FAST ? scale_x2_133(s[r][h]) : dup_bf16(s[r][h]);
-            sb[r] = FAST ? scale_x2_129(s[r][h]) : 0u;
-        }
-        const uint32_t w0[4] = {w[0][h].x, w[0][h].y, w[0][h].z, w[0][h].w};
-        const uint32_t w1[4] = {w[1][h].x, w[1][h].y, w[1][h].z, w[1][h].w};
-        if (BITS == 4) {
-#pragma unroll
-            for (int i = 0; i < 4; i++) {
-                uint32_t lo[4], hi[4];
-                if (FAST) {
-                    dequant4_fast(w0[i], sa[0], sb[0], b2[0], lo);
-                    dequant4_fast(w1[i], sa[1], sb[1], b2[1], hi);
-                } else {
-                    dequant4_general(w0[i], sa[0], b2[0], lo);
-                    dequant4_general(w1[i], sa[1], b2[1], hi);
-                }
-#pragma unroll
-                for (int mt = 0; mt < MT; mt++) {
-                    const uint4 bx = (mt == 0 || !kX1Shared) ? xr[mt][h * 4 + i] : xs[(h * 4 + i) * 32];
-                    mma_bf16(acc[mt][0], lo[0], hi[0], lo[1], hi[1], bx.x, bx.y);
-                    mma_bf16(acc[mt][1], lo[2], hi[2], lo[3], hi[3], bx.z, bx.w);
-                }
-            }
-        } else {
-#pragma unroll
-            for (int i = 0; i < 2; i++) {
-                uint32_t lo0[2], hi0[2], lo1[2], hi1[2];
-                if (FAST) {
-                    dequant8_fast(w0[2 * i], sa[0], b2[0], lo0);
-                    dequant8_fast(w1[2 * i], sa[1], b2[1], hi0);
-                    dequant8_fast(w0[2 * i + 1], sa[0], b2[0], lo1);
-                    dequant8_fast(w1[2 * i + 1], sa[1], b2[1], hi1);
-                } else {
-                    dequant8_general(w0[2 * i], sa[0], b2[0], lo0);
-                    dequant8_general(w1[2 * i], sa[1], b2[1], hi0);
-                    dequant8_general(w0[2 * i + 1], sa[0], b2[0], lo1);
-                    dequant8_general(w1[2 * i + 1], sa[1], b2[1], hi1);
-                }
-#pragma unroll
-                for (int mt = 0; mt < MT; mt++) {
-                    const uint4 bx = (mt == 0 || !kX1Shared) ? xr[mt][h * 2 + i] : xs[(h * 2 + i) * 32];
-                    mma_bf16(acc[mt][0], lo0[0], hi0[0], lo0[1], hi0[1], bx.x, bx.y);
-                    mma_bf16(acc[mt][1], lo1[0], hi1[0], lo1[1], hi1[1], bx.z, bx.w);
-                }
-            }
-        }
-    }
-}
-
-// x fragments of k-block kb for lane (g, t), in the order the unpack yields the weights.
-//   4-bit: fragment j = h*4+i covers k = kb*256 + h*128 + t*32 + i*8 + (0,4,1,5 | 2,6,3,7)
-//   8-bit: fragment j = h*2+i covers k = kb*128 + h*64  + t*16 + i*8 + (0,2,1,3 | 4,6,5,7)
-// PRO: what x is -- 0: the buffer as it is; 1: its rms-norm, row by row (the caller scales the fragments, see
-// rms_scale); 2: bf16(a + b + c) of the three column blocks [0,K), [K,2K), [2K,3K) of a wider row (fp32 adds,
-// left to right, one rounding: the bits of the stand-alone sum3 kernel).
-__device__ __forceinline__ uint32_t add3_bf16x2(uint32_t a, uint32_t b, uint32_t c) {
-    const float lo = __fadd_rn(__fadd_rn(__uint_as_float(a << 16), __uint_as_float(b << 16)), __uint_as_float(c << 16));
-    const float hi = __fadd_rn(__fadd_rn(__uint_as_float(a & 0xFFFF0000u), __uint_as_float(b & 0xFFFF0000u)), __uint_as_float(c & 0xFFFF0000u));
-    const __nv_bfloat162 r = __floats2bfloat162_rn(lo, hi);
-    return *reinterpret_cast<const uint32_t*>(&r);
-}
-__device__ __forceinline__ uint4 ldg_nc_v4(const uint4* src) {
-    uint4 v;
-    asm volatile("ld.global.nc.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(src));
-    return v;
-}
-template <int BITS, int MT, int PRO>
-__device__ __forceinline__ void load_x_raw(const Params& p, int kb, int g, int t, uint4 (&xr)[MT][BITS == 4 ? 8 : 4]) {
-    constexpr int XV = BITS == 4 ? 8 : 4;
-    constexpr int KB = 1024 / BITS;
-#pragma unroll
-    for (int mt = 0; mt < MT; mt++) {
-        const int m = mt * 8 + g;
-        const __nv_bfloat16* row = p.x + (size_t)m * (PRO == 0 ? p.K : p.x_ld) + kb * KB + t * (KB / 8);
-#pragma unroll
-        for (int j = 0; j < XV; j++) {
-            const int h = j / (XV / 2), i = j % (XV / 2);
-            xr[mt][j] = make_uint4(0, 0, 0, 0);
-            if (m < p.M) {
-                const uint4* src = reinterpret_cast<const uint4*>(row + h * (KB / 2) + i * 8);
-                if (PRO == 2) {
-                    const uint4 a = ldg_nc_v4(src), b = ldg_nc_v4(reinterpret_cast<const uint4*>(row + p.K + h * (KB / 2) + i * 8)),
-                                c = ldg_nc_v4(reinterpret_cast<const uint4*>(row + 2 * p.K + h * (KB / 2) + i * 8));
-                    xr[mt][j] = make_uint4(add3_bf16x2(a.x, b.x, c.x), add3_bf16x2(a.y, b.y, c.y), add3_bf16x2(a.z, b.z, c.z),
-                                           add3_bf16x2(a.w, b.w, c.w));
-                } else {
-                    xr[mt][j] = ldg_nc_v4(src);
-                }
-            }
-        }
-    }
-}
-// rms-norm prologue: the sum of squares of this lane's fragments (fp32), and the fragments scaled and rounded
-// as the stand-alone rms-norm kernel does it: bf16(fl32(x * inv)).
-template <int XV>
-__device__ __forceinline__ float sumsq_frags(const uint4 (&xr)[XV]) {
-    float ss = 0.0f;
-#pragma unroll
-    for (int j = 0; j < XV; j++) {
-        const uint32_t w[4] = {xr[j].x, xr[j].y, xr[j].z, xr[j].w};
-#pragma unroll
-        for (int e = 0; e < 4; e++) {
-            const float lo = __uint_as_float(w[e] << 16), hi = __uint_as_float(w[e] & 0xFFFF0000u);
-            ss = fmaf(lo, lo, ss);
-            ss = fmaf(hi, hi, ss);
-        }
-    }
-    return ss;
-}
-__device__ __forceinline__ uint32_t scale_bf16x2(uint32_t v, float inv) {
-    const __nv_bfloat162 r = __floats2bfloat162_rn(__fmul_rn(__uint_as_float(v << 16), inv), __fmul_rn(__uint_as_float(v & 0xFFFF0000u), inv));
-    return *reinterpret_cast<const uint32_t*>(&r);
-}
-template <int XV>
-__device__ __forceinline__ void rms_scale(uint4 (&xr)[XV], float inv) {
-#pragma unroll
-    for (int j = 0; j < XV; j++)
-        xr[j] = make_uint4(scale_bf16x2(xr[j].x, inv), scale_bf16x2(xr[j].y, inv), scale_bf16x2(xr[j].z, inv), scale_bf16x2(xr[j].w, inv));
-}
-template <int BITS, int MT>
-__device__ __forceinline__ void permute_x(uint4 (&xr)[MT][BITS == 4 ? 8 : 4]) {
-    constexpr int XV = BITS == 4 ? 8 : 4;
-#pragma unroll
-    for (int mt = 0; mt < MT; mt++)
-#pragma unroll
-        for (int j = 0; j < XV; j++) {
-            const uint4 v = xr[mt][j];
-            if (BITS == 4) {
-                xr[mt][j].x = prmt(v.x, v.z, 0x5410u);  // x0, x4
-                xr[mt][j].y = prmt(v.x, v.z, 0x7632u);  // x1, x5
-                xr[mt][j].z = prmt(v.y, v.w, 0x5410u);  // x2, x6
-                xr[mt][j].w = prmt(v.y, v.w, 0x7632u);  // x3, x7
-            } else {
-                xr[mt][j].x = prmt(v.x, v.y, 0x5410u);  // x0, x2
-                xr[mt][j].y = prmt(v.x, v.y, 0x7632u);  // x1, x3
-                xr[mt][j].z = prmt(v.z, v.w, 0x5410u);  // x4, x6
-                xr[mt][j].w = prmt(v.z, v.w, 0x7632u);  // x5, x7
-            }
-        }
-}
-
-// all four scales (raw bf16 bits) usable by the exponent-trick dequantiser?  Packed form of
-// scale_fast_ok: exponent field e in [1, 121]  <=>  ((s - 0x80) & 0x7F80) <= 0x3C00 per half.
-__device__ __forceinline__ bool scales_fast_ok4(uint32_t s00, uint32_t s01, uint32_t s10, uint32_t s11) {
-    const uint32_t a = (((s00 | (s10 << 16)) - 0x00800080u) & 0x7F807F80u) + 0x43804380u;
-    const uint32_t b = (((s01 | (s11 << 16)) - 0x00800080u) & 0x7F807F80u) + 0x43804380u;
-    return ((a | b) & 0x80008000u) == 0u;
-}
-
-// BITS: 4 | 8.  MT: number of 8-row blocks of x (M <= 8*MT).  PRO: prologue applied to x as it is loaded (load_x_raw;
+// BITS: 4 | 8.  MT: number of 8-row blocks of x (M <= 8*MT).  PRO: prologue applied to x as it is loaded (load_x_row;
 // MT == 1 only).
 template <int BITS, int MT, int PRO>
 __global__ void __launch_bounds__(kThreads, 1) qmv_mma_kernel(const __grid_constant__ Params p) {
@@ -503,6 +324,7 @@ __global__ void __launch_bounds__(kThreads, 1) qmv_mma_kernel(const __grid_const
     uint4* xs = reinterpret_cast<uint4*>(smem + p.xs_off) + (threadIdx.x >> 5) * (XV * 32) + (threadIdx.x & 31);
     __shared__ int s_flags[kMaxTb];
 
+    constexpr int KL = lane_weights(BITS), SPL = BITS == 4 ? 2 : 1;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int g = lane >> 2, t = lane & 3;
     const int ci = blockIdx.x % p.chunks, ksi = blockIdx.x / p.chunks;
@@ -513,7 +335,7 @@ __global__ void __launch_bounds__(kThreads, 1) qmv_mma_kernel(const __grid_const
     const size_t row_bytes = (size_t)p.K * BITS / 8;
     const int gpr = p.K >> p.gshift;   // groups per row
     const int gpk = KB >> p.gshift;    // groups per k-block
-    const unsigned char* wbase = reinterpret_cast<const unsigned char*>(p.wq) + t * 16;
+    const unsigned char* wbase = reinterpret_cast<const unsigned char*>(p.wq) + t * 32;
     const __nv_bfloat16* sb_src = lane < 16 ? p.scales : p.biases;
     const uint32_t ring_lo = smem_u32(smem) + warp * (D * kStageBytes) + lane * 16;  // this lane's slot, stage 0
     const int tail_tile = (p.N & 15) ? p.n_rt - 1 : -1;  // the tile whose rows must be clamped to N-1
@@ -525,7 +347,7 @@ __global__ void __launch_bounds__(kThreads, 1) qmv_mma_kernel(const __grid_const
     const size_t half_tile = 8 * row_bytes, tile_stride = 16 * row_bytes;
     int f_b0 = rt_lo, f_kb = kb_lo + warp, f_rt = rt_lo;  // the task fetched next
     uint32_t f_dst = ring_lo;                             // and the stage it goes to
-    // this lane's sources of that task: rows g and g+8 of the tile (its 16-byte pieces t and t+4 of the k-block),
+    // this lane's sources of that task: rows g and g+8 of the tile (its 32 bytes of the k-block),
     // the scales (lanes 0-15) or biases (16-31) of row lane%16.  Inside a run they move by constant strides.
     const unsigned char* f_p0 = nullptr;
     const unsigned char* f_p1 = nullptr;
@@ -546,9 +368,9 @@ __global__ void __launch_bounds__(kThreads, 1) qmv_mma_kernel(const __grid_const
     auto fetch_next = [&]() {
         if (has_work && f_b0 < rt_hi) {
             cp_async16(f_dst, f_p0);
-            cp_async16(f_dst + 512, f_p0 + 64);
+            cp_async16(f_dst + 512, f_p0 + 16);
             cp_async16(f_dst + 1024, f_p1);
-            cp_async16(f_dst + 1536, f_p1 + 64);
+            cp_async16(f_dst + 1536, f_p1 + 16);
             if (p.sb_bytes == 16) cp_async16(f_dst + 2048, f_sb);
             else if (p.sb_bytes == 8) cp_async8(f_dst + 2048, f_sb);
             else cp_async4(f_dst + 2048, reinterpret_cast<const void*>(reinterpret_cast<uintptr_t>(f_sb) & ~uintptr_t(3)));  // a lone scale travels with its neighbour
@@ -580,7 +402,14 @@ __global__ void __launch_bounds__(kThreads, 1) qmv_mma_kernel(const __grid_const
     // fetch code and spill; they stay behind it.)
     constexpr bool kXFirst = MT == 1;
     uint4 xr[MT][XV];
-    if (kXFirst && p.x_early && has_work) load_x_raw<BITS, MT, PRO>(p, kb_lo + warp, g, t, xr);
+    auto load_x = [&](int kb) {
+#pragma unroll
+        for (int mt = 0; mt < MT; mt++) {
+            const int m = mt * 8 + g;
+            load_x_row<BITS, PRO>(m < p.M ? p.x + (size_t)m * (PRO == 0 ? p.K : p.x_ld) : nullptr, p.K, kb, t, xr[mt]);
+        }
+    };
+    if (kXFirst && p.x_early && has_work) load_x(kb_lo + warp);
 #pragma unroll
     for (int i = 0; i < D - 1; i++) fetch_next();
 
@@ -599,7 +428,7 @@ __global__ void __launch_bounds__(kThreads, 1) qmv_mma_kernel(const __grid_const
         // (a relaxed store: it publishes no data of this kernel, only that the kernel has started)
         if (blockIdx.x == 0 && tid < p.sp.world && tid != p.sp.me) st_relaxed_sys(p.sp.flags[tid] + kFlagReady + p.sp.me, epoch);
     }
-    if (kXFirst && !p.x_early && has_work) load_x_raw<BITS, MT, PRO>(p, kb_lo + warp, g, t, xr);
+    if (kXFirst && !p.x_early && has_work) load_x(kb_lo + warp);
     bool x_loaded = kXFirst;  // (of the first run)
     // rms-norm prologue.  The host launches it only when every warp has at most one k-block and K is not split:
     // the fragments just loaded by the 16 warps are then the whole of x, each lane holding 1/4 of a k-block of
@@ -625,7 +454,7 @@ __global__ void __launch_bounds__(kThreads, 1) qmv_mma_kernel(const __grid_const
     }
 
     uint32_t src_c = ring_lo;  // stage of the task computed next (this lane's slot)
-    uint32_t sboff[2][2];      // byte offsets of this lane's scales inside a stage, by row half r and piece h
+    uint32_t sboff[2][SPL];    // byte offsets of this lane's scales inside a stage, by row half r
 #pragma unroll 1
     for (int b0 = rt_lo; b0 < rt_hi; b0 += tb) {
         const int nt = min(tb, rt_hi - b0);
@@ -634,12 +463,12 @@ __global__ void __launch_bounds__(kThreads, 1) qmv_mma_kernel(const __grid_const
             for (int kb = kb_lo + warp; kb < kb_hi; kb += kWarps) {
                 fetch_next();  // (the run's first fetch goes out ahead of the x loads)
                 if (!x_loaded) {
-                    load_x_raw<BITS, MT, PRO>(p, kb, g, t, xr);
+                    load_x(kb);
                     if (PRO == 1) rms_scale<XV>(xr[0], rms_inv);
                 }
                 x_loaded = false;
-                permute_x<BITS, MT>(xr);
-                if (MT == 2 && kX1Shared) {
+                for (int mt = 0; mt < MT; mt++) permute_x<BITS>(xr[mt]);
+                if (MT == 2) {
                     __syncwarp();  // (the previous run's reads of xs)
 #pragma unroll
                     for (int j = 0; j < XV; j++) xs[j * 32] = xr[MT - 1][j];
@@ -650,8 +479,8 @@ __global__ void __launch_bounds__(kThreads, 1) qmv_mma_kernel(const __grid_const
                     const int slot = g + 8 * r;
                     const int par = p.sb_bytes == 2 ? ((slot * gpr + kb) & 1) : 0;
 #pragma unroll
-                    for (int h = 0; h < 2; h++)
-                        sboff[r][h] = 2048 - lane * 16 + slot * 16 + ((((h * (KB / 2) + t * (KB / 8)) >> p.gshift) + par) << 1);
+                    for (int i = 0; i < SPL; i++)
+                        sboff[r][i] = 2048 - lane * 16 + slot * 16 + ((((t * KL + i * 32) >> p.gshift) + par) << 1);
                 }
                 if (p.sp.world > 1 && tid < p.sp.world && tid != p.sp.me)
                     ready_early = ld_relaxed_sys(p.sp.flags[p.sp.me] + kFlagReady + tid);  // used at the first push
@@ -661,30 +490,27 @@ __global__ void __launch_bounds__(kThreads, 1) qmv_mma_kernel(const __grid_const
                     if (rt != b0) fetch_next();
                     cp_async_wait<D - 1>();
                     __syncwarp();
-                    uint4 w[2][2];
-                    uint32_t s[2][2], b[2][2];
+                    uint32_t w[2][8];
+                    uint32_t s[2][SPL], b[2][SPL];
 #pragma unroll
-                    for (int r = 0; r < 2; r++)
+                    for (int r = 0; r < 2; r++) {
 #pragma unroll
-                        for (int h = 0; h < 2; h++) {
+                        for (int h = 0; h < 2; h++)
                             asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];"
-                                         : "=r"(w[r][h].x), "=r"(w[r][h].y), "=r"(w[r][h].z), "=r"(w[r][h].w)
+                                         : "=r"(w[r][4 * h]), "=r"(w[r][4 * h + 1]), "=r"(w[r][4 * h + 2]), "=r"(w[r][4 * h + 3])
                                          : "r"(src_c + (r * 2 + h) * 512));
-                            asm volatile("ld.shared.u16 %0, [%1];" : "=r"(s[r][h]) : "r"(src_c + sboff[r][h]));
-                            asm volatile("ld.shared.u16 %0, [%1+256];" : "=r"(b[r][h]) : "r"(src_c + sboff[r][h]));
+#pragma unroll
+                        for (int i = 0; i < SPL; i++) {
+                            asm volatile("ld.shared.u16 %0, [%1];" : "=r"(s[r][i]) : "r"(src_c + sboff[r][i]));
+                            asm volatile("ld.shared.u16 %0, [%1+%2];" : "=r"(b[r][i]) : "r"(src_c + sboff[r][i]), "n"(256));
                         }
-                    const bool fast = scales_fast_ok4(s[0][0], s[0][1], s[1][0], s[1][1]);
-                    float acc[MT][2][4];  // two independent accumulation chains per 8-row block of x
+                    }
+                    float4 out[MT];
+                    auto x_hi = [&](int j) { return xs[j * 32]; };
+                    if (__all_sync(0xffffffffu, scales_fast_ok<SPL>(s))) task_mma<BITS, MT, SPL, true>(w, s, b, xr[0], x_hi, out);
+                    else task_mma<BITS, MT, SPL, false>(w, s, b, xr[0], x_hi, out);
 #pragma unroll
-                    for (int mt = 0; mt < MT; mt++)
-#pragma unroll
-                        for (int c = 0; c < 2; c++) acc[mt][c][0] = acc[mt][c][1] = acc[mt][c][2] = acc[mt][c][3] = 0.0f;
-                    if (__all_sync(0xffffffffu, fast)) task_mma<BITS, MT, true>(w, s, b, xr, xs, acc);
-                    else task_mma<BITS, MT, false>(w, s, b, xr, xs, acc);
-#pragma unroll
-                    for (int mt = 0; mt < MT; mt++)
-                        dstp[mt * 32] = make_float4(acc[mt][0][0] + acc[mt][1][0], acc[mt][0][1] + acc[mt][1][1],
-                                                    acc[mt][0][2] + acc[mt][1][2], acc[mt][0][3] + acc[mt][1][3]);
+                    for (int mt = 0; mt < MT; mt++) dstp[mt * 32] = out[mt];
                     dstp += nkl * E4;
                     __syncwarp();  // every lane is done with the stage before it is refilled
                     src_c = src_c + kStageBytes == ring_lo + D * kStageBytes ? ring_lo : src_c + kStageBytes;
@@ -730,7 +556,7 @@ __global__ void __launch_bounds__(kThreads, 1) qmv_mma_kernel(const __grid_const
 }
 
 // ---- several matmuls of one shape per launch ------------------------------------------------------------
-constexpr int kMaxBatch = 48;
+constexpr int kMaxBatch = 48;  // = qmv_batch_max()
 struct BatchItem {
     const __nv_bfloat16* x;
     const uint32_t* wq;
@@ -745,28 +571,12 @@ struct BatchParams {
     int K, N, gshift, y_bf16;
     int nkb, n_rt, chunks, tb, sb_bytes, xs_off;
     BatchItem items[kMaxBatch];
-    // column-sharded launches only (SH): N is this rank's share of the columns
+    // N is this rank's share of the columns
     int ld, col0, yt_off;
     int* error;
     long long peer_wait_ns;
     ShardPush sp;
 };
-template <int BITS, int MT>
-__device__ __forceinline__ void load_x_item(const __nv_bfloat16* x, int M, int K, int kb, int g, int t, uint4 (&xr)[MT][BITS == 4 ? 8 : 4]) {
-    constexpr int XV = BITS == 4 ? 8 : 4;
-    constexpr int KB = 1024 / BITS;
-#pragma unroll
-    for (int mt = 0; mt < MT; mt++) {
-        const int m = mt * 8 + g;
-        const __nv_bfloat16* row = x + (size_t)m * K + kb * KB + t * (KB / 8);
-#pragma unroll
-        for (int j = 0; j < XV; j++) {
-            const int h = j / (XV / 2), i = j % (XV / 2);
-            xr[mt][j] = make_uint4(0, 0, 0, 0);
-            if (m < M) xr[mt][j] = ldg_nc_v4(reinterpret_cast<const uint4*>(row + h * (KB / 2) + i * 8));
-        }
-    }
-}
 // ytile (column-sharded launches): the tile's values once more in shared memory, [row of x][16 columns]
 template <int MT>
 __device__ __forceinline__ void store_tile_item(void* y, int M, int N, int ld, int col0, int y_bf16, int rt, int e, float sum,
@@ -788,15 +598,13 @@ __device__ __forceinline__ void store_tile_item(void* y, int M, int N, int ld, i
     }
 }
 
-// Several decode matmuls of one shape (K, N, bits, group; M <= 8*MT each) in ONE launch: qmv_mma_kernel's roles and
-// arithmetic with a loop over the matmuls around them.  A CTA keeps its range of row tiles through all of them and
-// its warps' rings never drain in between: the fetch iterator walks from the last task of one matmul into the
-// first of the next, so the start of a launch (first reads of parameters, x and weights) and its tail (the
-// ordered sum and the store of y), which are half of a single decode launch, are paid once per launch instead of
-// once per matmul -- the sum and the store of a matmul run while the next one's weights are already arriving.
-// No K split, no prologue (the host sends such calls one by one).
+// Several decode matmuls of one shape (K, N, bits, group; M <= 8*MT each) of a layer whose columns are sharded over
+// ranks, in ONE launch (unsharded: qmv_stream.cu): qmv_mma_kernel's roles and arithmetic with a loop over the matmuls
+// around them.  A CTA keeps its range of row tiles through all of them and its warps' rings never drain in between: the
+// fetch iterator walks from the last task of one matmul into the first of the next.  No K split, no prologue (the host
+// sends such calls one by one).
 //
-// SH: the layer is column-sharded over ranks and every y lives at the same offset of every rank's symmetric buffer.
+// Every y lives at the same offset of every rank's symmetric buffer.
 // The finished tiles of a matmul (staged in shared memory as they are stored locally) go straight into the peers'
 // copies of y, 16 bytes a store, while the warps are already in the next matmul.  The hand-shakes are paid once
 // per launch instead of once per matmul: ready[q] as in qmv_mma_kernel (before the first remote store: has every
@@ -811,7 +619,7 @@ __device__ __forceinline__ void store_tile_item(void* y, int M, int N, int ld, i
 // With four tasks in flight per warp instead of three, a matmul's four or five tasks per warp are (nearly) all on
 // their way before the previous matmul's end, so the memory system keeps working through it.
 constexpr int kDeepDepth = 5, kDeepStageBytes = 2048 + 256;
-template <int BITS, int MT, bool SH, bool DEEP>
+template <int BITS, int MT, bool DEEP>
 __global__ void __launch_bounds__(kThreads, 1) qmv_batch_kernel(const __grid_constant__ BatchParams p) {
     constexpr int XV = BITS == 4 ? 8 : 4;  // x fragments (uint4) per lane per k-block per 8-row block
     constexpr int KB = 1024 / BITS;        // weights per k-block (128 bytes per row)
@@ -825,6 +633,7 @@ __global__ void __launch_bounds__(kThreads, 1) qmv_batch_kernel(const __grid_con
     // after the partials (MT == 2): the x fragments of rows 8..15, [warp][fragment][lane]
     uint4* xs = reinterpret_cast<uint4*>(smem + p.xs_off) + (threadIdx.x >> 5) * (XV * 32) + (threadIdx.x & 31);
 
+    constexpr int KL = lane_weights(BITS), SPL = BITS == 4 ? 2 : 1;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int g = lane >> 2, t = lane & 3;
     const int ci = blockIdx.x;
@@ -859,7 +668,7 @@ __global__ void __launch_bounds__(kThreads, 1) qmv_batch_kernel(const __grid_con
     const int gpk = KB >> p.gshift;    // groups per k-block
     // the matmul whose weights are being fetched (f_pi) runs ahead of the one being computed (pi)
     int f_pi = 0;
-    const unsigned char* wbase = reinterpret_cast<const unsigned char*>(p.items[0].wq) + t * 16;
+    const unsigned char* wbase = reinterpret_cast<const unsigned char*>(p.items[0].wq) + t * 32;
     const __nv_bfloat16* sb_src = lane < 16 ? p.items[0].scales : p.items[0].biases;
     const uint32_t ring_lo = smem_u32(smem) + warp * (D * kStageBytes) + lane * 16;  // this lane's slot, stage 0
     const int tail_tile = (p.N & 15) ? p.n_rt - 1 : -1;  // the tile whose rows must be clamped to N-1
@@ -871,7 +680,7 @@ __global__ void __launch_bounds__(kThreads, 1) qmv_batch_kernel(const __grid_con
     const size_t half_tile = 8 * row_bytes, tile_stride = 16 * row_bytes;
     int f_b0 = rt_lo, f_kb = kb_lo + warp, f_rt = rt_lo;  // the task fetched next
     uint32_t f_dst = ring_lo;                             // and the stage it goes to
-    // this lane's sources of that task: rows g and g+8 of the tile (its 16-byte pieces t and t+4 of the k-block),
+    // this lane's sources of that task: rows g and g+8 of the tile (its 32 bytes of the k-block),
     // the scales (lanes 0-15) or biases (16-31) of row lane%16.  Inside a run they move by constant strides.
     const unsigned char* f_p0 = nullptr;
     const unsigned char* f_p1 = nullptr;
@@ -892,9 +701,9 @@ __global__ void __launch_bounds__(kThreads, 1) qmv_batch_kernel(const __grid_con
     auto fetch_next = [&]() {
         if (has_work && f_pi < p.n_items) {
             cp_async16(f_dst, f_p0);
-            cp_async16(f_dst + 512, f_p0 + 64);
+            cp_async16(f_dst + 512, f_p0 + 16);
             cp_async16(f_dst + 1024, f_p1);
-            cp_async16(f_dst + 1536, f_p1 + 64);
+            cp_async16(f_dst + 1536, f_p1 + 16);
             const uint32_t sb_dst = f_dst + 2048 - lane * (16 - kSlot);  // (f_dst is this lane's 16-byte slot of the stage)
             if (!DEEP && p.sb_bytes == 16) cp_async16(sb_dst, f_sb);
             else if (p.sb_bytes == 8) cp_async8(sb_dst, f_sb);
@@ -910,7 +719,7 @@ __global__ void __launch_bounds__(kThreads, 1) qmv_batch_kernel(const __grid_con
                 if (f_b0 >= f_hi && ++f_pi < p.n_items) {  // on to the next matmul: the next range of tiles, its weights
                     next_range(f_c, f_lo, f_hi, f_acc);
                     f_b0 = f_lo;
-                    wbase = reinterpret_cast<const unsigned char*>(p.items[f_pi].wq) + t * 16;
+                    wbase = reinterpret_cast<const unsigned char*>(p.items[f_pi].wq) + t * 32;
                     sb_src = lane < 16 ? p.items[f_pi].scales : p.items[f_pi].biases;
                 }
                 f_rt = f_b0;
@@ -928,20 +737,27 @@ __global__ void __launch_bounds__(kThreads, 1) qmv_batch_kernel(const __grid_con
 
     uint4 xr[MT][XV];
     bool x_ahead = false;  // xr already holds the fragments of the run about to start
+    auto load_x = [&](const __nv_bfloat16* x, int M, int kb) {
+#pragma unroll
+        for (int mt = 0; mt < MT; mt++) {
+            const int m = mt * 8 + g;
+            load_x_row<BITS, 0>(m < M ? x + (size_t)m * p.K : nullptr, p.K, kb, t, xr[mt]);
+        }
+    };
 #pragma unroll
     for (int i = 0; i < D - 1; i++) fetch_next();
     // column-sharded: this call's number, and the word to the peers that our copies of y may be overwritten
     // (the launch is an ordinary one: whatever this rank enqueued before has finished with them)
     uint32_t epoch = 0;
-    bool peers_ready = true, ready_checked = !SH;
-    if (SH) {
+    bool peers_ready = true, ready_checked = false;
+    {
         epoch = *reinterpret_cast<volatile uint32_t*>(p.sp.flags[p.sp.me] + kFlagEpoch) + 1;
         if (blockIdx.x == 0 && tid < p.sp.world && tid != p.sp.me) st_relaxed_sys(p.sp.flags[tid] + kFlagReady + p.sp.me, epoch);
     }
-    unsigned char* const ytiles = SH ? smem + p.yt_off : nullptr;
+    unsigned char* const ytiles = smem + p.yt_off;
     const int yt_bytes = p.y_bf16 ? 512 : 1024;  // of a staged tile
     uint32_t src_c = ring_lo;  // stage of the task computed next (this lane's slot)
-    uint32_t sboff[2][2];      // byte offsets of this lane's scales inside a stage, by row half r and piece h
+    uint32_t sboff[2][SPL];    // byte offsets of this lane's scales inside a stage, by row half r
 #pragma unroll 1
     for (int pi = 0; pi < p.n_items; pi++) {
     if (pi) next_range(rt_c, rt_lo, rt_hi, rt_acc);
@@ -955,10 +771,10 @@ __global__ void __launch_bounds__(kThreads, 1) qmv_batch_kernel(const __grid_con
 #pragma unroll 1
             for (int kb = kb_lo + warp; kb < kb_hi; kb += kWarps) {
                 fetch_next();  // (the run's first fetch goes out ahead of the x loads)
-                if (!x_ahead) load_x_item<BITS, MT>(x_cur, M_cur, p.K, kb, g, t, xr);
+                if (!x_ahead) load_x(x_cur, M_cur, kb);
                 x_ahead = false;
-                permute_x<BITS, MT>(xr);
-                if (MT == 2 && kX1Shared) {
+                for (int mt = 0; mt < MT; mt++) permute_x<BITS>(xr[mt]);
+                if (MT == 2) {
                     __syncwarp();  // (the previous run's reads of xs)
 #pragma unroll
                     for (int j = 0; j < XV; j++) xs[j * 32] = xr[MT - 1][j];
@@ -969,8 +785,8 @@ __global__ void __launch_bounds__(kThreads, 1) qmv_batch_kernel(const __grid_con
                     const int slot = g + 8 * r;
                     const int par = p.sb_bytes == 2 ? ((slot * gpr + kb) & 1) : 0;
 #pragma unroll
-                    for (int h = 0; h < 2; h++)
-                        sboff[r][h] = 2048 - lane * 16 + slot * kSlot + ((((h * (KB / 2) + t * (KB / 8)) >> p.gshift) + par) << 1);
+                    for (int i = 0; i < SPL; i++)
+                        sboff[r][i] = 2048 - lane * 16 + slot * kSlot + ((((t * KL + i * 32) >> p.gshift) + par) << 1);
                 }
                 float4* dstp = part + (kb - kb_lo) * E4 + lane;
 #pragma unroll 1
@@ -978,30 +794,27 @@ __global__ void __launch_bounds__(kThreads, 1) qmv_batch_kernel(const __grid_con
                     if (rt != b0) fetch_next();
                     cp_async_wait<D - 1>();
                     __syncwarp();
-                    uint4 w[2][2];
-                    uint32_t s[2][2], b[2][2];
+                    uint32_t w[2][8];
+                    uint32_t s[2][SPL], b[2][SPL];
 #pragma unroll
-                    for (int r = 0; r < 2; r++)
+                    for (int r = 0; r < 2; r++) {
 #pragma unroll
-                        for (int h = 0; h < 2; h++) {
+                        for (int h = 0; h < 2; h++)
                             asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];"
-                                         : "=r"(w[r][h].x), "=r"(w[r][h].y), "=r"(w[r][h].z), "=r"(w[r][h].w)
+                                         : "=r"(w[r][4 * h]), "=r"(w[r][4 * h + 1]), "=r"(w[r][4 * h + 2]), "=r"(w[r][4 * h + 3])
                                          : "r"(src_c + (r * 2 + h) * 512));
-                            asm volatile("ld.shared.u16 %0, [%1];" : "=r"(s[r][h]) : "r"(src_c + sboff[r][h]));
-                            asm volatile("ld.shared.u16 %0, [%1+%2];" : "=r"(b[r][h]) : "r"(src_c + sboff[r][h]), "n"(16 * kSlot));
+#pragma unroll
+                        for (int i = 0; i < SPL; i++) {
+                            asm volatile("ld.shared.u16 %0, [%1];" : "=r"(s[r][i]) : "r"(src_c + sboff[r][i]));
+                            asm volatile("ld.shared.u16 %0, [%1+%2];" : "=r"(b[r][i]) : "r"(src_c + sboff[r][i]), "n"(16 * kSlot));
                         }
-                    const bool fast = scales_fast_ok4(s[0][0], s[0][1], s[1][0], s[1][1]);
-                    float acc[MT][2][4];  // two independent accumulation chains per 8-row block of x
+                    }
+                    float4 out[MT];
+                    auto x_hi = [&](int j) { return xs[j * 32]; };
+                    if (__all_sync(0xffffffffu, scales_fast_ok<SPL>(s))) task_mma<BITS, MT, SPL, true>(w, s, b, xr[0], x_hi, out);
+                    else task_mma<BITS, MT, SPL, false>(w, s, b, xr[0], x_hi, out);
 #pragma unroll
-                    for (int mt = 0; mt < MT; mt++)
-#pragma unroll
-                        for (int c = 0; c < 2; c++) acc[mt][c][0] = acc[mt][c][1] = acc[mt][c][2] = acc[mt][c][3] = 0.0f;
-                    if (__all_sync(0xffffffffu, fast)) task_mma<BITS, MT, true>(w, s, b, xr, xs, acc);
-                    else task_mma<BITS, MT, false>(w, s, b, xr, xs, acc);
-#pragma unroll
-                    for (int mt = 0; mt < MT; mt++)
-                        dstp[mt * 32] = make_float4(acc[mt][0][0] + acc[mt][1][0], acc[mt][0][1] + acc[mt][1][1],
-                                                    acc[mt][0][2] + acc[mt][1][2], acc[mt][0][3] + acc[mt][1][3]);
+                    for (int mt = 0; mt < MT; mt++) dstp[mt * 32] = out[mt];
                     dstp += nkl * E4;
                     __syncwarp();  // every lane is done with the stage before it is refilled
                     src_c = src_c + kStageBytes == ring_lo + D * kStageBytes ? ring_lo : src_c + kStageBytes;
@@ -1013,10 +826,10 @@ __global__ void __launch_bounds__(kThreads, 1) qmv_batch_kernel(const __grid_con
         // spent in the sum and the store below instead of in front of the next matmul's first task.
         // (With 16 rows of x the fragments held across the block barrier spill: measured 16.5 against 11.2 us.)
         if (MT == 1 && has_work && kb_hi - kb_lo <= kWarps && rt_hi - rt_lo <= tb && pi + 1 < p.n_items) {
-            load_x_item<BITS, MT>(p.items[pi + 1].x, p.items[pi + 1].M, p.K, kb_lo + warp, g, t, xr);
+            load_x(p.items[pi + 1].x, p.items[pi + 1].M, kb_lo + warp);
             x_ahead = true;
         }
-        if (SH && !ready_checked) {  // before the first remote store: has every peer started this call?
+        if (!ready_checked) {  // before the first remote store: has every peer started this call?
             ready_checked = true;
             int ok = 1;
             if (tid < p.sp.world && tid != p.sp.me) ok = wait_flag(p.sp.flags[p.sp.me] + kFlagReady + tid, epoch, p.peer_wait_ns);
@@ -1028,12 +841,12 @@ __global__ void __launch_bounds__(kThreads, 1) qmv_batch_kernel(const __grid_con
             constexpr int E = 128 * MT;
             __syncthreads();
             for (int ti = tid / E; ti < nt; ti += kThreads / E)
-                store_tile_item<MT>(y_cur, M_cur, p.N, SH ? p.ld : p.N, SH ? p.col0 : 0, p.y_bf16, b0 + ti, tid % E,
+                store_tile_item<MT>(y_cur, M_cur, p.N, p.ld, p.col0, p.y_bf16, b0 + ti, tid % E,
                                     ordered_sum<false>(reinterpret_cast<const float*>(part) + ti * nkl * E + tid % E, nkl, E, 0.0f),
-                                    SH ? ytiles + ti * yt_bytes : nullptr);
+                                    ytiles + ti * yt_bytes);
             __syncthreads();  // the partial buffer is reused by the next batch (of this matmul or the next)
         }
-        if (SH && peers_ready) {
+        if (peers_ready) {
             // The staged tiles go to the peers, a 16-byte piece of a row per store.  (The staging area is written
             // again only behind the first barrier of the next batch end, which a thread reaches after these reads.)
             const int esz = p.y_bf16 ? 2 : 4;            // also the number of 16-byte pieces of a tile row
@@ -1053,7 +866,7 @@ __global__ void __launch_bounds__(kThreads, 1) qmv_batch_kernel(const __grid_con
     }
     }
     cp_async_wait<0>();
-    if (SH) {
+    {
         __syncthreads();  // every remote store of this CTA has been issued
         if (tid == 0) {
             __threadfence_system();  // ... and is ordered before the count below, for every observer
@@ -1191,12 +1004,26 @@ size_t qmv_mma_workspace_bytes(const QmmArgs& a, int sm_count) {
     return kCounterBytes + pl.scratch_bytes;
 }
 
+static const char* variant_name(int bits, int mt, int pro) {
+    if (bits == 4) return mt == 2 ? "qmv_mma<4,m16>" : pro == 1 ? "qmv_mma<4,m8,rms>" : pro == 2 ? "qmv_mma<4,m8,sum3>" : "qmv_mma<4,m8>";
+    return mt == 2 ? "qmv_mma<8,m16>" : pro == 1 ? "qmv_mma<8,m8,rms>" : pro == 2 ? "qmv_mma<8,m8,sum3>" : "qmv_mma<8,m8>";
+}
+
+// Launches of their own CTAs' whole K on one GPU go to qmv_stream.cu; this file's kernel takes the launches whose K is
+// split over CTAs and those that deliver y to peers.
 // workspace layout: [counters: kCounterBytes][partials]; the counters must be zero before the
 // first launch and are left zero by every launch.
 cudaError_t launch_qmv_mma(const QmmArgs& a, void* workspace, int sm_count, cudaStream_t stream, const char** name,
                            bool overlap_prev, const ShardPush* push, bool x_stable) {
     Plan pl;
-    if (!make_plan(a, sm_count, &pl, push && push->world > 1)) return cudaErrorInvalidValue;
+    const bool sharded = push && push->world > 1;
+    const bool on_grid = make_plan(a, sm_count, &pl, sharded);
+    if (!sharded && (!on_grid || pl.ks == 1)) {
+        // (the name: a K off the k-block grid belongs to the family that callers know for such shapes)
+        if (name) *name = on_grid ? variant_name(a.bits, a.M <= 8 ? 1 : 2, a.pro) : a.bits == 4 ? "qmv_simt<4,bf16,mma>" : "qmv_simt<8,bf16,mma>";
+        return launch_qmv_stream(&a, 1, sm_count, stream, overlap_prev, x_stable);
+    }
+    if (!on_grid) return cudaErrorInvalidValue;
     Params p;
     p.x = (const __nv_bfloat16*)a.x;
     p.wq = a.wq;
@@ -1231,24 +1058,22 @@ cudaError_t launch_qmv_mma(const QmmArgs& a, void* workspace, int sm_count, cuda
         p.error = a.error ? a.error : device_error_word();
         if (!p.error) return cudaErrorMemoryAllocation;
     }
+    if (name) *name = variant_name(a.bits, pl.mt, a.pro);
     if (a.bits == 4) {
-        if (name) *name = pl.mt == 2 ? "qmv_mma<4,m16>" : a.pro == 1 ? "qmv_mma<4,m8,rms>" : a.pro == 2 ? "qmv_mma<4,m8,sum3>" : "qmv_mma<4,m8>";
         if (pl.mt == 2) return launch_t<4, 2, 0>(p, pl, stream, overlap_prev);
         return a.pro == 1 ? launch_t<4, 1, 1>(p, pl, stream, overlap_prev)
              : a.pro == 2 ? launch_t<4, 1, 2>(p, pl, stream, overlap_prev) : launch_t<4, 1, 0>(p, pl, stream, overlap_prev);
     }
-    if (name) *name = pl.mt == 2 ? "qmv_mma<8,m16>" : a.pro == 1 ? "qmv_mma<8,m8,rms>" : a.pro == 2 ? "qmv_mma<8,m8,sum3>" : "qmv_mma<8,m8>";
     if (pl.mt == 2) return launch_t<8, 2, 0>(p, pl, stream, overlap_prev);
     return a.pro == 1 ? launch_t<8, 1, 1>(p, pl, stream, overlap_prev)
          : a.pro == 2 ? launch_t<8, 1, 2>(p, pl, stream, overlap_prev) : launch_t<8, 1, 0>(p, pl, stream, overlap_prev);
 }
 
-
 // Several matmuls of one shape in one launch (qmv_batch_kernel).  All items: the shape of items[0] but for M, with
 // M on the same side of 8; bf16; no K split for that shape.  cudaErrorNotSupported otherwise.
-template <int BITS, int MT, bool SH, bool DEEP>
+template <int BITS, int MT, bool DEEP>
 cudaError_t launch_batch_t(const BatchParams& p, const Plan& pl, cudaStream_t stream) {
-    auto kern = qmv_batch_kernel<BITS, MT, SH, DEEP>;
+    auto kern = qmv_batch_kernel<BITS, MT, DEEP>;
     static std::atomic<size_t> attr_smem[64];
     int dev = 0;
     cudaGetDevice(&dev);
@@ -1260,7 +1085,6 @@ cudaError_t launch_batch_t(const BatchParams& p, const Plan& pl, cudaStream_t st
     kern<<<pl.chunks, kThreads, pl.smem, stream>>>(p);
     return cudaGetLastError();
 }
-int qmv_batch_max() { return kMaxBatch; }
 cudaError_t launch_qmv_batch(const QmmArgs* items, int n, int sm_count, cudaStream_t stream, const char** name,
                              const ShardPush* push) {
     if (n < 1 || n > kMaxBatch) return cudaErrorInvalidValue;
@@ -1270,7 +1094,13 @@ cudaError_t launch_qmv_batch(const QmmArgs* items, int n, int sm_count, cudaStre
     int mmax = 0;
     for (int i = 0; i < n; i++) mmax = std::max(mmax, items[i].M);
     a0.M = mmax;
-    if (!make_plan(a0, sm_count, &pl, sh) || pl.ks != 1) return cudaErrorNotSupported;
+    const bool on_grid = make_plan(a0, sm_count, &pl, sh);
+    if (on_grid && pl.ks != 1) return cudaErrorNotSupported;
+    if (!sh) {
+        if (name) *name = a0.bits == 4 ? (mmax <= 8 ? "qmv_batch<4,m8>" : "qmv_batch<4,m16>") : (mmax <= 8 ? "qmv_batch<8,m8>" : "qmv_batch<8,m16>");
+        return launch_qmv_stream(items, n, sm_count, stream, false, false);
+    }
+    if (!on_grid) return cudaErrorNotSupported;
     // The deep ring (see the kernel) when a CTA's tiles of a matmul still fit into one batch beside it
     bool deep = false;
     if (pl.mt == 1 && pl.sb_bytes <= 8 && !getenv("LUXCUDA_QMV_BATCH_NO_DEEP")) {
@@ -1280,17 +1110,14 @@ cudaError_t launch_qmv_batch(const QmmArgs* items, int n, int sm_count, cudaStre
             deep = true;
         }
     }
+    if (push->world > kMaxShardWorld || (a0.N & 15)) return cudaErrorInvalidValue;  // whole 16-column tiles only
     BatchParams p;
-    p.ld = a0.N; p.col0 = 0; p.yt_off = pl.yt_off;
-    p.error = nullptr;
+    p.yt_off = pl.yt_off;
     p.peer_wait_ns = peer_wait_limit_ns();
-    if (sh) {
-        if (push->world > kMaxShardWorld || (a0.N & 15)) return cudaErrorInvalidValue;  // whole 16-column tiles only
-        p.sp = *push;
-        p.ld = push->ld; p.col0 = push->col0;
-        p.error = a0.error ? a0.error : device_error_word();
-        if (!p.error) return cudaErrorMemoryAllocation;
-    }
+    p.sp = *push;
+    p.ld = push->ld; p.col0 = push->col0;
+    p.error = a0.error ? a0.error : device_error_word();
+    if (!p.error) return cudaErrorMemoryAllocation;
     p.n_items = n;
     p.K = a0.K; p.N = a0.N; p.gshift = pl.gshift;
     p.y_bf16 = a0.y_dtype == LUX_DTYPE_BFLOAT16;
@@ -1301,24 +1128,19 @@ cudaError_t launch_qmv_batch(const QmmArgs* items, int n, int sm_count, cudaStre
             a.x_dtype != LUX_DTYPE_BFLOAT16 || a.sb_dtype != LUX_DTYPE_BFLOAT16 || a.M < 1 || (a.M <= 8) != (mmax <= 8) || a.pro)
             return cudaErrorNotSupported;
         if (((uintptr_t)a.wq | (uintptr_t)a.x | (uintptr_t)a.scales | (uintptr_t)a.biases) & 15) return cudaErrorInvalidValue;
-        uint32_t yoff = 0;
-        if (sh) {  // the item's y lies inside this rank's symmetric buffer: the peers' copies are at the same offset
-            const ptrdiff_t d = static_cast<const char*>(a.y) - static_cast<const char*>(push->y[push->me]);
-            if (d < 0 || d > (ptrdiff_t)0xFFFFFFF0ll || (d & 15)) return cudaErrorInvalidValue;
-            yoff = (uint32_t)d;
-        }
-        p.items[i] = BatchItem{(const __nv_bfloat16*)a.x, a.wq, (const __nv_bfloat16*)a.scales, (const __nv_bfloat16*)a.biases, a.y, a.M, yoff};
+        // the item's y lies inside this rank's symmetric buffer: the peers' copies are at the same offset
+        const ptrdiff_t d = static_cast<const char*>(a.y) - static_cast<const char*>(push->y[push->me]);
+        if (d < 0 || d > (ptrdiff_t)0xFFFFFFF0ll || (d & 15)) return cudaErrorInvalidValue;
+        p.items[i] = BatchItem{(const __nv_bfloat16*)a.x, a.wq, (const __nv_bfloat16*)a.scales, (const __nv_bfloat16*)a.biases, a.y, a.M, (uint32_t)d};
     }
     if (a0.bits == 4) {
-        if (name) *name = sh ? (pl.mt == 1 ? "qmv_batch<4,m8,push>" : "qmv_batch<4,m16,push>") : (pl.mt == 1 ? "qmv_batch<4,m8>" : "qmv_batch<4,m16>");
-        if (deep) return sh ? launch_batch_t<4, 1, true, true>(p, pl, stream) : launch_batch_t<4, 1, false, true>(p, pl, stream);
-        if (sh) return pl.mt == 1 ? launch_batch_t<4, 1, true, false>(p, pl, stream) : launch_batch_t<4, 2, true, false>(p, pl, stream);
-        return pl.mt == 1 ? launch_batch_t<4, 1, false, false>(p, pl, stream) : launch_batch_t<4, 2, false, false>(p, pl, stream);
+        if (name) *name = pl.mt == 1 ? "qmv_batch<4,m8,push>" : "qmv_batch<4,m16,push>";
+        if (pl.mt == 2) return launch_batch_t<4, 2, false>(p, pl, stream);
+        return deep ? launch_batch_t<4, 1, true>(p, pl, stream) : launch_batch_t<4, 1, false>(p, pl, stream);
     }
-    if (name) *name = sh ? (pl.mt == 1 ? "qmv_batch<8,m8,push>" : "qmv_batch<8,m16,push>") : (pl.mt == 1 ? "qmv_batch<8,m8>" : "qmv_batch<8,m16>");
-    if (deep) return sh ? launch_batch_t<8, 1, true, true>(p, pl, stream) : launch_batch_t<8, 1, false, true>(p, pl, stream);
-    if (sh) return pl.mt == 1 ? launch_batch_t<8, 1, true, false>(p, pl, stream) : launch_batch_t<8, 2, true, false>(p, pl, stream);
-    return pl.mt == 1 ? launch_batch_t<8, 1, false, false>(p, pl, stream) : launch_batch_t<8, 2, false, false>(p, pl, stream);
+    if (name) *name = pl.mt == 1 ? "qmv_batch<8,m8,push>" : "qmv_batch<8,m16,push>";
+    if (pl.mt == 2) return launch_batch_t<8, 2, false>(p, pl, stream);
+    return deep ? launch_batch_t<8, 1, true>(p, pl, stream) : launch_batch_t<8, 1, false>(p, pl, stream);
 }
 
 // ---------------------------------------------------------------------------------

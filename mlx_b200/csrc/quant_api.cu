@@ -129,7 +129,7 @@ LuxBackendError qmatmul_on_stream(Context* c, const QmmArgs& a) {
             // decode kernel, 16 rows of x per launch
             QmmArgs chunk = a;
             chunk.M = a.M < 16 ? a.M : 16;
-            if (qmv_mma_supported(chunk, c->dev->sm_count)) {
+            if (qmv_mma_supported(chunk, c->dev->sm_count) || qmv_stream_supported(chunk, c->dev->sm_count)) {
                 const size_t ws = qmv_mma_workspace_bytes(chunk, c->dev->sm_count);
                 LuxBackendError le = ensure_qmv_workspace(c, ws);
                 if (le != LUX_BACKEND_OK) return le;
@@ -139,7 +139,7 @@ LuxBackendError qmatmul_on_stream(Context* c, const QmmArgs& a) {
                     chunk.M = a.M - m0 < 16 ? a.M - m0 : 16;
                     chunk.x = (const char*)a.x + (size_t)m0 * a.K * 2;
                     chunk.y = (char*)a.y + (size_t)m0 * a.N * ysz;
-                    e = launch_qmv_mma(chunk, c->qmv_ws->ptr, c->dev->sm_count, c->stream, &name, decode_may_overlap(c, chunk),
+                    e = launch_qmv_mma(chunk, c->qmv_ws ? c->qmv_ws->ptr : nullptr, c->dev->sm_count, c->stream, &name, decode_may_overlap(c, chunk),
                                        nullptr, decode_x_stable(c, chunk));
                     if (e == cudaSuccess) {
                         c->launches++;
