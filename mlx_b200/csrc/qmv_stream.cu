@@ -122,6 +122,13 @@ __device__ __forceinline__ V8 ldg_v8(const void* p) {  // 32 bytes, through L1 a
     return r;
 }
 
+__device__ __forceinline__ V8 ldg_2v4(const void* p) {  // the same from a 16-byte boundary
+    V8 r;
+    asm volatile("ld.global.v4.b32 {%0,%1,%2,%3}, [%4];" : "=r"(r.v[0]), "=r"(r.v[1]), "=r"(r.v[2]), "=r"(r.v[3]) : "l"(p));
+    asm volatile("ld.global.v4.b32 {%0,%1,%2,%3}, [%4];" : "=r"(r.v[4]), "=r"(r.v[5]), "=r"(r.v[6]), "=r"(r.v[7]) : "l"((const char*)p + 16));
+    return r;
+}
+
 struct Item {
     const __nv_bfloat16* x;
     const __nv_bfloat16* scales;
@@ -141,6 +148,7 @@ struct Params {
     int stages, sum_warps, stage_bytes, tile_bytes, sb_off;  // bytes of weights per tile; offset of the scales in a stage
     int xs_off, run_off, bar_off;                 // offsets in shared memory
     int x_early, x_ld;      // see launch_qmv_mma
+    int x32;                // every row of every x starts on a 32-byte boundary (callers owe 16 bytes only)
     float eps;              // of the rms-norm prologue
     int* error;             // host-visible error word of the bounded waits
 };
@@ -405,9 +413,9 @@ __global__ void __launch_bounds__(kThreads, 1) qmv_stream_kernel(const __grid_co
                     for (int e = 0; e < 8; e++) v[h][i].v[e] = 0;
                     if (row + i * RPI < it.M && k < p.K) {
                         const __nv_bfloat16* s = it.x + (size_t)(row + i * RPI) * ld + k;
-                        v[h][i] = ldg_v8(s);
+                        v[h][i] = p.x32 ? ldg_v8(s) : ldg_2v4(s);
                         if (PRO == 2) {
-                            const V8 b = ldg_v8(s + p.K), d = ldg_v8(s + 2 * p.K);
+                            const V8 b = p.x32 ? ldg_v8(s + p.K) : ldg_2v4(s + p.K), d = p.x32 ? ldg_v8(s + 2 * p.K) : ldg_2v4(s + 2 * p.K);
 #pragma unroll
                             for (int e = 0; e < 8; e++) v[h][i].v[e] = add3_bf16x2(v[h][i].v[e], b.v[e], d.v[e]);
                         }
@@ -647,7 +655,9 @@ cudaError_t launch_items(const QmmArgs* items, int n, int mmax, const Plan& pl, 
     p.x_ld = a0.pro ? a0.x_ld : a0.K;
     p.eps = a0.eps;
     p.error = a0.error ? a0.error : device_error_word();
+    p.x32 = p.x_ld % 16 == 0;
     for (int i = 0; i < n; i++) {
+        if ((uintptr_t)items[i].x & 31) p.x32 = 0;
         if (!encode_weights(items[i], pl, &p.maps[i])) return cudaErrorInvalidValue;
         p.items[i] = Item{(const __nv_bfloat16*)items[i].x, (const __nv_bfloat16*)items[i].scales,
                           (const __nv_bfloat16*)items[i].biases, items[i].y, items[i].M};

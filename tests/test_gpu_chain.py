@@ -242,6 +242,34 @@ def test_prologues_equal_the_separate_steps(ctx, oracle, M, K, N, bits, group):
         assert np.array_equal(y_one.to_host(), first)
 
 
+@pytest.mark.parametrize("M,K,bits,group", [(1, 1024, 4, 64), (8, 1024, 8, 128), (16, 512, 4, 32), (5, 288, 4, 32)])
+def test_rows_of_x_on_16_byte_boundaries(ctx, oracle, M, K, bits, group):
+    """Callers owe 16-byte boundaries, not more: x at an odd multiple of 16 bytes (alone and as one item of a batch) and
+    rows x_ld apart with x_ld an odd multiple of 8 elements give the bits of the same values on wider boundaries."""
+    N = 80
+    wq, s, b = oracle.make_layer(N, K, bits, group, oracle.BF16, config_id=5, layer=K, proj=3)
+    bw, bs, bb = ctx.upload(wq), ctx.upload(s), ctx.upload(b)
+    x = oracle.make_x(M, K, oracle.BF16, config_id=5, tag=M)
+    ref, got, got2 = (ctx.empty((M, N), np.uint16) for _ in range(3))
+    bx = ctx.upload(x)
+    ctx.qmatmul(bx, bw, bs, bb, ref, M, K, N, bits, group, BF16, BF16, BF16)
+    room = ctx.upload(np.concatenate([np.zeros(8, np.uint16), x.ravel()]))
+    odd = ctx.wrap(room.device_ptr + 16, x.nbytes)
+    ctx.qmatmul(odd, bw, bs, bb, got, M, K, N, bits, group, BF16, BF16, BF16)
+    assert np.array_equal(got.to_host(), ref.to_host())
+    ctx.qmatmul_batch([bx, odd], [bw, bw], [bs, bs], [bb, bb], [got2, got], [M, M], K, N, bits, group, BF16)
+    assert np.array_equal(got.to_host(), ref.to_host()) and np.array_equal(got2.to_host(), ref.to_host())
+    if M <= 8 and K % (1024 // bits) == 0:
+        for pro, cols in ((P.PRO_RMS_NORM, K), (P.PRO_SUM3, 3 * K)):
+            w = oracle.make_x(M, cols, oracle.BF16, config_id=5, tag=100 + M)
+            ld = cols + 8
+            wide = np.zeros((M, ld), np.uint16)
+            wide[:, :cols] = w
+            ctx.qmatmul_pro(ctx.upload(w), bw, bs, bb, ref, M, K, N, bits, group, BF16, pro, cols, 1e-6)
+            ctx.qmatmul_pro(ctx.upload(wide), bw, bs, bb, got, M, K, N, bits, group, BF16, pro, ld, 1e-6)
+            assert np.array_equal(got.to_host(), ref.to_host())
+
+
 def test_prologue_refuses_what_it_does_not_take(ctx, oracle, plugin):
     K, N = 8192, 64
     wq, s, b = oracle.make_layer(N, K, 4, 64, oracle.BF16, config_id=5, layer=9)
