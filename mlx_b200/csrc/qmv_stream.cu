@@ -550,14 +550,13 @@ bool make_plan(const QmmArgs& a, int mmax, int sm_count, Plan* pl) {
     if ((long long)a.N * (a.K / a.group) > (1ll << 30) || (long long)pl->n_rt * pl->nkb > (1ll << 26)) return false;  // 32-bit indices
     pl->grid = std::min(pl->n_rt, sm_count);
     const int tiles_max = (pl->n_rt + pl->grid - 1) / pl->grid;
-    if (tiles_max > 4096) return false;  // (Walk::groups)
     pl->nch = (pl->nkb + kWarps - 1) / kWarps;
     pl->kbc = (pl->nkb + pl->nch - 1) / pl->nch;
     pl->nch = (pl->nkb + pl->kbc - 1) / pl->kbc;
     pl->tile_bytes = pl->kbc * 2048;
     const int sb = 32 * sb_row(a.bits == 4 && a.group == 32 ? 2 : 1), xs = kWarps * x_frags(a.bits) * 512 / (mt == 1 ? 2 : 1), bars = 8 * 3 * kMaxStages;
-    // K in one chunk: nothing is kept per tile; in several: the tiles' running sums
-    pl->tb = pl->nch == 1 ? tiles_max : std::min(tiles_max, 16 * 1024 / (mt * 512));
+    // K in one chunk: nothing is kept per tile (4096: as far as Walk::groups divides exactly); in several: the tiles' running sums
+    pl->tb = std::min(tiles_max, pl->nch == 1 ? 4096 : 16 * 1024 / (mt * 512));
     const int run = pl->nch == 1 ? 0 : pl->tb * mt * 512;
     // a short K: several tiles per stage keep the warps busy (as many as leave room for two stages)
     for (pl->ts = std::max(1, std::min(kWarps / pl->kbc, tiles_max));; pl->ts--) {

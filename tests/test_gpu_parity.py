@@ -354,3 +354,18 @@ def test_dispatch_rereads_its_parameter_buffer_only_when_it_changed(ctx, plugin,
     v.kernel_destroy(ctx.handle, k)
     for h in (bx, bw, bs, bb, y, want8):
         h.free()
+
+
+def test_more_rows_than_one_pass_of_the_decode_kernel(ctx, oracle):
+    """More than 4096 row tiles per CTA: the CTA passes over its tiles more than once.  The last rows and some around the
+    first pass's end are those of calls on these rows alone."""
+    K, N = 32, 16 * (4096 * 160 + 7) + 5   # (160: more CTAs than the GPU has SMs)
+    rng = np.random.default_rng(5)
+    wq = rng.integers(0, 1 << 32, (N, K // 8), dtype=np.uint32)
+    s = oracle.to_bf16(rng.uniform(0.005, 0.02, (N, 1)).astype(np.float32))
+    b = oracle.to_bf16(rng.uniform(-0.1, 0.1, (N, 1)).astype(np.float32))
+    x = oracle.make_x(2, K, oracle.BF16, config_id=3)
+    y, _ = run_qmatmul(ctx, x, wq, s, b, 4, 32, BF16)
+    for lo in (0, 16 * 4096 - 64, 16 * 4096 * 2, N // 2 // 8 * 8, (N - 500) // 8 * 8):
+        part, _ = run_qmatmul(ctx, x, wq[lo:lo + 500], s[lo:lo + 500], b[lo:lo + 500], 4, 32, BF16)
+        assert np.array_equal(y[:, lo:lo + 500], part)
