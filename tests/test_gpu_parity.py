@@ -369,3 +369,49 @@ def test_more_rows_than_one_pass_of_the_decode_kernel(ctx, oracle):
     for lo in (0, 16 * 4096 - 64, 16 * 4096 * 2, N // 2 // 8 * 8, (N - 500) // 8 * 8):
         part, _ = run_qmatmul(ctx, x, wq[lo:lo + 500], s[lo:lo + 500], b[lo:lo + 500], 4, 32, BF16)
         assert np.array_equal(y[:, lo:lo + 500], part)
+
+
+def _off(ctx, a, shift):
+    """`a` on the device, `shift` bytes past a 16-byte boundary (0: as it is)."""
+    room = ctx.upload(np.concatenate([np.zeros(shift, np.uint8), np.frombuffer(a.tobytes(), np.uint8)]))
+    return room, ctx.wrap(room.device_ptr + shift, a.nbytes, a.shape, a.dtype)
+
+
+@pytest.mark.parametrize("bits,group", [(b, g) for b in (4, 8) for g in (32, 64, 128)])
+@pytest.mark.parametrize("sbd", [BF16, F32])
+def test_requantisation_bit_exact(ctx, oracle, bits, group, sbd):
+    """quantize and dequantize against the oracle, bit for bit: sizes around the kernels' blocks, quotients on and next to
+    halves, constant groups, scales that leave the range of their reciprocal or of bf16, and buffers off the 16-byte grid."""
+    rng = np.random.default_rng(bits * group + sbd)
+    for N, K in ((1, group), (3, 5 * group), (37, 9 * group), (64, 512)):
+        w = (rng.standard_normal((N, K)) * 0.05 + 0.01).astype(np.float32)
+        flat = w.reshape(-1, group)
+        qmax = (1 << bits) - 1
+        for i, row in enumerate(flat):
+            kind = i % 8
+            if kind in (1, 2):      # quotients k + 1/2, and their neighbours
+                step = np.float32((1.0, 3.0)[kind - 1])
+                row[:] = (rng.integers(0, qmax, group) + 0.5).astype(np.float32) * step
+                row[1::3] = np.nextafter(row[1::3], np.float32(np.inf))
+                row[2::3] = np.nextafter(row[2::3], np.float32(-np.inf))
+                row[0], row[-1] = 1e-30, qmax * step
+            elif kind == 3:
+                row[:] = 0.25
+            elif kind == 4:         # reciprocal of the scale overflows, the scale is subnormal or zero in bf16
+                row[:] = np.linspace(0, 1, group, dtype=np.float32) * np.float32(10.0 ** -(37 + i % 4 * 2)) + np.float32(1e-45)
+            elif kind == 5:
+                row[:] = np.linspace(-1, 1, group, dtype=np.float32) * np.float32(1.5e38)
+            elif kind == 6:
+                row[:] = np.linspace(-1, 1, group, dtype=np.float32) * np.float32(3e37)
+        for shift in (0, 4):
+            wq, s, b = oracle.quantize(w, bits, group, sbd)
+            keep, bi = _off(ctx, w, shift)
+            bw, bs, bb = (ctx.empty(a.shape, a.dtype) for a in (wq, s, b))
+            ctx.quantize(bi, bw, bs, bb, N, K, bits, group, sbd)
+            assert np.array_equal(bs.to_host(), s) and np.array_equal(bb.to_host(), b)
+            assert np.array_equal(bw.to_host(), wq)
+            keep2, bw = _off(ctx, wq, shift)
+            for od in ((BF16, F32) if sbd == BF16 else (F32,)):
+                out = ctx.empty((N, K), np.uint16 if od == BF16 else np.float32)
+                ctx.dequantize(bw, bs, bb, out, N, K, bits, group, sbd, od)
+                assert np.array_equal(out.to_host().view(np.uint8), oracle.dequantize(wq, s, b, K, bits, group, od).view(np.uint8))
