@@ -1,28 +1,17 @@
-// Quantized GEMV on CUDA cores: y[M,N] = x[M,K] . dequant(Wq[N,K])^T for the
-// fp32 compute path (x fp32; w^ = fl32(fl32(s*q)+b)) and as the general
-// fallback of the bf16 path (w^ = one bf16 FMA) for shapes the tensor-core
-// kernels do not take.
-//
-// One warp owns R consecutive rows of W.  Per step every lane fetches one
-// 16-byte piece of each row (32 four-bit or 16 eight-bit weights, all inside
-// one quantisation group), dequantises it once, and reuses it for MB rows of
-// x; x comes through L1 (it is tiny and read by every warp).  The K-sum of a
-// row is split over the 32 lanes and finished with warp shuffles.  HBM-bound:
-// algorithmic bytes per row = K*bits/8 + 2*(K/group)*sizeof(scale).
+// Quantized matmul on CUDA cores: y[M,N] = x[M,K] . dequant(Wq[N,K])^T.
+//   qmv_f32_kernel   the fp32 compute path (x fp32; w^ = fl32(fl32(s*q)+b));
+//   qmv_simt_kernel  the bf16 path (w^ = one bf16 FMA) for what the tensor-core kernels do not take (index ranges past
+//                    their 32-bit limits).
+// HBM-bound with few rows of x: algorithmic bytes per row of W = K*bits/8 + 2*(K/group)*sizeof(scale).
 #include <cuda_bf16.h>
+
+#include <algorithm>
 
 #include "internal.h"
 
 namespace luxcuda {
 
 namespace {
-
-template <bool BF16>
-struct XT;
-template <>
-struct XT<false> { using type = float; };
-template <>
-struct XT<true> { using type = __nv_bfloat16; };
 
 __device__ __forceinline__ uint4 ldg_stream(const uint4* p) {
     uint4 r;
@@ -32,42 +21,32 @@ __device__ __forceinline__ uint4 ldg_stream(const uint4* p) {
     return r;
 }
 
-
-// PER consecutive activations (PER*sizeof(X) bytes, naturally aligned) as fp32
-template <int PER, bool XBF16>
+// ---- bf16 -----------------------------------------------------------------------------------------------------------
+// One warp owns R consecutive rows of W.  Per step every lane fetches one 16-byte piece of each row (32 four-bit or 16
+// eight-bit weights, all inside one quantisation group), dequantises it once, and reuses it for MB rows of x.
+// PER consecutive activations (naturally aligned) as fp32
+template <int PER>
 __device__ __forceinline__ void load_x(const void* p, float* out) {
-    if (XBF16) {
-        uint32_t v[PER / 2];
-        if (PER == 8) {
-            const uint4 t = __ldg((const uint4*)p);
-            v[0] = t.x; v[1] = t.y; v[PER / 2 - 2] = t.z; v[PER / 2 - 1] = t.w;
-        } else {
-            const uint2 t = __ldg((const uint2*)p);
-            v[0] = t.x; v[1] = t.y;
-        }
-#pragma unroll
-        for (int i = 0; i < PER / 2; i++) {
-            out[2 * i] = __uint_as_float(v[i] << 16);
-            out[2 * i + 1] = __uint_as_float(v[i] & 0xFFFF0000u);
-        }
+    uint32_t v[PER / 2];
+    if (PER == 8) {
+        const uint4 t = __ldg((const uint4*)p);
+        v[0] = t.x; v[1] = t.y; v[PER / 2 - 2] = t.z; v[PER / 2 - 1] = t.w;
     } else {
+        const uint2 t = __ldg((const uint2*)p);
+        v[0] = t.x; v[1] = t.y;
+    }
 #pragma unroll
-        for (int i = 0; i < PER / 4; i++) {
-            const float4 t = __ldg((const float4*)p + i);
-            out[4 * i] = t.x; out[4 * i + 1] = t.y; out[4 * i + 2] = t.z; out[4 * i + 3] = t.w;
-        }
+    for (int i = 0; i < PER / 2; i++) {
+        out[2 * i] = __uint_as_float(v[i] << 16);
+        out[2 * i + 1] = __uint_as_float(v[i] & 0xFFFF0000u);
     }
 }
 
-// BITS in {4,8}; XBF16: compute dtype; R rows per warp; MB x-rows per pass
-template <int BITS, bool XBF16, int R, int MB>
+template <int BITS, int R, int MB>
 __global__ void __launch_bounds__(256)
-qmv_simt_kernel(const void* __restrict__ xv, const uint32_t* __restrict__ wq, const void* __restrict__ scales,
-                const void* __restrict__ biases, void* __restrict__ yv, int M, int K, int N, int group,
-                int sb_dtype, int y_dtype) {
-    using X = typename XT<XBF16>::type;
+qmv_simt_kernel(const __nv_bfloat16* __restrict__ x, const uint32_t* __restrict__ wq, const __nv_bfloat16* __restrict__ scales,
+                const __nv_bfloat16* __restrict__ biases, void* __restrict__ yv, int M, int K, int N, int group, int y_dtype) {
     constexpr int KP = 128 / BITS;  // weights per 16-byte piece
-    const X* x = (const X*)xv;
     const int lane = threadIdx.x & 31;
     const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int n0 = warp * R;
@@ -85,19 +64,14 @@ qmv_simt_kernel(const void* __restrict__ xv, const uint32_t* __restrict__ wq, co
     for (int p = lane; p < pieces; p += 32) {
         const int k0 = p * KP;
         uint4 wv[R];
-        float s[R], b[R];
+        __nv_bfloat16 s[R], b[R];
 #pragma unroll
         for (int r = 0; r < R; r++) {
             const int n = min(n0 + r, N - 1);
             wv[r] = ldg_stream((const uint4*)(wq + (size_t)n * wpr) + p);
             const size_t gi = (size_t)n * gpr + k0 / group;
-            if (sb_dtype == LUX_DTYPE_BFLOAT16) {
-                s[r] = __bfloat162float(((const __nv_bfloat16*)scales)[gi]);
-                b[r] = __bfloat162float(((const __nv_bfloat16*)biases)[gi]);
-            } else {
-                s[r] = ((const float*)scales)[gi];
-                b[r] = ((const float*)biases)[gi];
-            }
+            s[r] = scales[gi];
+            b[r] = biases[gi];
         }
 #pragma unroll
         for (int w = 0; w < 4; w++) {
@@ -106,8 +80,7 @@ qmv_simt_kernel(const void* __restrict__ xv, const uint32_t* __restrict__ wq, co
 #pragma unroll
             for (int m = 0; m < MB; m++) {
                 const int mm = min(m0 + m, M - 1);
-                const X* xp = x + (size_t)mm * K + k0 + w * PER;
-                load_x<PER, XBF16>(xp, xr[m]);
+                load_x<PER>(x + (size_t)mm * K + k0 + w * PER, xr[m]);
             }
 #pragma unroll
             for (int r = 0; r < R; r++) {
@@ -115,13 +88,7 @@ qmv_simt_kernel(const void* __restrict__ xv, const uint32_t* __restrict__ wq, co
 #pragma unroll
                 for (int j = 0; j < PER; j++) {
                     const uint32_t q = (word >> (BITS * j)) & ((1u << BITS) - 1);
-                    float wf;
-                    if (XBF16) {
-                        wf = __bfloat162float(__hfma(__float2bfloat16_rn((float)q), __float2bfloat16_rn(s[r]),
-                                                     __float2bfloat16_rn(b[r])));
-                    } else {
-                        wf = __fadd_rn(__fmul_rn(s[r], (float)q), b[r]);
-                    }
+                    const float wf = __bfloat162float(__hfma(__float2bfloat16_rn((float)q), s[r], b[r]));
 #pragma unroll
                     for (int m = 0; m < MB; m++) acc[r][m] = fmaf(xr[m][j], wf, acc[r][m]);
                 }
@@ -143,31 +110,233 @@ qmv_simt_kernel(const void* __restrict__ xv, const uint32_t* __restrict__ wq, co
         }
 }
 
-template <int BITS, bool XBF16, int R, int MB>
+template <int BITS, int R, int MB>
 cudaError_t launch_one(const QmmArgs& a, cudaStream_t stream) {
     const int warps = (a.N + R - 1) / R;
     dim3 grid((warps + 7) / 8, (a.M + MB - 1) / MB);
-    qmv_simt_kernel<BITS, XBF16, R, MB><<<grid, 256, 0, stream>>>(a.x, a.wq, a.scales, a.biases, a.y, a.M, a.K, a.N,
-                                                                  a.group, a.sb_dtype, a.y_dtype);
+    qmv_simt_kernel<BITS, R, MB><<<grid, 256, 0, stream>>>((const __nv_bfloat16*)a.x, a.wq, (const __nv_bfloat16*)a.scales,
+                                                           (const __nv_bfloat16*)a.biases, a.y, a.M, a.K, a.N, a.group, a.y_dtype);
     return cudaGetLastError();
 }
+template <int BITS>
+cudaError_t launch_bf16(const QmmArgs& a, cudaStream_t stream) {
+    if (a.M == 1) return launch_one<BITS, 4, 1>(a, stream);
+    return a.M == 2 ? launch_one<BITS, 2, 2>(a, stream) : launch_one<BITS, 2, 4>(a, stream);
+}
 
-template <int BITS, bool XBF16>
-cudaError_t launch_bits(const QmmArgs& a, cudaStream_t stream) {
-    const bool wide = a.N >= 16384;
-    if (a.M == 1) return wide ? launch_one<BITS, XBF16, 4, 1>(a, stream) : launch_one<BITS, XBF16, 2, 1>(a, stream);
-    if (a.M == 2) return launch_one<BITS, XBF16, 2, 2>(a, stream);
-    return launch_one<BITS, XBF16, 2, 4>(a, stream);
+// ---- fp32 -----------------------------------------------------------------------------------------------------------
+// A warp computes R rows of W times MB rows of x over its part of K; the kw warps that share these rows take the pieces
+// of K in turn and add up through shared memory, in order.  A piece is V weights for each lane, side by side, so that
+// weights and x are read along their rows.  (A lane reading 32 weights at once needs x 128 bytes from the next lane's,
+// 32 lines per load.)  V = 8 for one or two rows of x (more bytes under way), 4 above, where x is most of what is loaded
+// and a 16-byte load of it must lie side by side.
+// Arithmetic runs on pairs (f32x2): per two weights two shifts, two and-ors (q + 2^23 as bits), the subtraction of 2^23,
+// s*q, + b and one FMA per row of x.
+// Eight 4096 x 4096 layers, 4 bit, group 64, fp32 scales, one row, call by call: 107 us with a lane's 32 weights at once and
+// a launch that waits for the one before it; 82 like this; 61 as programmatic dependents (84 MB: 1.4 TB/s).
+__device__ __forceinline__ uint64_t pack2(uint32_t lo, uint32_t hi) {
+    uint64_t r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "r"(lo), "r"(hi));
+    return r;
+}
+__device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b) {
+    uint64_t r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ uint64_t mul2(uint64_t a, uint64_t b) {
+    uint64_t r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
+    uint64_t r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+constexpr uint32_t kBits2p23 = 0x4B000000u;  // 2^23: or-ing q into it gives the float 2^23 + q
+constexpr uint64_t kMinus2p23x2 = 0xCB000000CB000000ull;
+
+// C values per lane over the 32 lanes -> every lane holds the sum of one of them, number lane >> (5 - log2 C)
+template <int C>
+__device__ __forceinline__ float reduce_warp(float (&v)[C], int lane) {
+    int o = 16;
+#pragma unroll
+    for (int c = C / 2; c >= 1; c /= 2, o /= 2) {
+        const bool up = lane & o;
+#pragma unroll
+        for (int i = 0; i < c; i++) {
+            const float keep = up ? v[i + c] : v[i], send = up ? v[i] : v[i + c];
+            v[i] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+        }
+    }
+#pragma unroll
+    for (; o >= 1; o /= 2) v[0] += __shfl_xor_sync(0xffffffffu, v[0], o);
+    return v[0];
+}
+
+__device__ __forceinline__ uint4 ld_v4(const void* p) {  // through L1, as the output of the launch before (no .nc)
+    uint4 v;
+    asm volatile("ld.global.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p) : "memory");
+    return v;
+}
+constexpr int kF32Warps = 8, kF32Rows = 4;
+// U pieces under way at a time; BLK blocks per SM
+template <int BITS, bool SB16, int V, int MB, int U, int BLK>
+__global__ void __launch_bounds__(kF32Warps * 32, BLK)
+qmv_f32_kernel(const float* x, const unsigned char* __restrict__ wq, const void* __restrict__ scales,
+               const void* __restrict__ biases, void* yv, int M, int K, int N, int gshift, int kw_shift, int y_bf16) {
+    constexpr int R = kF32Rows, WB = V * BITS / 8;  // bytes of weights per lane and piece: 2, 4 or 8
+    constexpr int WW = WB == 8 ? 2 : 1;
+    __shared__ float red[kF32Warps][R * MB];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, kw = 1 << kw_shift, part = warp & (kw - 1);
+    const int n0 = (blockIdx.x * (kF32Warps >> kw_shift) + (warp >> kw_shift)) * R, m0 = blockIdx.y * MB;
+    const size_t row_bytes = (size_t)K * BITS / 8, gpr = (size_t)K >> gshift;
+    const int pieces = (K + 32 * V - 1) / (32 * V);
+    uint64_t acc[R][MB];
+#pragma unroll
+    for (int r = 0; r < R; r++)
+#pragma unroll
+        for (int m = 0; m < MB; m++) acc[r][m] = 0;
+    uint32_t w[U][R][WW], s[U][R], b[U][R];
+    auto load_weights = [&](int p0) {
+#pragma unroll
+        for (int u = 0; u < U; u++) {
+            const int k = (p0 + u * kw) * (32 * V) + lane * V;
+#pragma unroll
+            for (int r = 0; r < R; r++) {
+                w[u][r][0] = w[u][r][WW - 1] = 0;
+                s[u][r] = b[u][r] = 0;
+                if (k >= K) continue;  // (past the end: w^ = 0, x = 0)
+                const size_t n = min(n0 + r, N - 1), gi = n * gpr + (k >> gshift);
+                const unsigned char* wp = wq + n * row_bytes + (size_t)k * BITS / 8;
+                if (WB == 2) {
+                    uint16_t t;
+                    asm volatile("ld.global.nc.L1::no_allocate.u16 %0, [%1];" : "=h"(t) : "l"(wp));
+                    w[u][r][0] = t;
+                } else if (WB == 4) {
+                    asm volatile("ld.global.nc.L1::no_allocate.u32 %0, [%1];" : "=r"(w[u][r][0]) : "l"(wp));
+                } else {
+                    asm volatile("ld.global.nc.L1::no_allocate.v2.u32 {%0,%1}, [%2];" : "=r"(w[u][r][0]), "=r"(w[u][r][WW - 1]) : "l"(wp));
+                }
+                if (SB16) {
+                    s[u][r] = (uint32_t)__ldg(static_cast<const uint16_t*>(scales) + gi) << 16;
+                    b[u][r] = (uint32_t)__ldg(static_cast<const uint16_t*>(biases) + gi) << 16;
+                } else {
+                    s[u][r] = __ldg(static_cast<const uint32_t*>(scales) + gi);
+                    b[u][r] = __ldg(static_cast<const uint32_t*>(biases) + gi);
+                }
+            }
+        }
+    };
+    // What precedes the wait touches only weights, scales and biases; behind it the next kernel of a chain may start its
+    // own fetch.
+    if (n0 < N) load_weights(part);
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    if (n0 < N) {
+        for (int p0 = part; p0 < pieces; p0 += kw * U) {
+            if (p0 != part) load_weights(p0);
+            uint64_t xr[MB == 1 ? U : 1][V / 2];
+            auto load_row = [&](int u, int m, uint64_t (&v)[V / 2]) {
+                const int k = (p0 + u * kw) * (32 * V) + lane * V;
+#pragma unroll
+                for (int i = 0; i < V / 2; i += 2) {
+                    uint4 t = make_uint4(0, 0, 0, 0);
+                    if (k < K) t = ld_v4(x + (size_t)min(m0 + m, M - 1) * K + k + 2 * i);
+                    v[i] = pack2(t.x, t.y);
+                    v[i + 1] = pack2(t.z, t.w);
+                }
+            };
+            if (MB == 1) {
+#pragma unroll
+                for (int u = 0; u < U; u++) load_row(u, 0, xr[MB == 1 ? u : 0]);
+            }
+#pragma unroll
+            for (int u = 0; u < U; u++) {
+                uint64_t wd[R][V / 2];
+#pragma unroll
+                for (int r = 0; r < R; r++) {
+                    const uint64_t s2 = pack2(s[u][r], s[u][r]), b2 = pack2(b[u][r], b[u][r]);
+#pragma unroll
+                    for (int i = 0; i < V / 2; i++) {
+                        constexpr uint32_t mask = (1u << BITS) - 1;
+                        const int bit = 2 * i * BITS;
+                        const uint32_t word = w[u][r][bit / 32 & (WW - 1)];
+                        const uint64_t q2 = pack2((word >> bit % 32 & mask) | kBits2p23, (word >> (bit + BITS) % 32 & mask) | kBits2p23);
+                        wd[r][i] = add2(mul2(s2, add2(q2, kMinus2p23x2)), b2);
+                    }
+                }
+#pragma unroll
+                for (int m = 0; m < MB; m++) {
+                    uint64_t xv[V / 2];
+                    if (MB > 1) load_row(u, m, xv);
+#pragma unroll
+                    for (int i = 0; i < V / 2; i++)
+#pragma unroll
+                        for (int r = 0; r < R; r++) acc[r][m] = fma2(MB > 1 ? xv[i] : xr[MB == 1 ? u : 0][i], wd[r][i], acc[r][m]);
+                }
+            }
+        }
+    }
+    float v[R * MB];
+#pragma unroll
+    for (int r = 0; r < R; r++)
+#pragma unroll
+        for (int m = 0; m < MB; m++) v[m * R + r] = __uint_as_float((uint32_t)acc[r][m]) + __uint_as_float((uint32_t)(acc[r][m] >> 32));
+    constexpr int LPV = 32 / (R * MB);  // lanes that hold the same value
+    const float sum = reduce_warp<R * MB>(v, lane);
+    if (lane % LPV == 0) red[warp][lane / LPV] = sum;
+    __syncthreads();
+    for (int i = threadIdx.x; i < (kF32Warps >> kw_shift) * R * MB; i += kF32Warps * 32) {
+        const int g = i / (R * MB), j = i % (R * MB), n = (blockIdx.x * (kF32Warps >> kw_shift) + g) * R + j % R, m = m0 + j / R;
+        if (n >= N || m >= M) continue;
+        float t = red[g << kw_shift][j];
+        for (int q = 1; q < kw; q++) t += red[(g << kw_shift) + q][j];
+        const size_t idx = (size_t)m * N + n;
+        if (y_bf16) static_cast<__nv_bfloat16*>(yv)[idx] = __float2bfloat16_rn(t);
+        else static_cast<float*>(yv)[idx] = t;
+    }
+}
+
+template <int BITS, bool SB16, int V, int MB, int U, int BLK>
+cudaError_t launch_f32_one(const QmmArgs& a, cudaStream_t stream, bool overlap_prev) {
+    const int groups = (a.N + kF32Rows - 1) / kF32Rows, gy = (a.M + MB - 1) / MB, pieces = (a.K + 32 * V - 1) / (32 * V);
+    // K is split over the warps of a block as long as the launch is a single wave and each has a round of pieces
+    int kw_shift = 0;
+    while (kw_shift < 3 && (long long)groups * gy << (kw_shift + 1) <= BLK * kF32Warps * kGridCapSMs && pieces > U << kw_shift) kw_shift++;
+    const int per_block = kF32Warps >> kw_shift;
+    if (gy > 65535) return cudaErrorInvalidConfiguration;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((groups + per_block - 1) / per_block, gy);
+    cfg.blockDim = dim3(kF32Warps * 32);
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = overlap_prev ? 1 : 0;
+    return cudaLaunchKernelEx(&cfg, qmv_f32_kernel<BITS, SB16, V, MB, U, BLK>, (const float*)a.x, (const unsigned char*)a.wq,
+                              (const void*)a.scales, (const void*)a.biases, (void*)a.y, a.M, a.K, a.N,
+                              a.group == 32 ? 5 : (a.group == 64 ? 6 : 7), kw_shift, (int)(a.y_dtype == LUX_DTYPE_BFLOAT16));
+}
+template <int BITS, bool SB16>
+cudaError_t launch_f32(const QmmArgs& a, cudaStream_t stream, bool overlap_prev) {
+    if (a.M == 1) return launch_f32_one<BITS, SB16, 8, 1, 2, 4>(a, stream, overlap_prev);
+    if (a.M == 2) return launch_f32_one<BITS, SB16, 8, 2, 2, 2>(a, stream, overlap_prev);
+    return a.M <= 4 ? launch_f32_one<BITS, SB16, 4, 4, 2, 2>(a, stream, overlap_prev)
+                    : launch_f32_one<BITS, SB16, 4, 8, 1, 2>(a, stream, overlap_prev);
 }
 
 }  // namespace
 
-cudaError_t launch_qmv_simt(const QmmArgs& a, cudaStream_t stream, const char** name) {
-    const bool xbf16 = a.x_dtype == LUX_DTYPE_BFLOAT16;
+cudaError_t launch_qmv_simt(const QmmArgs& a, cudaStream_t stream, const char** name, bool overlap_prev) {
+    const bool xbf16 = a.x_dtype == LUX_DTYPE_BFLOAT16, sb16 = a.sb_dtype == LUX_DTYPE_BFLOAT16;
     if (name) *name = xbf16 ? (a.bits == 4 ? "qmv_simt<4,bf16>" : "qmv_simt<8,bf16>")
                             : (a.bits == 4 ? "qmv_simt<4,f32>" : "qmv_simt<8,f32>");
-    if (a.bits == 4) return xbf16 ? launch_bits<4, true>(a, stream) : launch_bits<4, false>(a, stream);
-    return xbf16 ? launch_bits<8, true>(a, stream) : launch_bits<8, false>(a, stream);
+    if (xbf16) return a.bits == 4 ? launch_bf16<4>(a, stream) : launch_bf16<8>(a, stream);
+    if (a.bits == 4) return sb16 ? launch_f32<4, true>(a, stream, overlap_prev) : launch_f32<4, false>(a, stream, overlap_prev);
+    return sb16 ? launch_f32<8, true>(a, stream, overlap_prev) : launch_f32<8, false>(a, stream, overlap_prev);
 }
 
 }  // namespace luxcuda

@@ -55,7 +55,7 @@ void note_chain_launch(Context* c, const void* out, size_t out_bytes) {
 }
 bool decode_may_overlap(const Context* c, const QmmArgs& a) {
     if (!chain_is_open(c)) return false;
-    const size_t sb = (size_t)a.N * (a.K / a.group) * 2;
+    const size_t sb = (size_t)a.N * (a.K / a.group) * dtype_size(a.sb_dtype);
     return !ranges_overlap((const char*)a.wq, (size_t)a.N * a.K * a.bits / 8, c->chain_out_lo, c->chain_out_hi) &&
            !ranges_overlap((const char*)a.scales, sb, c->chain_out_lo, c->chain_out_hi) &&
            !ranges_overlap((const char*)a.biases, sb, c->chain_out_lo, c->chain_out_hi);
@@ -151,7 +151,12 @@ LuxBackendError qmatmul_on_stream(Context* c, const QmmArgs& a) {
             }
         }
     } else {
-        e = launch_qmv_simt(a, c->stream, &name);
+        launches = 0;
+        e = launch_qmv_simt(a, c->stream, &name, decode_may_overlap(c, a));
+        if (e == cudaSuccess) {
+            c->launches++;
+            note_decode_launch(c, a);
+        }
     }
     if (e != cudaSuccess) return map_cuda_error(e, name);
     c->last_kernel = name;

@@ -141,6 +141,50 @@ def test_fp32_compute(ctx, oracle, M, K, N, bits, group):
     check(oracle, y2, x, wq, s16, b16, bits, group, oracle.F32)
 
 
+@pytest.mark.parametrize("bits,group", [(4, 32), (4, 64), (8, 32), (8, 128)])
+@pytest.mark.parametrize("M", [1, 2, 3, 4, 5, 9, 33])
+def test_fp32_edges(ctx, oracle, bits, group, M):
+    """fp32 path: every number of rows per pass and its remainder; K below, at and past a lane's piece, a warp's round and
+    the split over the warps of a block; N off the four rows of a warp; bf16 and fp32 scales.  Bound: fp32 sums of K terms
+    in any order differ from the exact sum by at most K * 2^-24 of the sum of magnitudes."""
+    for K, N in ((group, 1), (group * 3, 7), (1024, 37), (256 * 33 // group * group, 5)):
+        for dt in (oracle.F32, oracle.BF16):
+            wq, s, b = oracle.make_layer(N, K, bits, group, dt, config_id=11, layer=K, proj=N)
+            x = oracle.make_x(M, K, oracle.F32, config_id=11, tag=M)
+            y, kern = run_qmatmul(ctx, x, wq, s, b, bits, group, F32)
+            assert kern.startswith("qmv_simt") and kern.endswith("f32>")
+            if dt == oracle.BF16:
+                s, b = oracle.from_bf16(s), oracle.from_bf16(b)
+            w = oracle.dequantize(wq, s, b, K, bits, group, oracle.F32).astype(np.float64)
+            t, mag = x.astype(np.float64) @ w.T, np.abs(x).astype(np.float64) @ np.abs(w).T
+            assert (np.abs(y - t) <= K * 2.0 ** -24 * mag + 1e-30).all()
+
+
+def test_fp32_launches_back_to_back(ctx, oracle):
+    """fp32 matmuls fed by one another without a synchronisation (each fetches its weights while the one before it runs):
+    the bits of the same calls one at a time."""
+    K = 1024
+    layers = []
+    for i in range(6):
+        wq, s, b = oracle.make_layer(K, K, 4, 64, oracle.F32, config_id=12, layer=i)
+        layers.append([ctx.upload(a) for a in (wq, s, b)])
+    x = ctx.upload(oracle.make_x(2, K, oracle.F32, config_id=12))
+    t = [ctx.empty((2, K), np.float32) for _ in layers]
+
+    def run(sync):
+        h = x
+        for (w, s, b), y in zip(layers, t):
+            ctx.qmatmul(h, w, s, b, y, 2, K, K, 4, 64, F32, F32, F32)
+            if sync:
+                ctx.sync()
+            h = y
+        return h.to_host()
+
+    ref = run(True)
+    for _ in range(10):
+        assert np.array_equal(run(False), ref)
+
+
 def test_fallback_shapes_bf16(ctx, oracle):
     """K not a multiple of the tensor-core k-blocks: the CUDA-core kernel takes over."""
     for (M, K, N, bits, group) in ((3, 192, 20, 4, 64), (2, 64, 7, 8, 64), (20, 96, 33, 4, 32)):
