@@ -60,16 +60,13 @@ constexpr int kStagesB = 3;  // k-stages in flight: B in shared memory, A in TME
 constexpr int kTileN = 128;        // rows of W per tile (MMA M)
 constexpr int kMaxBM = 256;        // rows of x per tile (MMA N)
 constexpr int kSub = 2;            // 64-weight sub-blocks per pipeline stage (one barrier round per 128 k)
-constexpr int kBBytes = kMaxBM * 128;   // one sub-block of B
 constexpr int kEpiStageBytes = 16 * 32 * 2;  // per epilogue warp: 16 rows of y x 32 columns, bf16
 constexpr int kWUnitBytes = kTileN * 64;  // one unit of packed weights: 128 rows x 64 bytes (128 k at 4 bit, 64 k at 8 bit)
 constexpr int kEpiWarps = 8, kDqGroups = 3, kDqWarps = 4 * kDqGroups;
-// A dequantising group goes from stage s straight to stage s + kDqGroups.  Its wait for that slot is by
-// phase parity, which cannot tell "freed once more" from "two frees behind": the group must never be able
-// to get two ring rounds ahead of the MMA, i.e. kDqGroups <= kStagesB.
-static_assert(kDqGroups <= kStagesB, "parity waits would alias");
-constexpr int kTmaWarp = kEpiWarps + kDqWarps, kMmaWarp = kTmaWarp + 1;
-constexpr int kNumThreads = (kMmaWarp + 1) * 32;
+constexpr int kMaxWSlots = 4;  // weight units in flight per dequantising group, at most (p.w_slots)
+static_assert(kDqGroups == kStagesB, "a group always owns the same slot (and its waits, by parity, cannot alias)");
+constexpr int kTmaWarp = kEpiWarps + kDqWarps, kMmaWarp = kTmaWarp + 1, kWWarp = kMmaWarp + 1;
+constexpr int kNumThreads = (kWWarp + 1) * 32;
 constexpr uint32_t kTmemCols = 512, kAColBase = 256, kAColsPerSub = kBK / 2, kAColsPerSlot = kSub * kAColsPerSub;
 constexpr uint32_t kSpinLimit = 1u << 20;
 constexpr size_t kWsFlagBytes = 1024;  // flag words of the stream-K workspace (one per CTA), ahead of the partials
@@ -86,8 +83,9 @@ __device__ __forceinline__ void mbar_expect_tx(uint64_t* b, uint32_t bytes) {
 }
 __device__ __forceinline__ bool mbar_try(uint64_t* b, uint32_t parity) {
     uint32_t ok;
-    asm volatile("{ .reg .pred p; mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2; selp.u32 %0, 1, 0, p; }"
-                 : "=r"(ok) : "r"(s32(b)), "r"(parity) : "memory");
+    // (the hint, in ns, lets the hardware hold a waiting warp instead of having it poll: polls take issue slots)
+    asm volatile("{ .reg .pred p; mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3; selp.u32 %0, 1, 0, p; }"
+                 : "=r"(ok) : "r"(s32(b)), "r"(parity), "r"(20000u) : "memory");
     return ok != 0;
 }
 // Bounded wait.  Returns false (and raises *abort_flag) when the barrier does not
@@ -102,23 +100,20 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* b, uint32_t parity, volatile
     return false;
 }
 
-// One look at a barrier, never suspended: the answer comes back some hundred cycles later, which the caller
-// can spend on other instructions.
-__device__ __forceinline__ bool mbar_test_addr(uint32_t bar, uint32_t parity) {
-    uint32_t ok;
-    asm volatile("{ .reg .pred p; mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2; selp.u32 %0, 1, 0, p; }"
-                 : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
-    return ok != 0;
-}
-
-// Same bound, no back-off: for the one thread whose wake-up latency is on the tensor pipe's critical path.
-__device__ __forceinline__ bool mbar_wait_spin(uint64_t* b, uint32_t parity, volatile int* abort_flag) {
+// Same bound, no back-off, for the warp whose wake-up latency is on the tensor pipe's critical path.  Whole warp; the vote
+// makes the answer, and with it the control flow behind it, uniform for the compiler.
+__device__ __forceinline__ bool mbar_wait_warp(uint64_t* b, uint32_t parity, volatile int* abort_flag) {
     for (uint32_t i = 0; i < kSpinLimit * 8; i++) {
-        if (mbar_try(b, parity)) return true;
-        if ((i & 4095u) == 4095u && *abort_flag) return false;
+        if (__all_sync(0xffffffffu, mbar_try(b, parity))) return true;
+        if ((i & 4095u) == 4095u && __any_sync(0xffffffffu, *abort_flag != 0)) return false;
     }
     *abort_flag = 1;
     return false;
+}
+__device__ __forceinline__ bool elect_one() {  // whole warp: true in one lane, always the same
+    uint32_t r;
+    asm volatile("{ .reg .pred p; elect.sync _|p, 0xffffffff; selp.u32 %0, 1, 0, p; }" : "=r"(r));
+    return r != 0;
 }
 
 // ---- tcgen05 / TMEM ------------------------------------------------------------
@@ -141,29 +136,12 @@ __device__ __forceinline__ void tc_mma_ts(uint32_t d_tmem, uint32_t a_tmem, uint
         "  tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p; }"
         ::"r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate) : "memory");
 }
-// The same with the B descriptor as two words:
-// only the low one, which holds the address, changes between calls.
-__device__ __forceinline__ void tc_mma_ts_acc(uint32_t d_tmem, uint32_t a_tmem, uint32_t b_lo, uint32_t b_hi, uint32_t idesc) {
+// 16 consecutive 32-bit columns of this thread's TMEM lane <- 16 registers
+__device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&r)[16]) {
     asm volatile(
-        "{ .reg .pred p; .reg .b64 bd; setp.eq.u32 p, 1, 1; mov.b64 bd, {%2, %3};\n"
-        "  tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], bd, %4, p; }"
-        ::"r"(d_tmem), "r"(a_tmem), "r"(b_lo), "r"(b_hi), "r"(idesc) : "memory");
-}
-__device__ __forceinline__ void tc_mma_ts_first(uint32_t d_tmem, uint32_t a_tmem, uint32_t b_lo, uint32_t b_hi, uint32_t idesc, uint32_t accumulate) {
-    asm volatile(
-        "{ .reg .pred p; .reg .b64 bd; setp.ne.b32 p, %5, 0; mov.b64 bd, {%2, %3};\n"
-        "  tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], bd, %4, p; }"
-        ::"r"(d_tmem), "r"(a_tmem), "r"(b_lo), "r"(b_hi), "r"(idesc), "r"(accumulate) : "memory");
-}
-// 32 consecutive 32-bit columns of this thread's TMEM lane <- 32 registers
-__device__ __forceinline__ void tmem_st32(uint32_t taddr, const uint32_t (&r)[32]) {
-    asm volatile(
-        "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], "
-        "{%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31,%32};"
+        "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};"
         ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]),
-          "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]), "r"(r[16]), "r"(r[17]),
-          "r"(r[18]), "r"(r[19]), "r"(r[20]), "r"(r[21]), "r"(r[22]), "r"(r[23]), "r"(r[24]), "r"(r[25]), "r"(r[26]),
-          "r"(r[27]), "r"(r[28]), "r"(r[29]), "r"(r[30]), "r"(r[31]) : "memory");
+          "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]) : "memory");
 }
 __device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&r)[32]) {
@@ -220,6 +198,7 @@ struct GemmParams {
     int world, ld, col0;     // copies of y to write (1 unless column-sharded), their row stride and this rank's first column
     void* y_all[kMaxShardWorld];
     int bm;                  // rows of x per tile (multiple of 16, <= 256)
+    int w_slots;             // weight units in flight per dequantising group
     int n_tiles, m_tiles;
     float* ws;               // partial accumulators of tiles shared between CTAs: [CTA][bm][128] fp32
     int y_tma;               // pair kernel: y leaves through shared memory; 1: by a TMA store (bf16, one copy of y, N % 8 == 0),
@@ -262,19 +241,10 @@ __device__ __forceinline__ int cta_of_unit(long long u, long long total_units) {
 }
 
 struct SmemLayout {
-    uint64_t full[kStagesB], empty[kStagesB], wfull[kDqGroups], tmem_full, tmem_empty;
+    uint64_t full[kStagesB], empty[kStagesB], wfull[kDqGroups * kMaxWSlots], wempty[kDqGroups * kMaxWSlots], tmem_full, tmem_empty;
     uint32_t tmem_base;
     int abort_flag;
 };
-
-// Barrier `id` over 128 threads that also ANDs a predicate: every participant gets the same answer.
-__device__ __forceinline__ bool group_all(int id, bool pred) {
-    uint32_t r;
-    asm volatile(
-        "{ .reg .pred p, q; setp.ne.u32 q, %1, 0; bar.red.and.pred p, %2, 128, q; selp.u32 %0, 1, 0, p; }"
-        : "=r"(r) : "r"((uint32_t)pred), "r"(id) : "memory");
-    return r != 0;
-}
 
 __device__ __forceinline__ uint32_t ldg_u16(const uint16_t* p) {  // zero-extended straight into a 32-bit register
     uint32_t v;
@@ -282,55 +252,255 @@ __device__ __forceinline__ uint32_t ldg_u16(const uint16_t* p) {  // zero-extend
     return v;
 }
 
-// 64 weights of one row (one k-stage) -> 32 registers of bf16 pairs in natural k order
+// 32 weights of one row (one scale) -> 16 registers of bf16 pairs in natural k order.
+// The matrix instruction wants neighbours in k side by side, which dequant.cuh's masks do not yield (they pair weights 4
+// apart, and a byte permute per pair put them in order afterwards: 9 integer operations per 8 weights at 4 bit, 10 at 8
+// bit).  Here a permute comes first.  4 bit: byte i of the word into both halves, one mask, q_2i in the low half and
+// 16 * q_2i+1 in the high one, whose scale is 2^-4 of the low one's: 8 operations.  8 bit: two bytes into the two halves,
+// which is all: 4 operations.  The products are the same (see dequant.cuh for the 2^-133 form).
 template <int BITS, bool FAST>
-__device__ __forceinline__ void dequant_row_stage(const uint32_t* w, uint32_t s0, uint32_t b0, uint32_t s1, uint32_t b1,
-                                                  uint32_t (&out)[32]) {
-    constexpr int WPC = kBK * BITS / 32 / 8;  // packed words per chunk of 8 weights
+__device__ __forceinline__ void dequant_32(const uint32_t* w, uint32_t s_bits, uint32_t b_bits, uint32_t (&out)[16]) {
+    const uint32_t b2 = dup_bf16(b_bits);
+    if (BITS == 4) {
+        const uint32_t s2 = FAST ? imad(s_bits, 0x00010001u, 0x40804280u) : dup_bf16(s_bits);  // FAST: (s * 2^133, s * 2^129)
 #pragma unroll
-    for (int c = 0; c < 8; c++) {
-        const uint32_t s_bits = c < 4 ? s0 : s1, b_bits = c < 4 ? b0 : b1;
-        const uint32_t b2 = dup_bf16(b_bits);
-        if (BITS == 4) {
-            uint32_t r[4];  // r[i] = (w^_i, w^_{i+4})
-            if (FAST) dequant4_fast(w[c], scale_x2_133(s_bits), scale_x2_129(s_bits), b2, r);
-            else dequant4_general(w[c], dup_bf16(s_bits), b2, r);
-            out[4 * c + 0] = prmt(r[0], r[1], 0x5410u);
-            out[4 * c + 1] = prmt(r[2], r[3], 0x5410u);
-            out[4 * c + 2] = prmt(r[0], r[1], 0x7632u);
-            out[4 * c + 3] = prmt(r[2], r[3], 0x7632u);
-        } else {
-            uint32_t r0[2], r1[2];  // (w^_0, w^_2), (w^_1, w^_3) of each word
+        for (int c = 0; c < 4; c++) {
             if (FAST) {
-                const uint32_t s133 = scale_x2_133(s_bits);
-                dequant8_fast(w[c * WPC], s133, b2, r0);
-                dequant8_fast(w[c * WPC + WPC - 1], s133, b2, r1);
+#pragma unroll
+                for (int i = 0; i < 4; i++) out[4 * c + i] = fma_bf16x2(prmt(w[c], 0u, 0x4040u + 0x0101u * i) & 0x00F0000Fu, s2, b2);
             } else {
-                dequant8_general(w[c * WPC], dup_bf16(s_bits), b2, r0);
-                dequant8_general(w[c * WPC + WPC - 1], dup_bf16(s_bits), b2, r1);
+                uint32_t r[4];  // r[i] = (w^_i, w^_{i+4})
+                dequant4_general(w[c], s2, b2, r);
+                out[4 * c + 0] = prmt(r[0], r[1], 0x5410u);
+                out[4 * c + 1] = prmt(r[2], r[3], 0x5410u);
+                out[4 * c + 2] = prmt(r[0], r[1], 0x7632u);
+                out[4 * c + 3] = prmt(r[2], r[3], 0x7632u);
             }
-            out[4 * c + 0] = prmt(r0[0], r0[1], 0x5410u);
-            out[4 * c + 1] = prmt(r0[0], r0[1], 0x7632u);
-            out[4 * c + 2] = prmt(r1[0], r1[1], 0x5410u);
-            out[4 * c + 3] = prmt(r1[0], r1[1], 0x7632u);
+        }
+    } else {
+        const uint32_t s2 = FAST ? scale_x2_133(s_bits) : dup_bf16(s_bits);
+#pragma unroll
+        for (int c = 0; c < 8; c++) {
+            if (FAST) {
+                out[2 * c] = fma_bf16x2(prmt(w[c], 0u, 0x4140u), s2, b2);
+                out[2 * c + 1] = fma_bf16x2(prmt(w[c], 0u, 0x4342u), s2, b2);
+            } else {
+                uint32_t r[2];  // (w^_0, w^_2), (w^_1, w^_3)
+                dequant8_general(w[c], s2, b2, r);
+                out[2 * c] = prmt(r[0], r[1], 0x5410u);
+                out[2 * c + 1] = prmt(r[0], r[1], 0x7632u);
+            }
         }
     }
 }
+
+// ---- roles common to the kernels ----
+// Whole tiles, every `step`-th one from `tile` on (the interface of SegIter).
+struct TileIter {
+    int tile_, step, total, nst;
+    __device__ __forceinline__ bool valid() const { return tile_ < total; }
+    __device__ __forceinline__ int tile() const { return tile_; }
+    __device__ __forceinline__ int s_lo() const { return 0; }
+    __device__ __forceinline__ int s_hi() const { return nst; }
+    __device__ __forceinline__ void next() { tile_ += step; }
+};
+// The CTA's stages are counted 0, 1, 2, ... along its sequence of segments, alike in every role; dequantising group g owns
+// the counts = g (mod kDqGroups).
+//
+// One thread: the packed weights, unit after unit into the ring of the group that owns the stage.  Three stages at a time,
+// one for each group: first units first, so that with a single slot per group no group waits for another's second unit
+// (8 bit).  Every stage is UPS units, so that the rings advance alike; the odd sub-block's partner is announced without a load.
+template <int BITS, class Seg, class RowOf>
+__device__ __forceinline__ void weight_producer(const GemmParams& p, const CUtensorMap* tmap_w, Seg seg, int nks, unsigned char* ring,
+                                                uint64_t* wfull, uint64_t* wempty, volatile int* abort_flag, const RowOf& row_of) {
+    constexpr int UPS = BITS == 8 ? 2 : 1;  // weight units (128 rows x 64 packed bytes) per pipeline stage
+    int row[kDqGroups], stage[kDqGroups], cnt = 0, slot = 0;
+    uint32_t ph = 1;
+    auto flush = [&]() {
+#pragma unroll
+        for (int u = 0; u < UPS; u++) {
+#pragma unroll
+            for (int g = 0; g < kDqGroups; g++) {
+                if (g >= cnt) break;
+                const int i = g * kMaxWSlots + slot;
+                if (!mbar_wait(wempty + i, ph, abort_flag)) return false;
+                if (u == 0 || stage[g] * kSub + u < nks) {
+                    mbar_expect_tx(wfull + i, kWUnitBytes);
+                    tma_load_2d(ring + (g * p.w_slots + slot) * kWUnitBytes, tmap_w, stage[g] * (kSub * kBK * BITS / 8) + u * 64, row[g], wfull + i);
+                } else {
+                    mbar_arrive(wfull + i);
+                }
+            }
+            if (++slot == p.w_slots) { slot = 0; ph ^= 1; }
+        }
+        cnt = 0;
+        return true;
+    };
+    for (; seg.valid(); seg.next()) {
+        const int n0 = row_of(seg.tile()), s_hi = seg.s_hi();
+        for (int st = seg.s_lo(); st < s_hi; st++) {
+#pragma unroll
+            for (int g = 0; g < kDqGroups; g++)
+                if (g == cnt) { row[g] = n0; stage[g] = st; }
+            if (++cnt == kDqGroups && !flush()) return;
+        }
+    }
+    flush();
+}
+// One warp (lane quarter of group grp; a warp may only touch its own quarter of the TMEM lanes): the thread owns row r of
+// every tile.  There are as many stages in flight as groups, so a group always writes the same slot.
+// What bounds it is its instructions, three such warps to a scheduler, and the instruction caches that all roles share;
+// hence row pointers per tile (a division each), one copy of the code for both sub-blocks, one arrival per warp.
+template <int BITS, class Seg, class RowOf, class Arrive>
+__device__ __forceinline__ void dequant_role(const GemmParams& p, Seg seg, int grp, int r, int nks, const unsigned char* wring, uint64_t* wfull,
+                                             uint64_t* wempty, uint64_t* empty, uint32_t a_tmem, volatile int* abort_flag,
+                                             const RowOf& row_of, const Arrive& arrive) {
+    constexpr int WPS = kBK * BITS / 32;    // packed words per row per sub-block: 8 | 16
+    constexpr int UPS = BITS == 8 ? 2 : 1;  // weight units (128 rows x 64 packed bytes) per pipeline stage
+    const int gpr = p.K >> p.gshift;
+    const int ng_full = (kSub * kBK) >> p.gshift;  // scale groups per full stage: 4, 2 or 1
+    const bool vec_ok = (gpr % ng_full) == 0;      // then a stage's scales of one row are one aligned vector
+    // row r of a unit in shared memory is 64 bytes, its 16-byte chunk c sits at c ^ ((r >> 1) & 3)
+    const uint32_t wsw = (uint32_t)(r >> 1) & 3u;
+    const unsigned char* wrow0 = wring + r * 64;
+    const uint16_t *srow = nullptr, *brow = nullptr;  // scales / biases of this thread's row of the tile
+    int st, end;
+    bool more = true;
+    auto new_rows = [&]() {
+        const size_t at = (size_t)min(row_of(seg.tile()) + r, p.N - 1) * gpr;
+        srow = reinterpret_cast<const uint16_t*>(p.scales) + at;
+        brow = reinterpret_cast<const uint16_t*>(p.biases) + at;
+    };
+    auto settle = [&]() {  // st lies past the segment's end: the stage as far into the segments after it
+        do {
+            const int over = st - end;
+            seg.next();
+            if (!seg.valid()) {
+                more = false;
+                return;
+            }
+            st = seg.s_lo() + over;
+            end = seg.s_hi();
+        } while (st >= end);
+        new_rows();
+    };
+    uint32_t sp[2], bp[2];  // scales / biases of the next owned stage of this row, bf16 pairs in group order
+    auto fetch_sb = [&]() {
+        const int g0 = (st * kSub * kBK) >> p.gshift;
+        const uint16_t *sr = srow + g0, *br = brow + g0;
+        sp[1] = 0; bp[1] = 0;
+        if (vec_ok && ng_full == 4) {
+            asm volatile("ld.global.nc.v2.u32 {%0,%1}, [%2];" : "=r"(sp[0]), "=r"(sp[1]) : "l"(sr));
+            asm volatile("ld.global.nc.v2.u32 {%0,%1}, [%2];" : "=r"(bp[0]), "=r"(bp[1]) : "l"(br));
+        } else if (vec_ok && ng_full == 2) {
+            asm volatile("ld.global.nc.u32 %0, [%1];" : "=r"(sp[0]) : "l"(sr));
+            asm volatile("ld.global.nc.u32 %0, [%1];" : "=r"(bp[0]) : "l"(br));
+        } else if (ng_full == 4 && (gpr & 1) == 0) {  // (a load is one line per lane: four of pairs, not eight)
+            asm volatile("ld.global.nc.u32 %0, [%1];" : "=r"(sp[0]) : "l"(sr));
+            asm volatile("ld.global.nc.u32 %0, [%1];" : "=r"(bp[0]) : "l"(br));
+            if (gpr - g0 > 2) {
+                asm volatile("ld.global.nc.u32 %0, [%1];" : "=r"(sp[1]) : "l"(sr + 2));
+                asm volatile("ld.global.nc.u32 %0, [%1];" : "=r"(bp[1]) : "l"(br + 2));
+            }
+        } else {
+            const int ng = min(gpr - g0, ng_full);
+            sp[0] = ldg_u16(sr); bp[0] = ldg_u16(br);
+            if (ng > 1) { sp[0] |= ldg_u16(sr + 1) << 16; bp[0] |= ldg_u16(br + 1) << 16; }
+            if (ng > 2) { sp[1] = ldg_u16(sr + 2); bp[1] = ldg_u16(br + 2); }
+            if (ng > 3) { sp[1] |= ldg_u16(sr + 3) << 16; bp[1] |= ldg_u16(br + 3) << 16; }
+        }
+    };
+    if (!seg.valid()) return;
+    st = seg.s_lo() + grp;
+    end = seg.s_hi();
+    if (st >= end) settle();
+    else new_rows();
+    if (more) fetch_sb();
+    const int half_shift = p.gshift == 5 ? 16 : 0, sub_shift = p.gshift == 6 ? 16 : 0;  // where the next half's, the next sub-block's scale is
+    int wslot = 0;
+    uint32_t wphase = 0, phase = 1;
+    while (more) {
+        const int nsub = min(kSub, nks - st * kSub);
+        uint32_t s_lo = sp[0], b_lo = bp[0];
+        const uint32_t s_hi = sp[1], b_hi = bp[1];
+        st += kDqGroups;
+        if (st >= end) settle();
+        // Three stages ahead of its use.  At 4 bit behind the proxy fence, which would wait for these loads too (777 rows in
+        // groups of 32: 30.9 against 33-40 us); at 8 bit, with a fence per sub-block, here (512 x 8192 x 28672: 204 against 257).
+        if (UPS == 2 && more) fetch_sb();
+        uint32_t w[WPS], wn[8];  // this sub-block's words; 4 bit: the next one's, from the same unit
+        bool ok = true;
+#pragma unroll 1
+        for (int u = 0; u < kSub; u++) {
+            if (UPS == 1 && u >= nsub) break;
+            if (UPS == 2 || u == 0) {
+                ok = mbar_wait(wfull + wslot, wphase, abort_flag) && ok;
+                const unsigned char* wrow = wrow0 + wslot * kWUnitBytes;
+#pragma unroll
+                for (int c = 0; c < 4; c++) {
+                    const uint4 v = *reinterpret_cast<const uint4*>(wrow + ((c ^ wsw) << 4));
+                    uint32_t* d = UPS == 2 ? w + (4 * c) % WPS : (c < 2 ? w + 4 * c : wn + 4 * (c - 2));
+                    d[0] = v.x; d[1] = v.y; d[2] = v.z; d[3] = v.w;
+                }
+                // The reads above are generic-proxy accesses, the refill is an async-proxy write: the proxy
+                // fence orders the two (without it a read still in the load pipe could see the next unit).
+                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+                __syncwarp();
+                if ((r & 31) == 0) mbar_arrive(wempty + wslot);
+                if (++wslot == p.w_slots) { wslot = 0; wphase ^= 1; }
+                if (UPS == 1 && more) fetch_sb();
+            }
+            if (u >= nsub) break;  // (the odd sub-block's partner at 8 bit: nothing in it)
+            if (u == 0) {
+                ok = __all_sync(0xFFFFFFFFu, mbar_wait(empty, phase, abort_flag) && ok);  // tcgen05.st below is warp-collective
+                phase ^= 1;
+                tc_fence_after();
+                if (!ok) break;
+            }
+            // the two 32-weight halves of the sub-block: in one group, or (groups of 32) in one each
+#pragma unroll
+            for (int h = 0; h < 2; h++) {
+                const uint32_t sv = (h ? s_lo >> half_shift : s_lo) & 0xFFFFu, bv = (h ? b_lo >> half_shift : b_lo) & 0xFFFFu;
+                uint32_t out[16];
+                if (scale_fast_ok(sv)) dequant_32<BITS, true>(w + h * (WPS / 2), sv, bv, out);
+                else dequant_32<BITS, false>(w + h * (WPS / 2), sv, bv, out);  // whole-block branch: not if-converted
+                __syncwarp();
+                tmem_st16(a_tmem + u * kAColsPerSub + h * 16, out);
+            }
+            if (UPS == 1) {
+#pragma unroll
+                for (int i = 0; i < 8; i++) w[i] = wn[i];
+            }
+            s_lo = half_shift ? s_hi : s_lo >> sub_shift;
+            b_lo = half_shift ? b_hi : b_lo >> sub_shift;
+        }
+        ok = __all_sync(0xFFFFFFFFu, ok);  // (8 bit: the second unit's wait)
+        if (!ok) {
+            *abort_flag = 1;
+            break;
+        }
+        tmem_st_wait();  // once per stage: both sub-blocks are in tensor memory
+        tc_fence_before();
+        __syncwarp();
+        if ((r & 31) == 0) arrive();
+    }
+}
+
 template <int BITS, bool SK>
 __global__ void __launch_bounds__(kNumThreads, 1)
 qmm_tc_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ CUtensorMap tmap_w,
               const __grid_constant__ GemmParams p) {
-    constexpr int WPS = kBK * BITS / 32;  // packed words per row per stage: 8 | 16
     extern __shared__ unsigned char smem_raw[];
     unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
     unsigned char* sB = smem;  // [kStagesB][bm rows][128 B], swizzled (TMA)
     const uint32_t b_bytes = (uint32_t)p.bm * 128;
-    unsigned char* sW = sB + (size_t)kStagesB * kSub * kBBytes;  // [kDqGroups][128 rows][64 B], 64-byte swizzle (TMA)
-    unsigned char* sEpi = sW + (size_t)kDqGroups * kWUnitBytes;  // [kEpiWarps][16 rows of x][32 rows of the tile] bf16: the epilogue's transposer
+    unsigned char* sW = sB + (size_t)kStagesB * kSub * b_bytes;  // [kDqGroups][w_slots][128 rows][64 B], 64-byte swizzle (TMA)
+    unsigned char* sEpi = sW + (size_t)kDqGroups * p.w_slots * kWUnitBytes;  // [kEpiWarps][16 rows of x][32 rows of the tile] bf16: the epilogue's transposer
     SmemLayout* sl = reinterpret_cast<SmemLayout*>(sEpi + (size_t)kEpiWarps * kEpiStageBytes);
     volatile int* abort_flag = &sl->abort_flag;
 
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int tid = threadIdx.x, lane = tid & 31;
+    const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);  // (uniform for the compiler too)
     const int nks = p.K / kBK;                  // 64-weight sub-blocks along K
     const int nst = (nks + kSub - 1) / kSub;    // pipeline stages per tile
     const int total_tiles = p.n_tiles * p.m_tiles;
@@ -338,10 +508,13 @@ qmm_tc_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant_
 
     if (tid == 0) {
         for (int s = 0; s < kStagesB; s++) {
-            mbar_init(&sl->full[s], 128 + 1);  // 128 dequantising threads + the TMA producer (with its byte count)
+            mbar_init(&sl->full[s], 4 + 1);  // the owning group's four warps + the TMA producer (with its byte count)
             mbar_init(&sl->empty[s], 1);        // one tcgen05.commit
         }
-        for (int g = 0; g < kDqGroups; g++) mbar_init(&sl->wfull[g], 1);  // the group leader's expect_tx
+        for (int g = 0; g < kDqGroups * kMaxWSlots; g++) {
+            mbar_init(&sl->wfull[g], 1);   // the weight producer's expect_tx
+            mbar_init(&sl->wempty[g], 4);  // the group's four warps have read their rows
+        }
         mbar_init(&sl->tmem_full, 1);
         mbar_init(&sl->tmem_empty, kEpiWarps * 32);
         sl->abort_flag = 0;
@@ -351,7 +524,7 @@ qmm_tc_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant_
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    const uint32_t tmem_base = sl->tmem_base;
+    const uint32_t tmem_base = __shfl_sync(0xffffffffu, sl->tmem_base, 0);
 
     if (warp == kTmaWarp) {
         // ---------------- TMA producer: x tiles ----------------
@@ -371,186 +544,62 @@ qmm_tc_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant_
                     if (!mbar_wait(&sl->empty[sb], ph ^ 1, abort_flag)) { ok = false; break; }
                     mbar_expect_tx(&sl->full[sb], b_bytes * nsub);
                     for (int u = 0; u < nsub; u++)
-                        tma_load_2d(sB + ((size_t)sb * kSub + u) * kBBytes, &tmap_x, (st * kSub + u) * kBK, m0, &sl->full[sb]);
+                        tma_load_2d(sB + (sb * kSub + u) * b_bytes, &tmap_x, (st * kSub + u) * kBK, m0, &sl->full[sb]);
                 }
             }
         }
     } else if (warp == kMmaWarp) {
         // ---------------- MMA issuer ----------------
-        if (lane == 0) {
+        // The whole warp walks the stages and one elected lane issues: addresses and descriptors then live in uniform
+        // registers, where the MMAs take them from.  (Walked by one lane, each MMA cost about 106 cycles of moves into
+        // them, 850 of the 1210 cycles that a stage took whatever the tile's height; the MMAs of a 256-row tile need 1024.)
+        {
             const uint32_t idesc = umma_idesc(kTileN, p.bm);
             uint32_t tile_i = 0, slot = 0, phase = 0;
             const uint64_t db0 = umma_desc_sw128(s32(sB));
-            const uint32_t b_hi = (uint32_t)(db0 >> 32), b_lo0 = (uint32_t)db0;  // the address is in the low word, 16-byte units
-            const uint32_t a0 = tmem_base + kAColBase, bar0 = s32(&sl->full[0]);
             bool ok = true;
-            // This thread's instructions are the pipeline's critical path (it shares its scheduler with working
-            // warps, and a look at a barrier costs it some hundred cycles even when the phase is long over): the
-            // barrier of the NEXT stage is looked at before the MMAs of the current one are issued, the answer read
-            // after; an MMA is an add or two and the instruction.
-            bool ready = false;
             SegIter<SK> seg;
             for (seg.init(total_units, nst); seg.valid() && ok; seg.next(), tile_i++) {
                 const int s_lo = seg.s_lo(), s_hi = seg.s_hi();
-                if (!mbar_wait(&sl->tmem_empty, (tile_i & 1) ^ 1, abort_flag)) break;
+                if (!mbar_wait_warp(&sl->tmem_empty, (tile_i & 1) ^ 1, abort_flag)) break;
                 tc_fence_after();
                 for (int st = s_lo; st < s_hi; st++) {
-                    if (!ready && !mbar_wait_spin(&sl->full[slot], phase, abort_flag)) { ok = false; break; }
+                    if (!mbar_wait_warp(&sl->full[slot], phase, abort_flag)) { ok = false; break; }
                     tc_fence_after();
-                    uint32_t nslot = slot + 1, nphase = phase;
-                    if (nslot == (uint32_t)kStagesB) { nslot = 0; nphase ^= 1; }
-                    const bool rn = mbar_test_addr(bar0 + 8 * nslot, nphase);  // (past the CTA's last stage: "not yet", and not used)
-                    const uint32_t b_lo = b_lo0 + slot * (uint32_t)(kSub * kBBytes >> 4);
-                    const uint32_t a_tmem = a0 + slot * kAColsPerSlot;
-                    // 16 k per MMA = 8 TMEM columns of A, 32 bytes of each B row
-                    tc_mma_ts_first(tmem_base, a_tmem, b_lo, b_hi, idesc, st != s_lo ? 1u : 0u);
+                    const uint64_t db = db0 + (uint64_t)(slot * (kSub * b_bytes >> 4));
+                    const uint32_t a_tmem = tmem_base + kAColBase + slot * kAColsPerSlot;
+                    if (elect_one()) {
+                        // 16 k per MMA = 8 TMEM columns of A, 32 bytes of each B row
 #pragma unroll
-                    for (int kk = 1; kk < kBK / 16; kk++) tc_mma_ts_acc(tmem_base, a_tmem + 8 * kk, b_lo + 2 * kk, b_hi, idesc);
-                    if (st * kSub + 1 < nks) {  // (the last stage of an odd K has one sub-block)
+                        for (int kk = 0; kk < kBK / 16; kk++) tc_mma_ts(tmem_base, a_tmem + 8 * kk, db + 2 * kk, idesc, (kk > 0 || st != s_lo) ? 1u : 0u);
+                        if (st * kSub + 1 < nks) {  // (the last stage of an odd K has one sub-block)
 #pragma unroll
-                        for (int kk = 0; kk < kBK / 16; kk++)
-                            tc_mma_ts_acc(tmem_base, a_tmem + kAColsPerSub + 8 * kk, b_lo + (kBBytes >> 4) + 2 * kk, b_hi, idesc);
+                            for (int kk = 0; kk < kBK / 16; kk++)
+                                tc_mma_ts(tmem_base, a_tmem + kAColsPerSub + 8 * kk, db + (b_bytes >> 4) + 2 * kk, idesc, 1u);
+                        }
+                        tc_commit(&sl->empty[slot]);  // arrives when the MMAs above have consumed their operands
                     }
-                    tc_commit(&sl->empty[slot]);  // arrives when the MMAs above have consumed their operands
-                    ready = rn;
-                    slot = nslot; phase = nphase;
+                    __syncwarp();
+                    if (++slot == kStagesB) { slot = 0; phase ^= 1; }
                 }
-                if (ok) tc_commit(&sl->tmem_full);
-            }
-        }
-    } else if (warp >= kEpiWarps) {
-        // ---------------- dequantisers: group grp owns the stages = grp (mod kDqGroups); thread owns row n0 + r ----------------
-        constexpr int UPS = BITS == 8 ? 2 : 1;  // weight units (128 rows x 64 packed bytes) per pipeline stage
-        const int q = warp & 3, grp = (warp - kEpiWarps) >> 2;
-        const int r = q * 32 + lane;
-        const bool leader = (q == 0 && lane == 0);
-        const int bar_id = 1 + grp;  // named barrier of the group (0 is __syncthreads)
-        const int gpr = p.K >> p.gshift;
-        const int ng_full = (kSub * kBK) >> p.gshift;  // scale groups per full stage: 4, 2 or 1
-        const bool vec_ok = (gpr % ng_full) == 0;      // then a stage's scales of one row are one aligned vector
-        const uint32_t lane_addr = tmem_base + ((uint32_t)(q * 32) << 16) + kAColBase;
-        // this group's weight unit in shared memory; row r is 64 bytes, its 16-byte chunk c sits at c ^ ((r >> 1) & 3)
-        const unsigned char* wrow = sW + (size_t)grp * kWUnitBytes + r * 64;
-        const uint32_t wsw = (uint32_t)(r >> 1) & 3u;
-        uint64_t* wbar = &sl->wfull[grp];
-        uint32_t wround = 0;  // units of this group consumed so far
-
-        // An owned stage: the CTA's stages are counted 0, 1, 2, ... along its range of units (the same count
-        // the producer and the MMA issuer keep); group grp owns the counts = grp (mod kDqGroups).
-        struct Cur { int tile, st; uint32_t it; };  // tile and stage in the tile of count `it`; tile >= total_tiles: past the end
-        const long long u_lo = SK ? total_units * blockIdx.x / gridDim.x : 0;
-        const uint32_t u_cnt = SK ? (uint32_t)(total_units * (blockIdx.x + 1) / gridDim.x - u_lo)
-                                  : (uint32_t)((total_tiles - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x * nst);
-        const int tile_lo = SK ? (int)(u_lo / nst) : (int)blockIdx.x;  // (the one 64-bit division of the walk)
-        const int st_lo = SK ? (int)(u_lo % nst) : 0;
-        const int tile_step = SK ? 1 : (int)gridDim.x;
-        auto advance = [&](Cur& c, int by) {  // `by` stages further along the CTA's sequence of stages
-            c.it += by;
-            if (c.it >= u_cnt) {
-                c.tile = total_tiles;
-                return;
-            }
-            c.st += by;
-            while (c.st >= nst) {
-                c.st -= nst;
-                c.tile += tile_step;
-            }
-        };
-        auto issue = [&](const Cur& c, int u) {  // leader: bring unit u of stage c into the group's slot
-            mbar_expect_tx(wbar, kWUnitBytes);
-            tma_load_2d(const_cast<unsigned char*>(sW) + (size_t)grp * kWUnitBytes, &tmap_w,
-                        c.st * (kSub * kBK * BITS / 8) + u * 64, (c.tile / p.m_tiles) * kTileN, wbar);
-        };
-        uint32_t sp[2], bp[2];  // scales / biases of the next owned stage of this row, bf16 pairs in group order
-        auto fetch_sb = [&](const Cur& c) {
-            const int n = min((c.tile / p.m_tiles) * kTileN + r, p.N - 1);
-            const int g0 = (c.st * kSub * kBK) >> p.gshift;
-            const int ng = min(gpr - g0, ng_full);
-            const uint16_t* sr = reinterpret_cast<const uint16_t*>(p.scales) + (size_t)n * gpr + g0;
-            const uint16_t* br = reinterpret_cast<const uint16_t*>(p.biases) + (size_t)n * gpr + g0;
-            sp[1] = 0; bp[1] = 0;
-            if (vec_ok && ng == ng_full && ng == 4) {
-                asm volatile("ld.global.nc.v2.u32 {%0,%1}, [%2];" : "=r"(sp[0]), "=r"(sp[1]) : "l"(sr));
-                asm volatile("ld.global.nc.v2.u32 {%0,%1}, [%2];" : "=r"(bp[0]), "=r"(bp[1]) : "l"(br));
-            } else if (vec_ok && ng == ng_full && ng == 2) {
-                asm volatile("ld.global.nc.u32 %0, [%1];" : "=r"(sp[0]) : "l"(sr));
-                asm volatile("ld.global.nc.u32 %0, [%1];" : "=r"(bp[0]) : "l"(br));
-            } else {
-                sp[0] = ldg_u16(sr); bp[0] = ldg_u16(br);
-                if (ng > 1) { sp[0] |= ldg_u16(sr + 1) << 16; bp[0] |= ldg_u16(br + 1) << 16; }
-                if (ng > 2) { sp[1] = ldg_u16(sr + 2); bp[1] = ldg_u16(br + 2); }
-                if (ng > 3) { sp[1] |= ldg_u16(sr + 3) << 16; bp[1] |= ldg_u16(br + 3) << 16; }
-            }
-        };
-
-        Cur cur{tile_lo, st_lo, 0u};
-        advance(cur, grp);
-        if (cur.tile < total_tiles) {
-            if (leader) issue(cur, 0);
-            fetch_sb(cur);
-        }
-        bool ok = true;
-        while (cur.tile < total_tiles) {
-            Cur nxt = cur;
-            advance(nxt, kDqGroups);
-            const uint32_t it = cur.it;
-            const int sa = it % kStagesB;
-            const int nsub = min(kSub, nks - cur.st * kSub);
-            const uint32_t sc[2] = {sp[0], sp[1]}, bc[2] = {bp[0], bp[1]};
-            if (nxt.tile < total_tiles) fetch_sb(nxt);  // three stages ahead of its use
-            uint32_t w[16];
-            bool group_fail = false;
-#pragma unroll
-            for (int u = 0; u < kSub; u++) {
-                if (u >= nsub) break;
-                if (UPS == 2 || u == 0) {
-                    const bool got = ok && mbar_wait(wbar, wround & 1, abort_flag);
-                    wround++;
-#pragma unroll
-                    for (int c = 0; c < 4; c++) {
-                        const uint4 v = *reinterpret_cast<const uint4*>(wrow + ((c ^ wsw) << 4));
-                        w[4 * c] = v.x; w[4 * c + 1] = v.y; w[4 * c + 2] = v.z; w[4 * c + 3] = v.w;
-                    }
-                    // The reads above are generic-proxy accesses, the refill is an async-proxy write: the proxy
-                    // fence orders the two (without it a read still in the load pipe could see the next unit).
-                    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-                    // every thread of the group has its bytes: the slot may be refilled.  The same barrier makes
-                    // a failed wait a decision of the whole group, so nobody is left waiting at it.
-                    ok = group_all(bar_id, got);
-                    if (!ok) { group_fail = true; break; }
-                    if (leader) {
-                        if (UPS == 2 && u + 1 < nsub) issue(cur, u + 1);
-                        else if (nxt.tile < total_tiles) issue(nxt, 0);
-                    }
-                }
-                // scales of the two 32-weight halves of this sub-block
-                const int h0 = (2 * u * 32) >> p.gshift, h1 = ((2 * u + 1) * 32) >> p.gshift;
-                const uint32_t s0 = (sc[h0 >> 1] >> ((h0 & 1) * 16)) & 0xFFFFu, b0 = (bc[h0 >> 1] >> ((h0 & 1) * 16)) & 0xFFFFu;
-                const uint32_t s1 = (sc[h1 >> 1] >> ((h1 & 1) * 16)) & 0xFFFFu, b1 = (bc[h1 >> 1] >> ((h1 & 1) * 16)) & 0xFFFFu;
-                uint32_t out[32];
-                const uint32_t (&ws)[WPS] = *reinterpret_cast<const uint32_t (*)[WPS]>(&w[BITS == 4 ? 8 * u : 0]);
-                if (scale_fast_ok(s0) && scale_fast_ok(s1)) dequant_row_stage<BITS, true>(ws, s0, b0, s1, b1, out);
-                else dequant_row_stage<BITS, false>(ws, s0, b0, s1, b1, out);  // whole-block branch: not if-converted
-                if (u == 0) {
-                    // (every lane waits: with one lane polling for the warp the wake-up came later and the launch
-                    // took 3 % longer)
-                    const bool freed = ok && mbar_wait(&sl->empty[sa], ((it / kStagesB) & 1) ^ 1, abort_flag);
-                    ok = __all_sync(0xFFFFFFFFu, freed);  // tcgen05.st below is warp-collective
-                    tc_fence_after();
-                }
+                if (ok && elect_one()) tc_commit(&sl->tmem_full);
                 __syncwarp();
-                if (ok) tmem_st32(lane_addr + sa * kAColsPerSlot + u * kAColsPerSub, out);
             }
-            if (ok) {
-                tmem_st_wait();  // once per stage: both sub-blocks are in tensor memory
-                tc_fence_before();
-                mbar_arrive(&sl->full[sa]);
-            } else if (!*abort_flag) {
-                *abort_flag = 1;
-            }
-            if (group_fail) break;  // decided by the whole group at its barrier
-            cur = nxt;                // a warp that failed alone goes on to the next barrier, where the group ends
         }
+    } else if (warp == kWWarp) {
+        // ---------------- TMA producer: packed weights ----------------
+        SegIter<SK> seg;
+        seg.init(total_units, nst);
+        if (lane == 0) weight_producer<BITS>(p, &tmap_w, seg, nks, sW, sl->wfull, sl->wempty, abort_flag, [&](int tile) { return (tile / p.m_tiles) * kTileN; });
+    } else if (warp >= kEpiWarps) {
+        // ---------------- dequantisers ----------------
+        const int q = warp & 3, grp = (warp - kEpiWarps) >> 2;
+        SegIter<SK> seg;
+        seg.init(total_units, nst);
+        dequant_role<BITS>(p, seg, grp, q * 32 + lane, nks, sW + (size_t)grp * p.w_slots * kWUnitBytes, &sl->wfull[grp * kMaxWSlots],
+                           &sl->wempty[grp * kMaxWSlots], &sl->empty[grp],
+                           tmem_base + ((uint32_t)(q * 32) << 16) + kAColBase + grp * kAColsPerSlot, abort_flag,
+                           [&](int tile) { return (tile / p.m_tiles) * kTileN; }, [&]() { mbar_arrive(&sl->full[grp]); });
     } else {
         // ---------------- epilogue: warp w reads TMEM lanes 32*(w%4).., half w/4 of the column blocks ----------------
         const int q = warp & 3, half = warp >> 2;
@@ -737,26 +786,29 @@ template <int BITS>
 __global__ void __launch_bounds__(kNumThreads, 1)
 qmm_tc_tiles_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ CUtensorMap tmap_w,
               const __grid_constant__ GemmParams p) {
-    constexpr int WPS = kBK * BITS / 32;  // packed words per row per stage: 8 | 16
     extern __shared__ unsigned char smem_raw[];
     unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
     unsigned char* sB = smem;  // [kStagesB][bm rows][128 B], swizzled (TMA)
     const uint32_t b_bytes = (uint32_t)p.bm * 128;
-    unsigned char* sW = sB + (size_t)kStagesB * kSub * kBBytes;  // [kDqGroups][128 rows][64 B], 64-byte swizzle (TMA)
-    SmemLayout* sl = reinterpret_cast<SmemLayout*>(sW + (size_t)kDqGroups * kWUnitBytes);
+    unsigned char* sW = sB + (size_t)kStagesB * kSub * b_bytes;  // [kDqGroups][w_slots][128 rows][64 B], 64-byte swizzle (TMA)
+    SmemLayout* sl = reinterpret_cast<SmemLayout*>(sW + (size_t)kDqGroups * p.w_slots * kWUnitBytes);
     volatile int* abort_flag = &sl->abort_flag;
 
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int tid = threadIdx.x, lane = tid & 31;
+    const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);  // (uniform for the compiler too)
     const int nks = p.K / kBK;                  // 64-weight sub-blocks along K
     const int nst = (nks + kSub - 1) / kSub;    // pipeline stages per tile
     const int total_tiles = p.n_tiles * p.m_tiles;
 
     if (tid == 0) {
         for (int s = 0; s < kStagesB; s++) {
-            mbar_init(&sl->full[s], 128 + 1);  // 128 dequantising threads + the TMA producer (with its byte count)
+            mbar_init(&sl->full[s], 4 + 1);  // the owning group's four warps + the TMA producer (with its byte count)
             mbar_init(&sl->empty[s], 1);        // one tcgen05.commit
         }
-        for (int g = 0; g < kDqGroups; g++) mbar_init(&sl->wfull[g], 1);  // the group leader's expect_tx
+        for (int g = 0; g < kDqGroups * kMaxWSlots; g++) {
+            mbar_init(&sl->wfull[g], 1);   // the weight producer's expect_tx
+            mbar_init(&sl->wempty[g], 4);  // the group's four warps have read their rows
+        }
         mbar_init(&sl->tmem_full, 1);
         mbar_init(&sl->tmem_empty, kEpiWarps * 32);
         sl->abort_flag = 0;
@@ -766,7 +818,7 @@ qmm_tc_tiles_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_con
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    const uint32_t tmem_base = sl->tmem_base;
+    const uint32_t tmem_base = __shfl_sync(0xffffffffu, sl->tmem_base, 0);
 
     if (warp == kTmaWarp) {
         // ---------------- TMA producer: x tiles ----------------
@@ -784,164 +836,55 @@ qmm_tc_tiles_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_con
                     if (!mbar_wait(&sl->empty[sb], ph ^ 1, abort_flag)) { ok = false; break; }
                     mbar_expect_tx(&sl->full[sb], b_bytes * nsub);
                     for (int u = 0; u < nsub; u++)
-                        tma_load_2d(sB + ((size_t)sb * kSub + u) * kBBytes, &tmap_x, (st * kSub + u) * kBK, m0, &sl->full[sb]);
+                        tma_load_2d(sB + (sb * kSub + u) * b_bytes, &tmap_x, (st * kSub + u) * kBK, m0, &sl->full[sb]);
                 }
             }
         }
     } else if (warp == kMmaWarp) {
-        // ---------------- MMA issuer ----------------
-        if (lane == 0) {
+        // ---------------- MMA issuer (as above: the whole warp, one elected lane) ----------------
+        {
             const uint32_t idesc = umma_idesc(kTileN, p.bm);
             uint32_t tile_i = 0, slot = 0, phase = 0;
             const uint64_t db0 = umma_desc_sw128(s32(sB));
             bool ok = true;
             for (int tile = blockIdx.x; tile < total_tiles && ok; tile += gridDim.x, tile_i++) {
-                if (!mbar_wait(&sl->tmem_empty, (tile_i & 1) ^ 1, abort_flag)) break;
+                if (!mbar_wait_warp(&sl->tmem_empty, (tile_i & 1) ^ 1, abort_flag)) break;
                 tc_fence_after();
                 for (int st = 0; st < nst; st++) {
-                    const int nsub = min(kSub, nks - st * kSub);
-                    if (!mbar_wait_spin(&sl->full[slot], phase, abort_flag)) { ok = false; break; }
+                    if (!mbar_wait_warp(&sl->full[slot], phase, abort_flag)) { ok = false; break; }
                     tc_fence_after();
-                    for (int u = 0; u < nsub; u++) {
-                        const uint64_t db = db0 + (uint64_t)(slot * kSub + u) * (kBBytes >> 4);
-                        const uint32_t a_tmem = tmem_base + kAColBase + slot * kAColsPerSlot + u * kAColsPerSub;
+                    const uint64_t db = db0 + (uint64_t)(slot * (kSub * b_bytes >> 4));
+                    const uint32_t a_tmem = tmem_base + kAColBase + slot * kAColsPerSlot;
+                    if (elect_one()) {
+                        // 16 k per MMA = 8 TMEM columns of A, 32 bytes of each B row
 #pragma unroll
-                        for (int kk = 0; kk < kBK / 16; kk++)  // 16 k = 8 TMEM columns of A, 32 bytes of each B row
-                            tc_mma_ts(tmem_base, a_tmem + 8 * kk, db + 2 * kk, idesc, (st | u | kk) != 0 ? 1u : 0u);
+                        for (int kk = 0; kk < kBK / 16; kk++) tc_mma_ts(tmem_base, a_tmem + 8 * kk, db + 2 * kk, idesc, (kk > 0 || st != 0) ? 1u : 0u);
+                        if (st * kSub + 1 < nks) {  // (the last stage of an odd K has one sub-block)
+#pragma unroll
+                            for (int kk = 0; kk < kBK / 16; kk++)
+                                tc_mma_ts(tmem_base, a_tmem + kAColsPerSub + 8 * kk, db + (b_bytes >> 4) + 2 * kk, idesc, 1u);
+                        }
+                        tc_commit(&sl->empty[slot]);  // arrives when the MMAs above have consumed their operands
                     }
-                    tc_commit(&sl->empty[slot]);  // arrives when the MMAs above have consumed their operands
+                    __syncwarp();
                     if (++slot == kStagesB) { slot = 0; phase ^= 1; }
                 }
-                if (ok) tc_commit(&sl->tmem_full);
-            }
-        }
-    } else if (warp >= kEpiWarps) {
-        // ---------------- dequantisers: group grp owns the stages = grp (mod kDqGroups); thread owns row n0 + r ----------------
-        constexpr int UPS = BITS == 8 ? 2 : 1;  // weight units (128 rows x 64 packed bytes) per pipeline stage
-        const int q = warp & 3, grp = (warp - kEpiWarps) >> 2;
-        const int r = q * 32 + lane;
-        const bool leader = (q == 0 && lane == 0);
-        const int bar_id = 1 + grp;  // named barrier of the group (0 is __syncthreads)
-        const int gpr = p.K >> p.gshift;
-        const int ng_full = (kSub * kBK) >> p.gshift;  // scale groups per full stage: 4, 2 or 1
-        const bool vec_ok = (gpr % ng_full) == 0;      // then a stage's scales of one row are one aligned vector
-        const uint32_t lane_addr = tmem_base + ((uint32_t)(q * 32) << 16) + kAColBase;
-        // this group's weight unit in shared memory; row r is 64 bytes, its 16-byte chunk c sits at c ^ ((r >> 1) & 3)
-        const unsigned char* wrow = sW + (size_t)grp * kWUnitBytes + r * 64;
-        const uint32_t wsw = (uint32_t)(r >> 1) & 3u;
-        uint64_t* wbar = &sl->wfull[grp];
-        uint32_t wround = 0;  // units of this group consumed so far
-
-        struct Cur { int tile, st; uint32_t it0; };  // an owned stage: tile, stage in the tile, stage counter at tile start
-        auto settle = [&](Cur& c) {  // first stage of c.tile owned by the group; tiles without one are skipped
-            while (c.tile < total_tiles) {
-                c.st = (int)((grp + kDqGroups - c.it0 % kDqGroups) % kDqGroups);
-                if (c.st < nst) break;
-                c.tile += gridDim.x;
-                c.it0 += nst;
-            }
-        };
-        auto advance = [&](Cur& c) {
-            c.st += kDqGroups;
-            if (c.st >= nst) {
-                c.tile += gridDim.x;
-                c.it0 += nst;
-                settle(c);
-            }
-        };
-        auto issue = [&](const Cur& c, int u) {  // leader: bring unit u of stage c into the group's slot
-            mbar_expect_tx(wbar, kWUnitBytes);
-            tma_load_2d(const_cast<unsigned char*>(sW) + (size_t)grp * kWUnitBytes, &tmap_w,
-                        c.st * (kSub * kBK * BITS / 8) + u * 64, (c.tile / p.m_tiles) * kTileN, wbar);
-        };
-        uint32_t sp[2], bp[2];  // scales / biases of the next owned stage of this row, bf16 pairs in group order
-        auto fetch_sb = [&](const Cur& c) {
-            const int n = min((c.tile / p.m_tiles) * kTileN + r, p.N - 1);
-            const int g0 = (c.st * kSub * kBK) >> p.gshift;
-            const int ng = min(gpr - g0, ng_full);
-            const uint16_t* sr = reinterpret_cast<const uint16_t*>(p.scales) + (size_t)n * gpr + g0;
-            const uint16_t* br = reinterpret_cast<const uint16_t*>(p.biases) + (size_t)n * gpr + g0;
-            sp[1] = 0; bp[1] = 0;
-            if (vec_ok && ng == ng_full && ng == 4) {
-                asm volatile("ld.global.nc.v2.u32 {%0,%1}, [%2];" : "=r"(sp[0]), "=r"(sp[1]) : "l"(sr));
-                asm volatile("ld.global.nc.v2.u32 {%0,%1}, [%2];" : "=r"(bp[0]), "=r"(bp[1]) : "l"(br));
-            } else if (vec_ok && ng == ng_full && ng == 2) {
-                asm volatile("ld.global.nc.u32 %0, [%1];" : "=r"(sp[0]) : "l"(sr));
-                asm volatile("ld.global.nc.u32 %0, [%1];" : "=r"(bp[0]) : "l"(br));
-            } else {
-                sp[0] = ldg_u16(sr); bp[0] = ldg_u16(br);
-                if (ng > 1) { sp[0] |= ldg_u16(sr + 1) << 16; bp[0] |= ldg_u16(br + 1) << 16; }
-                if (ng > 2) { sp[1] = ldg_u16(sr + 2); bp[1] = ldg_u16(br + 2); }
-                if (ng > 3) { sp[1] |= ldg_u16(sr + 3) << 16; bp[1] |= ldg_u16(br + 3) << 16; }
-            }
-        };
-
-        Cur cur{(int)blockIdx.x, 0, 0u};
-        settle(cur);
-        if (cur.tile < total_tiles) {
-            if (leader) issue(cur, 0);
-            fetch_sb(cur);
-        }
-        bool ok = true;
-        while (cur.tile < total_tiles) {
-            Cur nxt = cur;
-            advance(nxt);
-            const uint32_t it = cur.it0 + cur.st;
-            const int sa = it % kStagesB;
-            const int nsub = min(kSub, nks - cur.st * kSub);
-            const uint32_t sc[2] = {sp[0], sp[1]}, bc[2] = {bp[0], bp[1]};
-            if (nxt.tile < total_tiles) fetch_sb(nxt);  // three stages ahead of its use
-            uint32_t w[16];
-            bool group_fail = false;
-#pragma unroll
-            for (int u = 0; u < kSub; u++) {
-                if (u >= nsub) break;
-                if (UPS == 2 || u == 0) {
-                    const bool got = ok && mbar_wait(wbar, wround & 1, abort_flag);
-                    wround++;
-#pragma unroll
-                    for (int c = 0; c < 4; c++) {
-                        const uint4 v = *reinterpret_cast<const uint4*>(wrow + ((c ^ wsw) << 4));
-                        w[4 * c] = v.x; w[4 * c + 1] = v.y; w[4 * c + 2] = v.z; w[4 * c + 3] = v.w;
-                    }
-                    // The reads above are generic-proxy accesses, the refill is an async-proxy write: the proxy
-                    // fence orders the two (without it a read still in the load pipe could see the next unit).
-                    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-                    // every thread of the group has its bytes: the slot may be refilled.  The same barrier makes
-                    // a failed wait a decision of the whole group, so nobody is left waiting at it.
-                    ok = group_all(bar_id, got);
-                    if (!ok) { group_fail = true; break; }
-                    if (leader) {
-                        if (UPS == 2 && u + 1 < nsub) issue(cur, u + 1);
-                        else if (nxt.tile < total_tiles) issue(nxt, 0);
-                    }
-                }
-                // scales of the two 32-weight halves of this sub-block
-                const int h0 = (2 * u * 32) >> p.gshift, h1 = ((2 * u + 1) * 32) >> p.gshift;
-                const uint32_t s0 = (sc[h0 >> 1] >> ((h0 & 1) * 16)) & 0xFFFFu, b0 = (bc[h0 >> 1] >> ((h0 & 1) * 16)) & 0xFFFFu;
-                const uint32_t s1 = (sc[h1 >> 1] >> ((h1 & 1) * 16)) & 0xFFFFu, b1 = (bc[h1 >> 1] >> ((h1 & 1) * 16)) & 0xFFFFu;
-                uint32_t out[32];
-                const uint32_t (&ws)[WPS] = *reinterpret_cast<const uint32_t (*)[WPS]>(&w[BITS == 4 ? 8 * u : 0]);
-                if (scale_fast_ok(s0) && scale_fast_ok(s1)) dequant_row_stage<BITS, true>(ws, s0, b0, s1, b1, out);
-                else dequant_row_stage<BITS, false>(ws, s0, b0, s1, b1, out);  // whole-block branch: not if-converted
-                if (u == 0) {
-                    const bool freed = ok && mbar_wait(&sl->empty[sa], ((it / kStagesB) & 1) ^ 1, abort_flag);
-                    ok = __all_sync(0xFFFFFFFFu, freed);  // tcgen05.st below is warp-collective
-                    tc_fence_after();
-                }
+                if (ok && elect_one()) tc_commit(&sl->tmem_full);
                 __syncwarp();
-                if (ok) tmem_st32(lane_addr + sa * kAColsPerSlot + u * kAColsPerSub, out);
             }
-            if (ok) {
-                tmem_st_wait();  // once per stage: both sub-blocks are in tensor memory
-                tc_fence_before();
-                mbar_arrive(&sl->full[sa]);
-            } else if (!*abort_flag) {
-                *abort_flag = 1;
-            }
-            if (group_fail) break;  // decided by the whole group at its barrier
-            cur = nxt;                // a warp that failed alone goes on to the next barrier, where the group ends
         }
+    } else if (warp == kWWarp) {
+        // ---------------- TMA producer: packed weights ----------------
+        const TileIter seg{(int)blockIdx.x, (int)gridDim.x, total_tiles, nst};
+        if (lane == 0) weight_producer<BITS>(p, &tmap_w, seg, nks, sW, sl->wfull, sl->wempty, abort_flag, [&](int tile) { return (tile / p.m_tiles) * kTileN; });
+    } else if (warp >= kEpiWarps) {
+        // ---------------- dequantisers ----------------
+        const int q = warp & 3, grp = (warp - kEpiWarps) >> 2;
+        const TileIter seg{(int)blockIdx.x, (int)gridDim.x, total_tiles, nst};
+        dequant_role<BITS>(p, seg, grp, q * 32 + lane, nks, sW + (size_t)grp * p.w_slots * kWUnitBytes, &sl->wfull[grp * kMaxWSlots],
+                           &sl->wempty[grp * kMaxWSlots], &sl->empty[grp],
+                           tmem_base + ((uint32_t)(q * 32) << 16) + kAColBase + grp * kAColsPerSlot, abort_flag,
+                           [&](int tile) { return (tile / p.m_tiles) * kTileN; }, [&]() { mbar_arrive(&sl->full[grp]); });
     } else {
         // ---------------- epilogue: warp w reads TMEM lanes 32*(w%4).., half w/4 of the column blocks ----------------
         const int q = warp & 3, half = warp >> 2;
@@ -1002,14 +945,14 @@ qmm_tc_tiles_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_con
 // stream that bounds a stage is halved per SM, and x takes half the shared memory per stage.
 constexpr int kStagesP = 3;                   // k-stages in flight: x halves in shared memory, A in TMEM.  (Four, with
                                               // the 64 KB more of shared memory they take from L1, measured the same or slower.)
-constexpr int kPairBBytes = (kMaxBM / 2) * 128;  // one sub-block of this CTA's half of x
-constexpr int kPairYBytes = kMaxBM * kTileN * 2; // a finished tile of y as bf16
+// a finished tile of y as bf16 (the epilogue writes whole blocks of 32 rows of x)
+__host__ __device__ constexpr int pair_y_bytes(int bm) { return ((bm + 31) & ~31) * kTileN * 2; }
 constexpr int kPairEpiBar = 1 + kDqGroups;       // named barrier of the epilogue warps
-static_assert(kDqGroups <= kStagesP, "parity waits would alias");
+static_assert(kDqGroups == kStagesP, "a group always owns the same slot");
 static_assert(kAColBase + kStagesP * kAColsPerSlot <= kTmemCols, "A ring does not fit");
 constexpr uint32_t kPeerBitMask = 0xFEFFFFFFu;  // a shared::cluster address with this bit cleared is CTA 0's copy
 struct PairSmemLayout {
-    uint64_t full[kStagesP], empty[kStagesP], wfull[kDqGroups], tmem_full, tmem_empty;
+    uint64_t full[kStagesP], empty[kStagesP], wfull[kDqGroups * kMaxWSlots], wempty[kDqGroups * kMaxWSlots], tmem_full, tmem_empty;
     uint32_t tmem_base;
     int abort_flag;
 };
@@ -1058,22 +1001,22 @@ template <int BITS>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kNumThreads, 1)
 qmm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ CUtensorMap tmap_w,
                    const __grid_constant__ CUtensorMap tmap_y, const __grid_constant__ GemmParams p) {
-    constexpr int WPS = kBK * BITS / 32;  // packed words per row per stage: 8 | 16
     extern __shared__ unsigned char smem_raw[];
     unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
     unsigned char* sB = smem;  // [kStagesP][kSub][bm/2 rows][128 B], swizzled (TMA): this CTA's half of the x tile
     const uint32_t b_bytes = (uint32_t)(p.bm >> 1) * 128;
-    unsigned char* sW = sB + (size_t)kStagesP * kSub * kPairBBytes;  // [kDqGroups][128 rows][64 B], 64-byte swizzle (TMA)
-    unsigned char* sY = sW + (size_t)kDqGroups * kWUnitBytes;  // [bm rows of x][128 columns] bf16: a finished tile on its way out
+    unsigned char* sW = sB + (size_t)kStagesP * kSub * b_bytes;  // [kDqGroups][w_slots][128 rows][64 B], 64-byte swizzle (TMA)
+    unsigned char* sY = sW + (size_t)kDqGroups * p.w_slots * kWUnitBytes;  // [bm rows of x][128 columns] bf16: a finished tile on its way out
     // (without the staging buffer the shared memory is that much smaller, and L1, which holds the rows' scales and
     // biases over a tile, that much larger: worth 4 % on this kernel)
-    PairSmemLayout* sl = reinterpret_cast<PairSmemLayout*>(sY + (p.y_tma ? kPairYBytes : 0));
+    PairSmemLayout* sl = reinterpret_cast<PairSmemLayout*>(sY + (p.y_tma ? pair_y_bytes(p.bm) : 0));
     uint32_t rank;  // of this CTA in its pair: 0 issues the MMAs of both
     asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
     const int cl = (int)(blockIdx.x >> 1), ncl = (int)(gridDim.x >> 1);
     volatile int* abort_flag = &sl->abort_flag;
 
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int tid = threadIdx.x, lane = tid & 31;
+    const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);  // (uniform for the compiler too)
     const int nks = p.K / kBK;                  // 64-weight sub-blocks along K
     const int nst = (nks + kSub - 1) / kSub;    // pipeline stages per tile
     // A pair takes two neighbouring 128-row tiles of W (CTA `rank` the tile 2*np + rank) against the same rows of x;
@@ -1088,7 +1031,10 @@ qmm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_cons
             mbar_init(&sl->full[s], 4 + 4 + 1);
             mbar_init(&sl->empty[s], 1);  // one tcgen05.commit, multicast to both CTAs
         }
-        for (int g = 0; g < kDqGroups; g++) mbar_init(&sl->wfull[g], 1);  // the group leader's expect_tx
+        for (int g = 0; g < kDqGroups * kMaxWSlots; g++) {
+            mbar_init(&sl->wfull[g], 1);   // the weight producer's expect_tx
+            mbar_init(&sl->wempty[g], 4);  // the group's four warps have read their rows
+        }
         mbar_init(&sl->tmem_full, 1);
         mbar_init(&sl->tmem_empty, 2 * kEpiWarps);  // (used in CTA 0 only) the epilogue warps of both CTAs
         sl->abort_flag = 0;
@@ -1099,7 +1045,7 @@ qmm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_cons
     __syncthreads();
     cluster_sync();  // the peer's barriers are initialised before anything arrives on them
     tc_fence_after();
-    const uint32_t tmem_base = sl->tmem_base;
+    const uint32_t tmem_base = __shfl_sync(0xffffffffu, sl->tmem_base, 0);
 
     if (warp == kTmaWarp) {
         // ---------------- TMA producer: x tiles ----------------
@@ -1118,165 +1064,55 @@ qmm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_cons
                     // both halves complete on CTA 0's barrier, which expects the bytes of both
                     if (rank == 0) mbar_expect_tx(&sl->full[sb], 2 * b_bytes * nsub);
                     for (int u = 0; u < nsub; u++)
-                        tma_load_2d_pair(sB + ((size_t)sb * kSub + u) * kPairBBytes, &tmap_x, (st * kSub + u) * kBK, m0, &sl->full[sb]);
+                        tma_load_2d_pair(sB + (sb * kSub + u) * b_bytes, &tmap_x, (st * kSub + u) * kBK, m0, &sl->full[sb]);
                 }
             }
         }
     } else if (warp == kMmaWarp) {
-        // ---------------- MMA issuer ----------------
-        if (lane == 0 && rank == 0) {
+        // ---------------- MMA issuer (as above: the whole warp, one elected lane) ----------------
+        if (rank == 0) {
             const uint32_t idesc = umma_idesc(2 * kTileN, p.bm);  // 256 rows of W over the two CTAs x bm rows of x
             uint32_t tile_i = 0, slot = 0, phase = 0;
             const uint64_t db0 = umma_desc_sw128(s32(sB));
             bool ok = true;
             for (int tile = cl; tile < total_tiles && ok; tile += ncl, tile_i++) {
-                if (!mbar_wait(&sl->tmem_empty, (tile_i & 1) ^ 1, abort_flag)) break;
+                if (!mbar_wait_warp(&sl->tmem_empty, (tile_i & 1) ^ 1, abort_flag)) break;
                 tc_fence_after();
                 for (int st = 0; st < nst; st++) {
-                    const int nsub = min(kSub, nks - st * kSub);
-                    if (!mbar_wait_spin(&sl->full[slot], phase, abort_flag)) { ok = false; break; }
+                    if (!mbar_wait_warp(&sl->full[slot], phase, abort_flag)) { ok = false; break; }
                     tc_fence_after();
-                    for (int u = 0; u < nsub; u++) {
-                        const uint64_t db = db0 + (uint64_t)(slot * kSub + u) * (kPairBBytes >> 4);
-                        const uint32_t a_tmem = tmem_base + kAColBase + slot * kAColsPerSlot + u * kAColsPerSub;
+                    const uint64_t db = db0 + (uint64_t)(slot * (kSub * b_bytes >> 4));
+                    const uint32_t a_tmem = tmem_base + kAColBase + slot * kAColsPerSlot;
+                    if (elect_one()) {
+                        // 16 k per MMA = 8 TMEM columns of A, 32 bytes of each B row
 #pragma unroll
-                        for (int kk = 0; kk < kBK / 16; kk++)  // 16 k = 8 TMEM columns of A, 32 bytes of each B row
-                            tc_mma_ts_pair(tmem_base, a_tmem + 8 * kk, db + 2 * kk, idesc, (st | u | kk) != 0 ? 1u : 0u);
+                        for (int kk = 0; kk < kBK / 16; kk++) tc_mma_ts_pair(tmem_base, a_tmem + 8 * kk, db + 2 * kk, idesc, (kk > 0 || st != 0) ? 1u : 0u);
+                        if (st * kSub + 1 < nks) {  // (the last stage of an odd K has one sub-block)
+#pragma unroll
+                            for (int kk = 0; kk < kBK / 16; kk++)
+                                tc_mma_ts_pair(tmem_base, a_tmem + kAColsPerSub + 8 * kk, db + (b_bytes >> 4) + 2 * kk, idesc, 1u);
+                        }
+                        tc_commit_pair(&sl->empty[slot]);  // arrives, in both CTAs, when the MMAs above have consumed their operands
                     }
-                    tc_commit_pair(&sl->empty[slot]);  // arrives, in both CTAs, when the MMAs above have consumed their operands
+                    __syncwarp();
                     if (++slot == kStagesP) { slot = 0; phase ^= 1; }
                 }
-                if (ok) tc_commit_pair(&sl->tmem_full);
+                if (ok && elect_one()) tc_commit_pair(&sl->tmem_full);
+                __syncwarp();
             }
         }
+    } else if (warp == kWWarp) {
+        // ---------------- TMA producer: packed weights ----------------
+        const TileIter seg{cl, ncl, total_tiles, nst};
+        if (lane == 0) weight_producer<BITS>(p, &tmap_w, seg, nks, sW, sl->wfull, sl->wempty, abort_flag, n0_of);
     } else if (warp >= kEpiWarps) {
-        // ---------------- dequantisers: group grp owns the stages = grp (mod kDqGroups); thread owns row n0 + r ----------------
-        constexpr int UPS = BITS == 8 ? 2 : 1;  // weight units (128 rows x 64 packed bytes) per pipeline stage
+        // ---------------- dequantisers ----------------
         const int q = warp & 3, grp = (warp - kEpiWarps) >> 2;
-        const int r = q * 32 + lane;
-        const bool leader = (q == 0 && lane == 0);
-        const int bar_id = 1 + grp;  // named barrier of the group (0 is __syncthreads)
-        const int gpr = p.K >> p.gshift;
-        const int ng_full = (kSub * kBK) >> p.gshift;  // scale groups per full stage: 4, 2 or 1
-        const bool vec_ok = (gpr % ng_full) == 0;      // then a stage's scales of one row are one aligned vector
-        const uint32_t lane_addr = tmem_base + ((uint32_t)(q * 32) << 16) + kAColBase;
-        // this group's weight unit in shared memory; row r is 64 bytes, its 16-byte chunk c sits at c ^ ((r >> 1) & 3)
-        const unsigned char* wrow = sW + (size_t)grp * kWUnitBytes + r * 64;
-        const uint32_t wsw = (uint32_t)(r >> 1) & 3u;
-        uint64_t* wbar = &sl->wfull[grp];
-        uint32_t wround = 0;  // units of this group consumed so far
-
-        struct Cur { int tile, st; uint32_t it0; };  // an owned stage: tile, stage in the tile, stage counter at tile start
-        auto settle = [&](Cur& c) {  // first stage of c.tile owned by the group; tiles without one are skipped
-            while (c.tile < total_tiles) {
-                c.st = (int)((grp + kDqGroups - c.it0 % kDqGroups) % kDqGroups);
-                if (c.st < nst) break;
-                c.tile += ncl;
-                c.it0 += nst;
-            }
-        };
-        auto advance = [&](Cur& c) {
-            c.st += kDqGroups;
-            if (c.st >= nst) {
-                c.tile += ncl;
-                c.it0 += nst;
-                settle(c);
-            }
-        };
-        auto issue = [&](const Cur& c, int u) {  // leader: bring unit u of stage c into the group's slot
-            mbar_expect_tx(wbar, kWUnitBytes);
-            tma_load_2d(const_cast<unsigned char*>(sW) + (size_t)grp * kWUnitBytes, &tmap_w,
-                        c.st * (kSub * kBK * BITS / 8) + u * 64, n0_of(c.tile), wbar);
-        };
-        uint32_t sp[2], bp[2];  // scales / biases of the next owned stage of this row, bf16 pairs in group order
-        auto fetch_sb = [&](const Cur& c) {
-            const int n = min(n0_of(c.tile) + r, p.N - 1);
-            const int g0 = (c.st * kSub * kBK) >> p.gshift;
-            const int ng = min(gpr - g0, ng_full);
-            const uint16_t* sr = reinterpret_cast<const uint16_t*>(p.scales) + (size_t)n * gpr + g0;
-            const uint16_t* br = reinterpret_cast<const uint16_t*>(p.biases) + (size_t)n * gpr + g0;
-            sp[1] = 0; bp[1] = 0;
-            if (vec_ok && ng == ng_full && ng == 4) {
-                asm volatile("ld.global.nc.v2.u32 {%0,%1}, [%2];" : "=r"(sp[0]), "=r"(sp[1]) : "l"(sr));
-                asm volatile("ld.global.nc.v2.u32 {%0,%1}, [%2];" : "=r"(bp[0]), "=r"(bp[1]) : "l"(br));
-            } else if (vec_ok && ng == ng_full && ng == 2) {
-                asm volatile("ld.global.nc.u32 %0, [%1];" : "=r"(sp[0]) : "l"(sr));
-                asm volatile("ld.global.nc.u32 %0, [%1];" : "=r"(bp[0]) : "l"(br));
-            } else {
-                sp[0] = ldg_u16(sr); bp[0] = ldg_u16(br);
-                if (ng > 1) { sp[0] |= ldg_u16(sr + 1) << 16; bp[0] |= ldg_u16(br + 1) << 16; }
-                if (ng > 2) { sp[1] = ldg_u16(sr + 2); bp[1] = ldg_u16(br + 2); }
-                if (ng > 3) { sp[1] |= ldg_u16(sr + 3) << 16; bp[1] |= ldg_u16(br + 3) << 16; }
-            }
-        };
-
-        Cur cur{cl, 0, 0u};
-        settle(cur);
-        if (cur.tile < total_tiles) {
-            if (leader) issue(cur, 0);
-            fetch_sb(cur);
-        }
-        bool ok = true;
-        while (cur.tile < total_tiles) {
-            Cur nxt = cur;
-            advance(nxt);
-            const uint32_t it = cur.it0 + cur.st;
-            const int sa = it % kStagesP;
-            const int nsub = min(kSub, nks - cur.st * kSub);
-            const uint32_t sc[2] = {sp[0], sp[1]}, bc[2] = {bp[0], bp[1]};
-            if (nxt.tile < total_tiles) fetch_sb(nxt);  // three stages ahead of its use
-            uint32_t w[16];
-            bool group_fail = false;
-#pragma unroll
-            for (int u = 0; u < kSub; u++) {
-                if (u >= nsub) break;
-                if (UPS == 2 || u == 0) {
-                    const bool got = ok && mbar_wait(wbar, wround & 1, abort_flag);
-                    wround++;
-#pragma unroll
-                    for (int c = 0; c < 4; c++) {
-                        const uint4 v = *reinterpret_cast<const uint4*>(wrow + ((c ^ wsw) << 4));
-                        w[4 * c] = v.x; w[4 * c + 1] = v.y; w[4 * c + 2] = v.z; w[4 * c + 3] = v.w;
-                    }
-                    // The reads above are generic-proxy accesses, the refill is an async-proxy write: the proxy
-                    // fence orders the two (without it a read still in the load pipe could see the next unit).
-                    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-                    // every thread of the group has its bytes: the slot may be refilled.  The same barrier makes
-                    // a failed wait a decision of the whole group, so nobody is left waiting at it.
-                    ok = group_all(bar_id, got);
-                    if (!ok) { group_fail = true; break; }
-                    if (leader) {
-                        if (UPS == 2 && u + 1 < nsub) issue(cur, u + 1);
-                        else if (nxt.tile < total_tiles) issue(nxt, 0);
-                    }
-                }
-                // scales of the two 32-weight halves of this sub-block
-                const int h0 = (2 * u * 32) >> p.gshift, h1 = ((2 * u + 1) * 32) >> p.gshift;
-                const uint32_t s0 = (sc[h0 >> 1] >> ((h0 & 1) * 16)) & 0xFFFFu, b0 = (bc[h0 >> 1] >> ((h0 & 1) * 16)) & 0xFFFFu;
-                const uint32_t s1 = (sc[h1 >> 1] >> ((h1 & 1) * 16)) & 0xFFFFu, b1 = (bc[h1 >> 1] >> ((h1 & 1) * 16)) & 0xFFFFu;
-                uint32_t out[32];
-                const uint32_t (&ws)[WPS] = *reinterpret_cast<const uint32_t (*)[WPS]>(&w[BITS == 4 ? 8 * u : 0]);
-                if (scale_fast_ok(s0) && scale_fast_ok(s1)) dequant_row_stage<BITS, true>(ws, s0, b0, s1, b1, out);
-                else dequant_row_stage<BITS, false>(ws, s0, b0, s1, b1, out);  // whole-block branch: not if-converted
-                if (u == 0) {
-                    const bool freed = ok && mbar_wait(&sl->empty[sa], ((it / kStagesP) & 1) ^ 1, abort_flag);
-                    ok = __all_sync(0xFFFFFFFFu, freed);  // tcgen05.st below is warp-collective
-                    tc_fence_after();
-                }
-                __syncwarp();
-                if (ok) tmem_st32(lane_addr + sa * kAColsPerSlot + u * kAColsPerSub, out);
-            }
-            if (ok) {
-                tmem_st_wait();  // once per stage: both sub-blocks are in tensor memory
-                tc_fence_before();
-                __syncwarp();
-                if (lane == 0) mbar_arrive_cta0(&sl->full[sa]);  // one arrival per warp, on the barrier the MMA issuer waits at
-            } else if (!*abort_flag) {
-                *abort_flag = 1;
-            }
-            if (group_fail) break;  // decided by the whole group at its barrier
-            cur = nxt;                // a warp that failed alone goes on to the next barrier, where the group ends
-        }
+        const TileIter seg{cl, ncl, total_tiles, nst};
+        dequant_role<BITS>(p, seg, grp, q * 32 + lane, nks, sW + (size_t)grp * p.w_slots * kWUnitBytes, &sl->wfull[grp * kMaxWSlots],
+                           &sl->wempty[grp * kMaxWSlots], &sl->empty[grp],
+                           tmem_base + ((uint32_t)(q * 32) << 16) + kAColBase + grp * kAColsPerSlot, abort_flag,
+                           n0_of, [&]() { mbar_arrive_cta0(&sl->full[grp]); });
     } else {
         // ---------------- epilogue: warp w reads TMEM lanes 32*(w%4).., half w/4 of the column blocks ----------------
         const int q = warp & 3, half = warp >> 2;
@@ -1417,11 +1253,13 @@ int* error_word() {
 }
 
 struct GemmPlan {
-    int bm, m_tiles, n_tiles, streamk, pair;
+    int bm, m_tiles, n_tiles, streamk, pair, w_slots;
+    int y_tma;  // see GemmParams
     size_t smem;
 };
 
-bool make_gemm_plan(const QmmArgs& a, int sm_count, GemmPlan* pl) {
+bool make_gemm_plan(const QmmArgs& a, int sm_count, const ShardPush* push, GemmPlan* pl) {
+    if (push && push->world <= 1) push = nullptr;
     if (a.x_dtype != LUX_DTYPE_BFLOAT16 || a.sb_dtype != LUX_DTYPE_BFLOAT16) return false;
     if (a.bits != 4 && a.bits != 8) return false;
     if (a.group != 32 && a.group != 64 && a.group != 128) return false;
@@ -1429,36 +1267,51 @@ bool make_gemm_plan(const QmmArgs& a, int sm_count, GemmPlan* pl) {
     if (((uintptr_t)a.x | (uintptr_t)a.wq | (uintptr_t)a.scales | (uintptr_t)a.biases | (uintptr_t)a.y) & 15) return false;
     if ((long long)a.N * (a.K / a.group) > (1ll << 31) - 1) return false;
     pl->n_tiles = (a.N + kTileN - 1) / kTileN;
-    // rows of x per tile: as many as the MMA takes.  The time of a tile is set by the dequantisation of
-    // its 128 x K weights, not by its height, so fewer, taller tiles always win (measured: 176-row tiles
-    // for M = 512 were 20 % slower than 256-row tiles although they need one round of tiles less).
-    (void)sm_count;
-    pl->m_tiles = (a.M + kMaxBM - 1) / kMaxBM;
-    pl->bm = (((a.M + pl->m_tiles - 1) / pl->m_tiles) + 15) & ~15;
-    pl->smem = 1024 + (size_t)kStagesB * kSub * kBBytes + (size_t)kDqGroups * kWUnitBytes + (size_t)kEpiWarps * kEpiStageBytes +
-               sizeof(SmemLayout) + 64;
-    // Schedule.  In units of one k-stage of a tile (about 0.8 us) of the whole-tile kernel: an epilogue costs
-    // about e = 4 * bm/256 (the accumulator is single: nothing else runs meanwhile), handing over and adding one
-    // partial accumulator about 7 * bm/256 more, and a stage of the stream-K kernel about 1.3 (fitted to
-    // measurements of both kernels on shapes from 32 to 512 tiles).  Whole tiles: ceil(T/G) * (nst + e).
-    // Stream-K: 1.3 * T*nst/G, one epilogue more, and the partials of the tile a CTA starts.  Stream-K wins
-    // where the tiles are few against the SMs (a column-sharded slice, a small M).
-    {
-        const double T = (double)pl->n_tiles * pl->m_tiles, G = sm_count, nst = (a.K / kBK + kSub - 1) / kSub;
-        const double e = 4.0 * pl->bm / 256.0, rounds = std::ceil(T / G);
-        const double parts = T < G ? std::ceil(G / T) : 1.0;
-        const double whole = rounds * (nst + e);
-        const double sk = 1.3 * T * nst / G + (rounds + 1.0) * e + 7.0 * pl->bm / 256.0 * parts;
-        pl->streamk = sk < whole && T * nst >= G;
-        if (const char* env = getenv("LUXCUDA_QMM_SCHEDULE")) pl->streamk = env[0] == 's';  // "streamk" | "tiles" (experiments)
+    // Schedule and tile height, by the estimated time in microseconds (fitted to measurements of the three kernels on
+    // shapes from 32 to 512 tiles).  A k-stage of a tile costs about 0.45 + 0.001 * bm whatever the kernel (dequantisation,
+    // then the MMAs), so a lower tile pays where it saves no round of tiles: 777 x 2880 x 5003 took 35.6 us in 208-row
+    // tiles and 30.8 in 112-row ones, two rounds either way.
+    //   whole tiles: ceil(T/G) rounds, each with an epilogue of 3 * bm/256 that nothing else overlaps;
+    //   CTA pairs:   rounds of pair tiles; the epilogue overlaps where y leaves by TMA; 3 to set up; 0.1 more per stage for
+    //                groups of 32, whose scales outgrow the L1 that this kernel leaves (777 rows: 35.4 against 30.8 us);
+    //   stream-K:    T*nst/G stages of up to 1.6 times the cost, an epilogue more, and the exchange of partials.
+    const double G = sm_count, nst = (a.K / kBK + kSub - 1) / kSub;
+    const bool y_fast = a.y_dtype == LUX_DTYPE_BFLOAT16 && ((push ? push->ld | push->col0 : a.N) & 7) == 0;
+    const char *force = getenv("LUXCUDA_QMM_SCHEDULE"), *force_pair = getenv("LUXCUDA_QMM_PAIR");  // "streamk" | "tiles"; "0" | "1" (experiments)
+    const int m0 = (a.M + kMaxBM - 1) / kMaxBM;
+    double best = 1e30;
+    for (int mt = m0; mt <= std::min(2 * m0, m0 + 8); mt++) {  // (with many tile rows a round is a small part of the whole)
+        const int bm = (((a.M + mt - 1) / mt) + 15) & ~15;
+        if ((a.M + bm - 1) / bm != mt) continue;  // (a tile row without rows)
+        const double h = bm / 256.0, stage = 0.45 + 0.001 * bm, e = 3.0 * h, T = (double)pl->n_tiles * mt;
+        const double rounds = std::ceil(T / G), prounds = std::ceil((pl->n_tiles + 1) / 2 * (double)mt / (sm_count / 2));
+        const double cost[3] = {
+            rounds * (nst * stage + e),
+            3.0 + prounds * (nst * (stage + (a.group == 32 ? 0.1 : 0.0)) + (y_fast ? 0.5 : e)),
+            T * nst < G ? 1e30 : 2.0 + (1.1 + 0.5 * h) * T * nst / G * stage + (rounds + 1.0) * e + 4.0 * h * (T < G ? std::ceil(G / T) : 1.0)};
+        for (int k = 0; k < 3; k++) {
+            if (k == 1 && (sm_count & 1)) continue;
+            if (force && (force[0] == 's') != (k == 2)) continue;
+            if (force_pair && k < 2 && (force_pair[0] == '1') != (k == 1)) continue;
+            if (cost[k] >= best && !(force && k == 2 && mt == m0)) continue;
+            best = cost[k];
+            pl->m_tiles = mt; pl->bm = bm; pl->pair = k == 1; pl->streamk = k == 2;
+        }
     }
-    // Whole tiles on CTA pairs when the tiles about fill the SMs (measured against the one-CTA kernel on the same
-    // box: 256 tiles 59.2 against 60.1 us, 512 tiles 110.6 against 116.3, 448 tiles of the 8-bit shape 215 against
-    // 243, 112 tiles 60.3 against 64.0; below that the one-CTA kernel is 2-3 % ahead).
-    pl->pair = !pl->streamk && (sm_count & 1) == 0 && 10 * pl->n_tiles * pl->m_tiles >= 7 * sm_count;
-    if (const char* env = getenv("LUXCUDA_QMM_PAIR")) pl->pair = !pl->streamk && (sm_count & 1) == 0 && env[0] == '1';  // (experiments)
-    if (pl->pair)
-        pl->smem = 1024 + (size_t)kStagesP * kSub * kPairBBytes + (size_t)kDqGroups * kWUnitBytes + kPairYBytes + sizeof(PairSmemLayout) + 64;
+    if (best > 1e29 && !(force && force[0] == 's')) return false;
+    // Shared memory: the ring of x, as tall as the tile, and the rings of weights, a stage of each group's if there is room
+    // (one unit at 4 bit, two at 8 bit; more only take from L1, which holds the rows' scales: 3-5 % slower).
+    pl->y_tma = 0;
+    size_t fixed;
+    if (pl->pair) {
+        if (a.y_dtype == LUX_DTYPE_BFLOAT16 && !getenv("LUXCUDA_QMM_NO_YTMA"))
+            pl->y_tma = !push ? ((a.N & 7) == 0 ? 1 : 0) : (((push->ld | push->col0) & 7) == 0 ? 2 : 0);
+        fixed = 1024 + (size_t)kStagesP * kSub * (pl->bm / 2) * 128 + (pl->y_tma ? pair_y_bytes(pl->bm) : 0) + sizeof(PairSmemLayout) + 64;
+    } else {
+        fixed = 1024 + (size_t)kStagesB * kSub * pl->bm * 128 + (size_t)kEpiWarps * kEpiStageBytes + sizeof(SmemLayout) + 64;
+    }
+    pl->w_slots = (int)std::min<size_t>(a.bits == 8 ? 2 : 1, (227 * 1024 - fixed) / (kDqGroups * kWUnitBytes));
+    pl->smem = fixed + (size_t)kDqGroups * pl->w_slots * kWUnitBytes;
     return encode_tiled_fn() != nullptr;
 }
 
@@ -1502,7 +1355,7 @@ cudaError_t launch_gemm_t(const CUtensorMap& tmap, const CUtensorMap& tmap_w, co
 
 bool qmm_tc_supported(const QmmArgs& a, int sm_count) {
     GemmPlan pl;
-    return make_gemm_plan(a, sm_count, &pl);
+    return make_gemm_plan(a, sm_count, nullptr, &pl);
 }
 
 // Scratch of a launch: one partial accumulator and one flag word per CTA (see SegIter).  The flags must be zero
@@ -1512,7 +1365,7 @@ size_t qmm_tc_workspace_bytes(int sm_count) { return kWsFlagBytes + (size_t)sm_c
 cudaError_t launch_qmm_tc(const QmmArgs& a, void* workspace, int sm_count, cudaStream_t stream, const char** name,
                           const ShardPush* push) {
     GemmPlan pl;
-    if (!make_gemm_plan(a, sm_count, &pl) || !workspace || sm_count * sizeof(uint32_t) > kWsFlagBytes) return cudaErrorInvalidValue;
+    if (!make_gemm_plan(a, sm_count, push, &pl) || !workspace || sm_count * sizeof(uint32_t) > kWsFlagBytes) return cudaErrorInvalidValue;
     int* err = a.error ? a.error : error_word();
     if (!err) return cudaErrorMemoryAllocation;
     // x as a 2-D tensor [M rows][K], boxes of 64 elements (128 bytes) x bm rows, 128-byte swizzle;
@@ -1566,25 +1419,26 @@ cudaError_t launch_qmm_tc(const QmmArgs& a, void* workspace, int sm_count, cudaS
         for (int r = 0; r < push->world; r++)
             if (r != push->me) p.y_all[k++] = push->y[r];
     }
-    p.bm = pl.bm; p.n_tiles = pl.n_tiles; p.m_tiles = pl.m_tiles;
+    p.bm = pl.bm; p.w_slots = pl.w_slots; p.n_tiles = pl.n_tiles; p.m_tiles = pl.m_tiles;
     p.ws_flags = static_cast<uint32_t*>(workspace);
     p.ws = reinterpret_cast<float*>(static_cast<unsigned char*>(workspace) + kWsFlagBytes);
     p.y_tma = 0;
     if (pl.pair) {
         // y as a 2-D tensor [M rows][N] of bf16, boxes of 128 columns x bm rows, for the epilogue's TMA store
         CUtensorMap tmap_y = tmap;
-        if (p.y_bf16 && p.world == 1 && (a.N & 7) == 0 && !getenv("LUXCUDA_QMM_NO_YTMA")) {
+        p.y_tma = pl.y_tma;
+        if (p.y_tma == 1) {
             const cuuint64_t ydims[2] = {(cuuint64_t)a.N, (cuuint64_t)a.M};
             const cuuint64_t ystrides[1] = {(cuuint64_t)a.N * 2};
             const cuuint32_t ybox[2] = {(cuuint32_t)kTileN, (cuuint32_t)pl.bm};
             r = encode_tiled_fn()(&tmap_y, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, a.y, ydims, ystrides, ybox, estr,
                                   CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_NONE,
                                   CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-            p.y_tma = r == CUDA_SUCCESS ? 1 : 0;
-        } else if (p.y_bf16 && p.world > 1 && ((p.ld | p.col0) & 7) == 0 && !getenv("LUXCUDA_QMM_NO_YTMA")) {
-            p.y_tma = 2;
+            if (r != CUDA_SUCCESS) {
+                set_last_error("cuTensorMapEncodeTiled (y) failed (%d)", (int)r);
+                return cudaErrorInvalidValue;
+            }
         }
-        if (!p.y_tma) pl.smem -= kPairYBytes;
         if (name) *name = a.bits == 4 ? "qmm_tc<4,pairs>" : "qmm_tc<8,pairs>";
         return a.bits == 4 ? launch_gemm_pair_t<4>(tmap, tmap_w, tmap_y, p, pl, sm_count, stream)
                            : launch_gemm_pair_t<8>(tmap, tmap_w, tmap_y, p, pl, sm_count, stream);
