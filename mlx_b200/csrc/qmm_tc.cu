@@ -19,26 +19,20 @@
 // (64 weights = 32 columns each) from column 256 on, one slot per k-stage in
 // flight.  Shared memory: the matching ring of B stages (32 KiB each).
 //
-// One persistent CTA per SM, 22 warps:
+// One persistent CTA per SM, 23 warps:
 //   warps 0-7   epilogue: warp w reads TMEM lanes 32*(w%4).., half w/4 of the
 //               columns, rounds to bf16/fp32, stores y[m][n];
-//   warps 8-19  dequantisers in three groups of four warps: group j owns the
-//               pipeline stages = j (mod 3); inside a group warp q owns TMEM lanes
-//               32q.. (a warp may only touch its own lane quarter), so thread
-//               (q, lane) owns row n0 + 32q + lane.  The group's leader thread
-//               brings the group's next 128 rows x 64 packed bytes into the
-//               group's own shared-memory slot by TMA (64-byte swizzle, so the
-//               row-per-thread reads are bank-conflict free); a thread reads its
-//               64 bytes, the group meets at a named barrier, the leader refills
-//               the slot for the group's next stage.  (Row-per-thread loads from
-//               global memory were one L1 wavefront per lane and kept the load
-//               pipe 70-80 % busy; through the slot it is 4 wavefronts per warp.)
-//               Scales / biases of a stage are one small vector load per thread,
-//               fetched one owned stage ahead.  Then dequantise (dequant.cuh)
-//               and write 32 TMEM columns per 64 weights;
+//   warps 8-19  dequantisers in three groups of four warps (dequant_role): group j owns the
+//               pipeline stages = j (mod 3); inside a group warp q owns TMEM lanes 32q..,
+//               so thread (q, lane) owns row n0 + 32q + lane.  A unit of 128 rows x 64 packed
+//               bytes comes through shared memory (64-byte swizzle, so the row-per-thread
+//               reads are bank-conflict free; row-per-thread loads from global memory were one
+//               L1 wavefront per lane).  Scales / biases of a stage are one small vector load
+//               per thread, fetched one owned stage ahead.  32 TMEM columns per 64 weights;
 //   warp 20     TMA producer for x;
-//   warp 21     allocates TMEM, issues tcgen05.mma (one elected thread) and the
-//               commits that release A slots / B stages and publish D.
+//   warp 21     allocates TMEM, issues tcgen05.mma (one elected lane) and the
+//               commits that release A slots / B stages and publish D;
+//   warp 22     TMA producer for the packed weights (weight_producer).
 // Hand-over uses mbarriers; every wait is bounded: on a time-out the kernel
 // raises an error word (host-visible) and all roles drain and return.
 #include <cuda.h>
