@@ -148,3 +148,17 @@ def test_both_schedules(ctx, oracle, monkeypatch, schedule, M, K, N, bits, group
         assert np.array_equal(y.to_host(), first)
     for h in (bx, bw, bs, bb, y):
         h.free()
+
+
+@pytest.mark.parametrize("schedule,pair", [("tiles", "0"), ("tiles", "1"), ("streamk", "0")])
+@pytest.mark.parametrize("M,K,N,bits,group", [(17, 64, 5, 8, 64), (33, 192, 130, 8, 32), (40, 192, 257, 4, 32), (241, 320, 384, 8, 64), (300, 704, 261, 4, 64)])
+def test_odd_stage_counts_on_every_schedule(ctx, oracle, monkeypatch, schedule, pair, M, K, N, bits, group):
+    """K of an odd number of 64-weight sub-blocks (the last stage is half a stage: at 8 bit its second unit of weights is
+    announced but not loaded), stages that do not divide by the three dequantising groups, tiles past M and N."""
+    monkeypatch.setenv("LUXCUDA_QMM_SCHEDULE", schedule)
+    monkeypatch.setenv("LUXCUDA_QMM_PAIR", pair)
+    wq, s, b = oracle.make_layer(N, K, bits, group, oracle.BF16, config_id=3, layer=K, proj=N)
+    x = oracle.make_x(M, K, oracle.BF16, config_id=3, layer=K, tag=M)
+    y, kern = run_qmatmul(ctx, x, wq, s, b, bits, group, BF16)
+    assert kern.startswith("qmm_tc"), kern
+    check(oracle, y, x, wq, s, b, bits, group, oracle.BF16)
