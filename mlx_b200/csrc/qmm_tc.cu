@@ -39,25 +39,17 @@
 #include <cuda_bf16.h>
 
 #include <algorithm>
-#include <cmath>
 #include <atomic>
 
 #include "dequant.cuh"
 #include "internal.h"
+#include "qmm_plan.h"
 
 namespace luxcuda {
 
 namespace {
 
-constexpr int kBK = 64;            // weights (k) per pipeline stage = one 128-byte swizzle row of bf16
-constexpr int kStagesB = 3;  // k-stages in flight: B in shared memory, A in TMEM, one barrier pair per stage
-constexpr int kTileN = 128;        // rows of W per tile (MMA M)
-constexpr int kMaxBM = 256;        // rows of x per tile (MMA N)
-constexpr int kSub = 2;            // 64-weight sub-blocks per pipeline stage (one barrier round per 128 k)
-constexpr int kEpiStageBytes = 16 * 32 * 2;  // per epilogue warp: 16 rows of y x 32 columns, bf16
-constexpr int kWUnitBytes = kTileN * 64;  // one unit of packed weights: 128 rows x 64 bytes (128 k at 4 bit, 64 k at 8 bit)
-constexpr int kEpiWarps = 8, kDqGroups = 3, kDqWarps = 4 * kDqGroups;
-constexpr int kMaxWSlots = 4;  // weight units in flight per dequantising group, at most (p.w_slots)
+constexpr int kDqWarps = 4 * kDqGroups;
 static_assert(kDqGroups == kStagesB, "a group always owns the same slot (and its waits, by parity, cannot alias)");
 constexpr int kTmaWarp = kEpiWarps + kDqWarps, kMmaWarp = kTmaWarp + 1, kWWarp = kMmaWarp + 1;
 constexpr int kNumThreads = (kWWarp + 1) * 32;
@@ -937,10 +929,6 @@ qmm_tc_tiles_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_con
 // The MMA is 256 rows of W (128 from each CTA's tensor memory) x bm rows of x, of which each CTA stages half in
 // its shared memory; the thread that issues it (in CTA 0) issues for both tensor cores, so the instruction
 // stream that bounds a stage is halved per SM, and x takes half the shared memory per stage.
-constexpr int kStagesP = 3;                   // k-stages in flight: x halves in shared memory, A in TMEM.  (Four, with
-                                              // the 64 KB more of shared memory they take from L1, measured the same or slower.)
-// a finished tile of y as bf16 (the epilogue writes whole blocks of 32 rows of x)
-__host__ __device__ constexpr int pair_y_bytes(int bm) { return ((bm + 31) & ~31) * kTileN * 2; }
 constexpr int kPairEpiBar = 1 + kDqGroups;       // named barrier of the epilogue warps
 static_assert(kDqGroups == kStagesP, "a group always owns the same slot");
 static_assert(kAColBase + kStagesP * kAColsPerSlot <= kTmemCols, "A ring does not fit");
@@ -950,6 +938,7 @@ struct PairSmemLayout {
     uint32_t tmem_base;
     int abort_flag;
 };
+static_assert(sizeof(SmemLayout) <= kGemmCtlBytes && sizeof(PairSmemLayout) <= kGemmCtlBytes, "the plan's share of shared memory");
 __device__ __forceinline__ void cluster_sync() {
     asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
     asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
@@ -1246,12 +1235,6 @@ int* error_word() {
     return g_error_host;
 }
 
-struct GemmPlan {
-    int bm, m_tiles, n_tiles, streamk, pair, w_slots;
-    int y_tma;  // see GemmParams
-    size_t smem;
-};
-
 bool make_gemm_plan(const QmmArgs& a, int sm_count, const ShardPush* push, GemmPlan* pl) {
     if (push && push->world <= 1) push = nullptr;
     if (a.x_dtype != LUX_DTYPE_BFLOAT16 || a.sb_dtype != LUX_DTYPE_BFLOAT16) return false;
@@ -1260,53 +1243,13 @@ bool make_gemm_plan(const QmmArgs& a, int sm_count, const ShardPush* push, GemmP
     if (a.M <= 16 || a.N < 1 || a.K % kBK) return false;
     if (((uintptr_t)a.x | (uintptr_t)a.wq | (uintptr_t)a.scales | (uintptr_t)a.biases | (uintptr_t)a.y) & 15) return false;
     if ((long long)a.N * (a.K / a.group) > (1ll << 31) - 1) return false;
-    pl->n_tiles = (a.N + kTileN - 1) / kTileN;
-    // Schedule and tile height, by the estimated time in microseconds (fitted to measurements of the three kernels on
-    // shapes from 32 to 512 tiles).  A k-stage of a tile costs about 0.45 + 0.001 * bm whatever the kernel (dequantisation,
-    // then the MMAs), so a lower tile pays where it saves no round of tiles: 777 x 2880 x 5003 took 35.6 us in 208-row
-    // tiles and 30.8 in 112-row ones, two rounds either way.
-    //   whole tiles: ceil(T/G) rounds, each with an epilogue of 3 * bm/256 that nothing else overlaps;
-    //   CTA pairs:   rounds of pair tiles; the epilogue overlaps where y leaves by TMA; 3 to set up; 0.1 more per stage for
-    //                groups of 32, whose scales outgrow the L1 that this kernel leaves (777 rows: 35.4 against 30.8 us);
-    //   stream-K:    T*nst/G stages of up to 1.6 times the cost, an epilogue more, and the exchange of partials.
-    const double G = sm_count, nst = (a.K / kBK + kSub - 1) / kSub;
-    const bool y_fast = a.y_dtype == LUX_DTYPE_BFLOAT16 && ((push ? push->ld | push->col0 : a.N) & 7) == 0;
-    const char *force = getenv("LUXCUDA_QMM_SCHEDULE"), *force_pair = getenv("LUXCUDA_QMM_PAIR");  // "streamk" | "tiles"; "0" | "1" (experiments)
-    const int m0 = (a.M + kMaxBM - 1) / kMaxBM;
-    double best = 1e30;
-    for (int mt = m0; mt <= std::min(2 * m0, m0 + 8); mt++) {  // (with many tile rows a round is a small part of the whole)
-        const int bm = (((a.M + mt - 1) / mt) + 15) & ~15;
-        if ((a.M + bm - 1) / bm != mt) continue;  // (a tile row without rows)
-        const double h = bm / 256.0, stage = 0.45 + 0.001 * bm, e = 3.0 * h, T = (double)pl->n_tiles * mt;
-        const double rounds = std::ceil(T / G), prounds = std::ceil((pl->n_tiles + 1) / 2 * (double)mt / (sm_count / 2));
-        const double cost[3] = {
-            rounds * (nst * stage + e),
-            3.0 + prounds * (nst * (stage + (a.group == 32 ? 0.1 : 0.0)) + (y_fast ? 0.5 : e)),
-            T * nst < G ? 1e30 : 2.0 + (1.1 + 0.5 * h) * T * nst / G * stage + (rounds + 1.0) * e + 4.0 * h * (T < G ? std::ceil(G / T) : 1.0)};
-        for (int k = 0; k < 3; k++) {
-            if (k == 1 && (sm_count & 1)) continue;
-            if (force && (force[0] == 's') != (k == 2)) continue;
-            if (force_pair && k < 2 && (force_pair[0] == '1') != (k == 1)) continue;
-            if (cost[k] >= best && !(force && k == 2 && mt == m0)) continue;
-            best = cost[k];
-            pl->m_tiles = mt; pl->bm = bm; pl->pair = k == 1; pl->streamk = k == 2;
-        }
-    }
-    if (best > 1e29 && !(force && force[0] == 's')) return false;
-    // Shared memory: the ring of x, as tall as the tile, and the rings of weights, a stage of each group's if there is room
-    // (one unit at 4 bit, two at 8 bit; more only take from L1, which holds the rows' scales: 3-5 % slower).
-    pl->y_tma = 0;
-    size_t fixed;
-    if (pl->pair) {
-        if (a.y_dtype == LUX_DTYPE_BFLOAT16 && !getenv("LUXCUDA_QMM_NO_YTMA"))
-            pl->y_tma = !push ? ((a.N & 7) == 0 ? 1 : 0) : (((push->ld | push->col0) & 7) == 0 ? 2 : 0);
-        fixed = 1024 + (size_t)kStagesP * kSub * (pl->bm / 2) * 128 + (pl->y_tma ? pair_y_bytes(pl->bm) : 0) + sizeof(PairSmemLayout) + 64;
-    } else {
-        fixed = 1024 + (size_t)kStagesB * kSub * pl->bm * 128 + (size_t)kEpiWarps * kEpiStageBytes + sizeof(SmemLayout) + 64;
-    }
-    pl->w_slots = (int)std::min<size_t>(a.bits == 8 ? 2 : 1, (227 * 1024 - fixed) / (kDqGroups * kWUnitBytes));
-    pl->smem = fixed + (size_t)kDqGroups * pl->w_slots * kWUnitBytes;
-    return encode_tiled_fn() != nullptr;
+    // LUXCUDA_QMM_SCHEDULE = "streamk" | "tiles", LUXCUDA_QMM_PAIR = "0" | "1" (experiments)
+    const char *schedule = getenv("LUXCUDA_QMM_SCHEDULE"), *pair = getenv("LUXCUDA_QMM_PAIR");
+    GemmForce force;
+    if (schedule) force.streamk = schedule[0] == 's';
+    if (pair) force.pair = pair[0] == '1';
+    const GemmShape shape{a.M, a.K, a.N, a.bits, a.group, a.y_dtype == LUX_DTYPE_BFLOAT16, push != nullptr, push ? push->ld : a.N, push ? push->col0 : 0};
+    return choose_gemm_plan(shape, sm_count, force, getenv("LUXCUDA_QMM_NO_YTMA") != nullptr, pl) && encode_tiled_fn() != nullptr;
 }
 
 template <int BITS>
