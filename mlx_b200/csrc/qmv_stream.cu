@@ -40,8 +40,10 @@ constexpr int kThreads = (kWarps + 1 + kSumWarps) * 32;
 constexpr int kMaxStages = 6;
 constexpr int kMaxBatch = 48;  // matmuls per launch
 constexpr int kSmemLimit = 227 * 1024 - 1024;  // dynamic; the rest is for the static part
-// Registers: 640 threads x 96 at launch; the working warps take what the helper warps do not need.
-constexpr int kLaunchRegs = 96, kWorkRegs = 112, kHelperRegs = 32;
+// Registers: 640 threads x 96 at launch; the working warps take what the helper warps do not need.  With 112 and 32 the
+// helpers spilled at 4 bit with groups of 32 or 16 rows (88-104 bytes), which cost more than the working warps gained:
+// 8 x 4096 x 5003, groups of 32: 7.13 us against 5.51, groups of 64: the same; 16 x 2880 x 5003: 7.10 against 5.67.
+constexpr int kLaunchRegs = 96, kWorkRegs = 104, kHelperRegs = 56;
 static_assert(kWarps * 32 * kWorkRegs + (kThreads - kWarps * 32) * kHelperRegs <= kThreads * kLaunchRegs, "register split");
 // A stage: [tile][k-block][16 rows][128 bytes] of weights, then per tile the scales and biases, [rows 0-7: scales][rows 0-7:
 // biases][rows 8-15: scales][rows 8-15: biases], a row's being the 16-byte pieces that hold those of the chunk.  Rows of
@@ -442,15 +444,16 @@ __global__ void __launch_bounds__(kThreads, 1) qmv_stream_kernel(const __grid_co
             if (MT == 2) pass_x(8, true);
         };
         // What precedes the wait touches only weights, scales and biases (and x where the host knows that the previous
-        // kernel of the stream does not write it); behind it the next kernel of the chain may start its own fetch.
+        // kernel of the stream does not write it); behind it the next kernel of the chain may start its own fetch.  (One
+        // load_x in the code, ahead of the wait or behind it: two of them cost the 16-row form 100 bytes of spills.)
         int mine = my_groups();
-        bool x_loaded = false;
-        if (NI == 1 && p.x_early && mine) {
-            load_x();
-            x_loaded = true;
-        }
-        asm volatile("griddepcontrol.wait;" ::: "memory");
-        asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+        bool waited = false;
+        auto wait_prev = [&]() {
+            asm volatile("griddepcontrol.wait;" ::: "memory");
+            asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+            waited = true;
+        };
+        if (NI > 1 || !p.x_early) wait_prev();
 
         // this lane's place in the stage that comes next: 16-byte pieces 2t and 2t+1 of row g of the k-block
         const uint32_t in_tile = kq * 2048 + g * 128 + (((2 * t) ^ g) << 4), sa0 = ring + tsub * p.tile_bytes + in_tile;
@@ -464,7 +467,8 @@ __global__ void __launch_bounds__(kThreads, 1) qmv_stream_kernel(const __grid_co
         };
         for (;;) {
             const int ng = wk.ng;
-            if (mine && !x_loaded) load_x();
+            if (mine) load_x();
+            if (NI == 1 && !waited) wait_prev();
             if (PRO == 1) {
                 // the rows' sums of squares: a k-block's owner (tsub == 0) adds its four lanes per row, then the k-blocks in
                 // order through shared memory; every working warp ends up with the factor of its rows
@@ -526,7 +530,6 @@ __global__ void __launch_bounds__(kThreads, 1) qmv_stream_kernel(const __grid_co
             }
             if (!ok || !wk.next_run(p)) break;
             mine = my_groups();
-            x_loaded = false;
         }
     }
     __syncthreads();
