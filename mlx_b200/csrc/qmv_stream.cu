@@ -256,6 +256,8 @@ __global__ void __launch_bounds__(kThreads, 1) qmv_stream_kernel(const __grid_co
                 odd = __any_sync(0xffffffffu, odd);
                 for (int g = 0; g < wk.ng; g++) {
                     const int tile0 = wk.b0 + g * p.ts, tiles = min(p.ts, t_end - tile0);
+                    // (the ring is full and nobody works on it before the previous kernel has ended: see the summing warps)
+                    if (issued == p.stages) asm volatile("griddepcontrol.wait;" ::: "memory");
                     ok = bar_wait<true>(empty + 8 * st, ph ^ 1, abort);
                     if (!ok) break;
                     if (lane == 0) bar_expect(full + 8 * st, tiles * (p.k_tail ? ops : p.kbc) * 2048);
@@ -314,6 +316,9 @@ __global__ void __launch_bounds__(kThreads, 1) qmv_stream_kernel(const __grid_co
             // Stages are taken in turn.  (No more warps than stages: a warp's wait for a stage is then never a whole round
             // ahead of the stage's barrier, whose phase it tells by parity.)
             int turn = role - kSumWarp;
+            // The waits below are bounded by the clock, which must not start before the previous kernel of the stream has ended:
+            // it may itself be waiting, for a peer, for as long as its caller allows.
+            asm volatile("griddepcontrol.wait;" ::: "memory");
             do {
                 // the sums carried from chunk to chunk change hands (all these warps come here in every run, after an abort too)
                 if (p.nch > 1) asm volatile("bar.sync 2, %0;" ::"r"(p.sum_warps * 32) : "memory");

@@ -159,3 +159,46 @@ def test_a_wait_for_a_peer_runs_out_and_is_reported(M, batch):
     assert "STILL_WORKS True" in r.stdout, r.stdout
     if M <= 16:
         assert "PEER_COLUMNS_UNTOUCHED True" in r.stdout, r.stdout
+
+
+BEHIND_A_WAIT = r"""
+import sys
+sys.path.insert(0, %r)
+import numpy as np
+import mlx_b200
+from mlx_b200 import BF16, BackendError
+from mlx_b200 import plugin as P
+import oracle as O
+plugin = mlx_b200.Plugin(require_gpu=True)
+ctx = plugin.context(0)
+M, K, Nl, N2 = 8, 1024, 16, 16 * 1200
+wq, s, b = O.make_layer(N2, K, 4, 64, O.BF16, config_id=8)
+x = O.make_x(M, K, O.BF16, config_id=8)
+bx, bw, bs, bb = ctx.upload(x), ctx.upload(wq), ctx.upload(s), ctx.upload(b)
+y = ctx.empty((M, N2), np.uint16)
+ctx.qmatmul(bx, bw, bs, bb, y, M, K, N2, 4, 64, BF16, BF16, BF16)
+want = y.to_host().copy()
+y.from_host(np.zeros((M, N2), np.uint16))
+mine, other = P.SymmBuffer(ctx, 0, 2, (M, 2 * Nl), np.uint16), P.SymmBuffer(ctx, 1, 2, (M, 2 * Nl), np.uint16)
+hs = [mine.export(), other.export()]
+mine.attach(hs)
+other.attach(hs)
+mine.qmatmul(bx, bw, bs, bb, M, K, Nl, 4, 64, BF16)         # one CTA, which waits for the peer until the limit
+ctx.qmatmul(bx, bw, bs, bb, y, M, K, N2, 4, 64, BF16, BF16, BF16)
+try:
+    ctx.sync()
+except BackendError as e:
+    print("SYNC_ERROR", e)
+print("RESULT_WHOLE", bool(np.array_equal(y.to_host(), want)))
+"""
+
+
+def test_a_matmul_behind_a_wait_for_a_peer_keeps_its_own_limit():
+    """A launch chained behind a column-sharded one may be resident while that one waits for a peer, here for 3 s: longer
+    than the two seconds after which its own warps give one another up.  Their clocks start when the launch before has
+    ended, so its result is whole (several stages per CTA: the ring is filled more than once)."""
+    env = dict(os.environ, LUXCUDA_PEER_WAIT_MS="3000")
+    r = subprocess.run([sys.executable, "-c", BEHIND_A_WAIT % ROOT], capture_output=True, text=True, timeout=120, env=env, cwd=ROOT)
+    assert r.returncode == 0, r.stderr[-2000:]
+    assert "SYNC_ERROR" in r.stdout, r.stdout
+    assert "RESULT_WHOLE True" in r.stdout, r.stdout
