@@ -63,6 +63,12 @@ bool decode_may_overlap(const Context* c, const QmmArgs& a) {
 bool decode_x_stable(const Context* c, const QmmArgs& a) {
     return !ranges_overlap((const char*)a.x, (size_t)a.M * a.K * 2, c->chain_out_lo, c->chain_out_hi);
 }
+// A graph's recording, its end and its launch each end a chain: recording counts launches that do not run, and ends by
+// taking them off the counter again, which may thus come back to an earlier value.
+static void close_chain(Context* c) {
+    std::lock_guard<std::mutex> lk(c->mu);
+    c->chain_launches = ~0ull;
+}
 void note_decode_launch(Context* c, const QmmArgs& a) {
     c->chain_launches = c->launches.load();
     c->chain_copies = c->copies.load();
@@ -120,6 +126,7 @@ LuxBackendError qmatmul_on_stream(Context* c, const QmmArgs& a) {
     const char* name = "";
     cudaError_t e = cudaSuccess;
     int launches = 1;
+    bool overlaps = false;  // the (last) launch may start beside the one before it
     if (a.x_dtype == LUX_DTYPE_BFLOAT16) {
         if (a.M > 16 && qmm_tc_supported(a, c->dev->sm_count)) {
             LuxBackendError le = ensure_qmm_workspace(c);
@@ -139,7 +146,8 @@ LuxBackendError qmatmul_on_stream(Context* c, const QmmArgs& a) {
                     chunk.M = a.M - m0 < 16 ? a.M - m0 : 16;
                     chunk.x = (const char*)a.x + (size_t)m0 * a.K * 2;
                     chunk.y = (char*)a.y + (size_t)m0 * a.N * ysz;
-                    e = launch_qmv_mma(chunk, c->qmv_ws ? c->qmv_ws->ptr : nullptr, c->dev->sm_count, c->stream, &name, decode_may_overlap(c, chunk),
+                    overlaps = decode_may_overlap(c, chunk);
+                    e = launch_qmv_mma(chunk, c->qmv_ws ? c->qmv_ws->ptr : nullptr, c->dev->sm_count, c->stream, &name, overlaps,
                                        nullptr, decode_x_stable(c, chunk));
                     if (e == cudaSuccess) {
                         c->launches++;
@@ -152,7 +160,8 @@ LuxBackendError qmatmul_on_stream(Context* c, const QmmArgs& a) {
         }
     } else {
         launches = 0;
-        e = launch_qmv_simt(a, c->stream, &name, decode_may_overlap(c, a));
+        overlaps = decode_may_overlap(c, a);
+        e = launch_qmv_simt(a, c->stream, &name, overlaps);
         if (e == cudaSuccess) {
             c->launches++;
             note_decode_launch(c, a);
@@ -161,7 +170,8 @@ LuxBackendError qmatmul_on_stream(Context* c, const QmmArgs& a) {
     if (e != cudaSuccess) return map_cuda_error(e, name);
     c->last_kernel = name;
     c->launches += launches;
-    if (getenv("LUXCUDA_TRACE")) fprintf(stderr, "luxcuda: qmatmul M=%d K=%d N=%d bits=%d group=%d -> %s\n", a.M, a.K, a.N, a.bits, a.group, name);
+    if (getenv("LUXCUDA_TRACE"))
+        fprintf(stderr, "luxcuda: qmatmul M=%d K=%d N=%d bits=%d group=%d -> %s%s\n", a.M, a.K, a.N, a.bits, a.group, name, overlaps ? " overlapping" : "");
     return LUX_BACKEND_OK;
 }
 
@@ -555,6 +565,7 @@ LuxBackendError graph_begin(LuxBackendContext* ctx) {
     Context* c = as_ctx(ctx);
     if (!c) return LUX_BACKEND_ERROR_INVALID_ARGUMENT;
     DeviceGuard g(c->dev->device());
+    close_chain(c);
     LUX_CUDA_TRY(cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal));
     t_capture_base = c->launches.load();
     return LUX_BACKEND_OK;
@@ -563,6 +574,7 @@ LuxBackendError graph_end(LuxBackendContext* ctx, LuxCudaGraph** out) {
     Context* c = as_ctx(ctx);
     if (!c || !out) return LUX_BACKEND_ERROR_INVALID_ARGUMENT;
     DeviceGuard g(c->dev->device());
+    close_chain(c);
     cudaGraph_t graph = nullptr;
     LUX_CUDA_TRY(cudaStreamEndCapture(c->stream, &graph));
     auto* gr = new (std::nothrow) LuxCudaGraph();
@@ -587,6 +599,7 @@ LuxBackendError graph_launch(LuxBackendContext* ctx, LuxCudaGraph* gr) {
     Context* c = as_ctx(ctx);
     if (!c || !gr || !gr->exec || gr->device != c->dev->device()) return LUX_BACKEND_ERROR_INVALID_ARGUMENT;
     DeviceGuard g(c->dev->device());
+    close_chain(c);
     LUX_CUDA_TRY(cudaGraphLaunch(gr->exec, c->stream));
     c->launches += gr->launches;
     return LUX_BACKEND_OK;

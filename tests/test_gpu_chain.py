@@ -283,3 +283,38 @@ def test_prologue_refuses_what_it_does_not_take(ctx, oracle, plugin):
     with pytest.raises(P.BackendError) as ei:   # x_ld too short for three column blocks
         ctx.qmatmul_pro(x16, bw, bs, bb, y, 8, K // 4, N, 4, 64, BF16, P.PRO_SUM3, K // 2)
     assert ei.value.code == P.ERR_INVALID
+
+
+@pytest.mark.parametrize("dt", [P.BF16, P.F32])
+def test_a_recorded_graph_leaves_no_chain_open(ctx, oracle, monkeypatch, capfd, dt):
+    """Recording counts launches and takes them off again.  A matmul whose weights a quantize has just written must not start
+    beside it, however many launches lie between the recording and it; one behind another matmul may."""
+    M, N, K, sd = 2, 256, 512, oracle.BF16 if dt == P.BF16 else oracle.F32
+    x = ctx.upload(oracle.make_x(M, K, sd, config_id=5, tag=3))
+    w = (np.random.default_rng(9).standard_normal((N, K)) * 0.05).astype(np.float32)
+    wq, s, b = oracle.quantize(w, 4, 64, sd)
+    bf, bw, bs, bb = ctx.upload(w), ctx.upload(wq), ctx.upload(s), ctx.upload(b)
+    y = ctx.empty((M, N), np.uint16 if dt == P.BF16 else np.float32)
+
+    def mm():
+        ctx.qmatmul(x, bw, bs, bb, y, M, K, N, 4, 64, dt, dt, dt)
+    mm()
+    ctx.sync()
+    monkeypatch.setenv("LUXCUDA_TRACE", "1")
+    for recorded in (1, 2):
+        ctx.graph_begin()
+        for _ in range(recorded):
+            mm()
+        g = ctx.graph_end()
+        capfd.readouterr()
+        for _ in range(recorded):
+            ctx.quantize(bf, bw, bs, bb, N, K, 4, 64, dt)
+        mm()
+        mm()
+        first, second = [ln for ln in capfd.readouterr().err.splitlines() if "qmatmul M=" in ln]
+        assert not first.endswith("overlapping") and second.endswith("overlapping")
+        ctx.graph_launch(g)
+        mm()
+        assert not capfd.readouterr().err.rstrip().endswith("overlapping")
+        ctx.sync()
+        ctx.graph_destroy(g)
