@@ -1192,6 +1192,7 @@ extern "C" LUX_GPU_BACKEND_EXPORT LuxBackendError lux_gpu_cuda_qmatmul_decode_no
     }
     QmmArgs a{bx->ptr, (const uint32_t*)bw->ptr, bs->ptr, bb->ptr, by->ptr, M, K, N, bits, group,
               LUX_DTYPE_BFLOAT16, LUX_DTYPE_BFLOAT16, (int)y_dtype};
+    a.error = c->err_dev;  // (without it the first launch of a process would allocate the word that processes share)
     std::lock_guard<std::mutex> lk(c->mu);
     DeviceGuard g(c->dev->device());
     const size_t need = qmv_mma_workspace_bytes(a, c->dev->sm_count);

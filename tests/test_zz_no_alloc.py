@@ -10,6 +10,10 @@ and that an over-sized request is refused rather than overrunning the array.
 
 Collected last on purpose: a failure here must not hide the other GPU tests under `-x`.
 """
+import os
+import subprocess
+import sys
+
 import numpy as np
 import pytest
 
@@ -103,3 +107,34 @@ def test_noalloc_scratch_shared_between_split_shapes(plugin, ctx, oracle):
                 h.free()
     finally:
         fresh.close()
+
+
+FIRST_CALL = r"""
+import sys
+sys.path.insert(0, %r)
+import os
+import subprocess
+import sys
+
+import numpy as np
+import mlx_b200
+from mlx_b200 import BF16
+import oracle as O
+ctx = mlx_b200.Plugin(require_gpu=True).context(0)
+M, K, N = 2, 1024, 100
+wq, s, b = O.make_layer(N, K, 4, 64, O.BF16, config_id=13)
+x = O.make_x(M, K, O.BF16, config_id=13)
+bx, bw, bs, bb, y = ctx.upload(x), ctx.upload(wq), ctx.upload(s), ctx.upload(b), ctx.empty((M, N), np.uint16)
+ctx.graph_begin()
+ctx.qmatmul_decode_noalloc(bx, bw, bs, bb, y, M, K, N, 4, 64, BF16)
+g = ctx.graph_end()
+ctx.graph_launch(g)
+print("RESULT", bool(O.rel_err(y.to_host(), O.qmatmul_truth(x, wq, s, b, 4, 64))[0] <= 1e-2))
+"""
+
+
+def test_noalloc_as_the_first_call_of_a_process_inside_a_recording():
+    """Nothing is set up on the way: the call records even where it is the first one of its process."""
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    r = subprocess.run([sys.executable, "-c", FIRST_CALL % root], capture_output=True, text=True, timeout=120, cwd=root)
+    assert r.returncode == 0 and "RESULT True" in r.stdout, (r.stdout[-500:], r.stderr[-1500:])
