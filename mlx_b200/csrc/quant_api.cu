@@ -409,37 +409,37 @@ LuxBackendError qmatmul_batch(LuxBackendContext* ctx, int n, LuxBackendBuffer* c
     }
     std::lock_guard<std::mutex> lk(c->mu);
     DeviceGuard g(c->dev->device());
-    const char* name = "";
-    bool batched = false;
+    auto one_by_one = [&](const QmmArgs* a, size_t count) {
+        LuxBackendError r = LUX_BACKEND_OK;
+        for (size_t i = 0; i < count && r == LUX_BACKEND_OK; i++) r = qmatmul_on_stream(c, a[i]);
+        return r;
+    };
     if (decode) {
         // the items with M <= 8 and those with M > 8, each kind in launches of at most qmv_batch_max()
-        batched = true;
         std::vector<QmmArgs> kind;
-        for (int hi = 0; hi < 2 && batched; hi++) {
+        for (int hi = 0; hi < 2; hi++) {
             kind.clear();
             for (const QmmArgs& a : items)
                 if ((a.M > 8) == (hi == 1)) kind.push_back(a);
-            for (size_t i0 = 0; i0 < kind.size() && batched; i0 += (size_t)qmv_batch_max()) {
+            for (size_t i0 = 0; i0 < kind.size(); i0 += (size_t)qmv_batch_max()) {
                 const int cnt = (int)std::min(kind.size() - i0, (size_t)qmv_batch_max());
+                const char* name = "";
                 cudaError_t e = launch_qmv_batch(kind.data() + i0, cnt, c->dev->sm_count, c->stream, &name);
-                if (e == cudaErrorNotSupported && hi == 0 && i0 == 0) {
+                if (e == cudaErrorNotSupported) {  // K split over CTAs, ...
                     cudaGetLastError();
-                    batched = false;  // nothing launched yet: one by one below
+                    LuxBackendError r = one_by_one(kind.data() + i0, (size_t)cnt);
+                    if (r != LUX_BACKEND_OK) return r;
                 } else if (e != cudaSuccess) {
                     return map_cuda_error(e, name);
                 } else {
                     c->launches++;
+                    c->last_kernel = name;
                 }
             }
         }
-    }
-    if (!batched) {
-        for (const QmmArgs& a : items) {
-            LuxBackendError r = qmatmul_on_stream(c, a);
-            if (r != LUX_BACKEND_OK) return r;
-        }
     } else {
-        c->last_kernel = name;
+        LuxBackendError r = one_by_one(items.data(), items.size());
+        if (r != LUX_BACKEND_OK) return r;
     }
     for (int i = 0; i < n; i++)
         as_buf(x[i])->last_stream = as_buf(wq[i])->last_stream = as_buf(scales[i])->last_stream = as_buf(biases[i])->last_stream =

@@ -312,7 +312,7 @@ def test_scale_extremes_bit_exact(ctx, oracle, bits, group):
 
 
 @pytest.mark.parametrize("K,N,bits,group,Ms", [(4096, 1200, 4, 64, [1, 4, 8, 16, 3, 12, 8, 1]), (2048, 528, 8, 128, [2, 16, 16, 7]),
-                                                  (1024, 100, 4, 32, [5]), (8192, 64, 4, 64, [8, 1, 16]),
+                                                  (1024, 100, 4, 32, [5]), (8192, 64, 4, 64, [8, 1, 16]), (8192, 64, 4, 64, [16, 12]),
                                                   # more matmuls than CTAs (the CTAs' tile ranges rotate from one matmul to the
                                                   # next and wrap around), 4 bytes of scales per row and k-block
                                                   (2048, 272, 4, 128, [8, 1, 3, 5, 2, 7, 4, 6, 8, 1, 2, 3, 4, 5, 6, 7, 8, 1, 2, 3]),
