@@ -47,7 +47,9 @@ constexpr int kLaunchRegs = 96, kWorkRegs = 104, kHelperRegs = 56;
 static_assert(kWarps * 32 * kWorkRegs + (kThreads - kWarps * 32) * kHelperRegs <= kThreads * kLaunchRegs, "register split");
 // A stage: [tile][k-block][16 rows][128 bytes] of weights, then per tile the scales and biases, [rows 0-7: scales][rows 0-7:
 // biases][rows 8-15: scales][rows 8-15: biases], a row's being the 16-byte pieces that hold those of the chunk.  Rows of
-// sb_row bytes: 16 k-blocks' worth and up to 14 bytes of what lies before; an odd multiple of 16 bytes, for the banks.
+// sb_row bytes: 16 k-blocks' worth and up to 14 bytes of what lies before; an odd multiple of 16 bytes, for the banks.  (K cut
+// off inside a k-block leaves room for the zeros behind the last group: a group of a k-block is missing, or at SPL = 2 all 272
+// bytes are used.)
 constexpr int sb_row(int spl) { return spl == 2 ? 16 * 16 + 16 : 16 * 8 + 16; }
 
 __device__ __forceinline__ uint32_t s32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
@@ -238,20 +240,25 @@ __global__ void __launch_bounds__(kThreads, 1) qmv_stream_kernel(const __grid_co
             // Lane (r, k) of a load: piece k of row r.  LPR pieces of a row side by side, RPI rows per load, rows r and r + 8
             // by the same distance (16*gpr bytes keep the 16-byte boundaries).
             constexpr int LPR = SPL == 2 ? 16 : 8, RPI = 32 / LPR, NB = 8 / RPI;
-            const uint32_t gpr = (uint32_t)p.K >> p.gshift, total = 2u * p.N * gpr, half = 16u * gpr, k16 = 16u * (lane % LPR);
+            // Pieces are cut off at the row's end and filled up with zeros.  Where K ends inside a k-block, the groups that the
+            // lanes past K would have read their scales from are zeros, too (for those a piece of nothing else, if need be): zero
+            // codes with the last group's own scale and bias would add 0 * infinity where these are infinite.
+            const uint32_t gpr = (uint32_t)p.K >> p.gshift, half = 16u * gpr, k16 = 16u * (lane % LPR);
             do {
                 const int t_end = wk.tile_end(p), kb0 = wk.c * p.kbc, ops = p.k_tail ? wk.kb_cnt(p) : 1;
                 const CUtensorMap* map = &p.maps[wk.item];
                 const uint32_t g0 = (uint32_t)(wk.c * p.kbc) * KB >> p.gshift, bytes = 2u * min((uint32_t)wk.kb_cnt(p) * KB >> p.gshift, gpr - g0);
                 const char *sc = reinterpret_cast<const char*>(p.items[wk.item].scales), *bi = reinterpret_cast<const char*>(p.items[wk.item].biases);
-                // where this lane's pieces of the run's first tile begin, as far as there are any
-                uint32_t lo[NB], some = 0, odd = 0;
+                const uint32_t need = bytes + (p.k_tail && wk.c + 1 == p.nch ? 2u * SPL : 0u);
+                // where this lane's pieces of the run's first tile begin, as far as there are any, and their bytes of the row
+                uint32_t lo[NB], cnt[NB], some = 0, odd = 0;
 #pragma unroll
                 for (int i = 0; i < NB; i++) {
                     const uint32_t at = 2u * (((uint32_t)wk.b0 * 16 + i * RPI + lane / LPR) * gpr + g0);
                     lo[i] = (at & ~15u) + k16;
-                    some |= (lo[i] < at + bytes ? 1u : 0u) << i;
-                    odd |= (at & ~15u) + 16 * LPR < at + bytes ? 1u : 0u;  // a row that needs a piece more
+                    cnt[i] = lo[i] < at + bytes ? min(16u, at + bytes - lo[i]) : 0u;
+                    some |= (lo[i] < at + need ? 1u : 0u) << i;
+                    odd |= (at & ~15u) + 16 * LPR < at + need ? 1u : 0u;  // a row that needs a piece more
                 }
                 odd = __any_sync(0xffffffffu, odd);
                 for (int g = 0; g < wk.ng; g++) {
@@ -272,14 +279,14 @@ __global__ void __launch_bounds__(kThreads, 1) qmv_stream_kernel(const __grid_co
                     issued++;
                     uint32_t dst = stage + p.sb_off + (lane / LPR) * SROW + k16;
                     for (int ti = 0; ti < tiles; ti++, dst += 32 * SROW) {
-                        if ((tile0 + ti) * 16 + 16 < p.N) {  // every piece lies inside the arrays
+                        if ((tile0 + ti) * 16 + 16 <= p.N) {
 #pragma unroll
                             for (int i = 0; i < NB; i++)
                                 if (some >> i & 1) {
 #pragma unroll
                                     for (int h = 0; h < 2; h++) {
-                                        cp_async16(dst + i * RPI * SROW + h * 16 * SROW, sc + (lo[i] + h * half), 16);
-                                        cp_async16(dst + i * RPI * SROW + h * 16 * SROW + 8 * SROW, bi + (lo[i] + h * half), 16);
+                                        cp_async16(dst + i * RPI * SROW + h * 16 * SROW, sc + (lo[i] + h * half), cnt[i]);
+                                        cp_async16(dst + i * RPI * SROW + h * 16 * SROW + 8 * SROW, bi + (lo[i] + h * half), cnt[i]);
                                     }
                                 }
                         } else {
@@ -287,17 +294,18 @@ __global__ void __launch_bounds__(kThreads, 1) qmv_stream_kernel(const __grid_co
                                 for (int h = 0; h < 2; h++) {
                                     const uint32_t src = lo[i] + h * half;
                                     if ((some >> i & 1) && (tile0 + ti) * 16 + i * RPI + lane / LPR + 8 * h < p.N) {
-                                        cp_async16(dst + i * RPI * SROW + h * 16 * SROW, sc + src, min(16u, total - src));
-                                        cp_async16(dst + i * RPI * SROW + h * 16 * SROW + 8 * SROW, bi + src, min(16u, total - src));
+                                        cp_async16(dst + i * RPI * SROW + h * 16 * SROW, sc + src, cnt[i]);
+                                        cp_async16(dst + i * RPI * SROW + h * 16 * SROW + 8 * SROW, bi + src, cnt[i]);
                                     }
                                 }
                         }
                         if (odd && lane < 16) {
                             const uint32_t n = (tile0 + ti) * 16 + lane, at = 2u * (n * gpr + g0), src = (at & ~15u) + 16 * LPR;
                             const uint32_t d = stage + p.sb_off + ti * (32 * SROW) + (lane >> 3) * (16 * SROW) + (lane & 7) * SROW + 16 * LPR;
-                            if (n < (uint32_t)p.N && src < at + bytes) {
-                                cp_async16(d, sc + src, min(16u, total - src));
-                                cp_async16(d + 8 * SROW, bi + src, min(16u, total - src));
+                            if (n < (uint32_t)p.N && src < at + need) {
+                                const uint32_t c = src < at + bytes ? min(16u, at + bytes - src) : 0u;
+                                cp_async16(d, sc + src, c);
+                                cp_async16(d + 8 * SROW, bi + src, c);
                             }
                         }
 #pragma unroll
@@ -488,14 +496,13 @@ __global__ void __launch_bounds__(kThreads, 1) qmv_stream_kernel(const __grid_co
                 for (int w = 0; w < kWarps; w++) tot += s_rms[w][g];
                 rms_scale<XV>(xr, __fdiv_rn(1.0f, sqrtf(__fadd_rn(__fdiv_rn(tot, (float)p.K), p.eps))));
             }
-            // this lane's scales in a stage, from its weights: its group (the row's last one where K ends before it) in the
-            // row's pieces, which begin up to 14 bytes ahead of the chunk's first one (the same for rows 8 apart)
-            uint32_t sb_lane, sb_second = 0;
+            // this lane's scales in a stage, from its weights: its group (the zeros behind the row's last one where K ends before
+            // it) in the row's pieces, which begin up to 14 bytes ahead of the chunk's first one (the same for rows 8 apart)
+            uint32_t sb_lane;
             {
-                const int kb0 = wk.c * p.kbc, gpr = p.K >> p.gshift, g0 = kb0 * KB >> p.gshift, gi = min(((kb0 + kq) * KB + t * KL) >> p.gshift, gpr - 1);
+                const int kb0 = wk.c * p.kbc, gpr = p.K >> p.gshift, g0 = kb0 * KB >> p.gshift, gi = min(((kb0 + kq) * KB + t * KL) >> p.gshift, gpr);
                 const int n = (wk.b0 + tsub) * 16 + g;
                 sb_lane = p.sb_off + tsub * (32 * SROW - p.tile_bytes) + g * SROW + ((uint32_t)((n * gpr + g0) * 2) & 15u) + 2 * (gi - g0) - in_tile;
-                if (SPL == 2 && gi + 1 < gpr) sb_second = 2;
             }
 #pragma unroll 1
             for (int gi = 0; gi < mine; gi++) {
@@ -505,8 +512,8 @@ __global__ void __launch_bounds__(kThreads, 1) qmv_stream_kernel(const __grid_co
                 for (int r = 0; r < 2; r++)
 #pragma unroll
                     for (int i = 0; i < SPL; i++) {
-                        s[r][i] = lds_u16(sa + sb_lane + (i ? sb_second : 0) + r * 16 * SROW);
-                        b[r][i] = lds_u16(sa + sb_lane + (i ? sb_second : 0) + r * 16 * SROW + 8 * SROW);
+                        s[r][i] = lds_u16(sa + sb_lane + 2 * i + r * 16 * SROW);
+                        b[r][i] = lds_u16(sa + sb_lane + 2 * i + r * 16 * SROW + 8 * SROW);
                     }
 #pragma unroll
                 for (int r = 0; r < 2; r++)

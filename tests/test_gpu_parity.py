@@ -195,6 +195,24 @@ def test_fallback_shapes_bf16(ctx, oracle):
         check(oracle, y, x, wq, s, b, bits, group, oracle.BF16)
 
 
+@pytest.mark.parametrize("bits,group,K", [(4, 32, 32), (4, 32, 288), (4, 32, 4128), (4, 64, 320), (4, 128, 640), (8, 32, 32), (8, 64, 192), (8, 32, 2080)])
+@pytest.mark.parametrize("M", [1, 9])
+def test_infinite_weights_in_the_last_group(ctx, oracle, bits, group, K, M):
+    """K inside a k-block: what lies past K adds nothing, also where the scale or the bias of the last group is infinite
+    (positive x and codes of at least 1: such rows of W give plus infinity and nothing else)."""
+    N = 20
+    wq, s, b = oracle.make_layer(N, K, bits, group, oracle.BF16, config_id=15)
+    wq |= np.uint32(0x11111111 if bits == 4 else 0x01010101)
+    x = oracle.make_x(M, K, oracle.BF16, config_id=15) & 0x7FFF
+    x[x == 0] = 0x3F80
+    b[3, -1] = 0x7F80
+    s[11, -1] = 0x7F80
+    y, _ = run_qmatmul(ctx, x, wq, s, b, bits, group, F32)
+    rows = np.r_[0:3, 4:11, 12:N]
+    assert np.isposinf(y[:, [3, 11]]).all()
+    check(oracle, np.ascontiguousarray(y[:, rows]), x, wq[rows], s[rows], b[rows], bits, group, oracle.BF16)
+
+
 def test_rows_of_x_are_independent(ctx, oracle):
     """M=1 result equals the matching row of the M=16 result bit for bit, and
     repeated rows of x give identical rows of y."""
