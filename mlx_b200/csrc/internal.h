@@ -221,7 +221,7 @@ struct ShardPush {
 // decode GEMV, bf16 activations: mma.sync m16n8k16 with in-register dequant
 bool qmv_mma_supported(const QmmArgs& a, int sm_count);
 // the same without K split or peers, any K (a multiple of the group): weights through bulk copies (qmv_stream.cu);
-// n items of one shape and one side of M = 8 in one launch
+// n items of one shape and one side of M = 8 in one launch, or one matmul of any number of rows
 bool qmv_stream_supported(const QmmArgs& a, int sm_count);
 cudaError_t launch_qmv_stream(const QmmArgs* items, int n, int sm_count, cudaStream_t stream, bool overlap_prev, bool x_stable);
 size_t qmv_mma_workspace_bytes(const QmmArgs& a, int sm_count);

@@ -1,4 +1,5 @@
-// Decode-regime quantized matmul for bf16 activations, M <= 16, one launch for one matmul or for several of one shape:
+// Decode-regime quantized matmul for bf16 activations, one launch for one matmul or for several of one shape, 16 rows of x at
+// a time:
 //   y[M,N] = x[M,K] . dequant(Wq[N,K])^T,  w^ = RNE_bf16(s*q + b)  (one bf16 FMA)
 //
 // HBM-bound: every packed word, scale and bias is read once; algorithmic bytes per output row: K*bits/8 + 4*K/group.
@@ -24,6 +25,10 @@
 // the tiles are carried along in shared memory and x is reloaded per chunk.
 //
 // K need not be a multiple of the k-block: x reads as zero past K, and the last box of a row is cut off there.
+//
+// More than 16 rows of x (the prefill kernel takes them where K is a multiple of 64) are items of 16 rows on the same
+// weights, dealt over the grid's y as far as few row tiles leave SMs over.  (A launch for every 16 rows: 4096 x 96 x 16 took
+// 544 us; the CUDA-core kernel 12; this way 6.)
 #include <algorithm>
 #include <atomic>
 
@@ -133,6 +138,7 @@ __device__ __forceinline__ V8 ldg_2v4(const void* p) {  // the same from a 16-by
     return r;
 }
 
+constexpr int kItemRows = 16;  // rows of x of an item, at most (more of one matmul: several items, see Params)
 struct Item {
     const __nv_bfloat16* x;
     const __nv_bfloat16* scales;
@@ -140,11 +146,15 @@ struct Item {
     void* y;
     int M;
 };
+// NI: how many matmuls of a batch, at most; 1: one; 0: one whose rows of x are n_items items of 16 (M: all of them).
 template <int NI>
 struct Params {
-    alignas(64) CUtensorMap maps[NI];  // the packed weights of each item
-    Item items[NI];
+    static constexpr bool kRows = NI == 0;
+    static constexpr int kArray = kRows ? 1 : NI;
+    alignas(64) CUtensorMap maps[kArray];  // the packed weights
+    Item items[kArray];
     int n_items, K, N, gshift, y_bf16;
+    __device__ __forceinline__ const Item& item(int i) const { return items[kRows ? 0 : i]; }
     int rt_q, rt_rem;       // row tiles per CTA, and how many CTAs have one more
     int ts_inv, kbc_inv;    // 65536 / ts, 65536 / kbc, rounded up
     int nkb, nch, kbc, ts, tb;  // k-blocks; chunks of K and k-blocks per chunk (at most); row tiles per stage, and per pass over K
@@ -157,9 +167,9 @@ struct Params {
     int* error;             // host-visible error word of the bounded waits
 };
 
-// The CTA's work, walked in the same order by every role: items; passes of at most tb row tiles; chunks of K; groups of
-// ts tiles (one stage each).  The row tiles are dealt out in gridDim.x ranges of rt_q or rt_q + 1 tiles; the CTA takes
-// range (blockIdx.x + i) mod grid of item i, which evens out the one tile by which they differ.  (No divisions: they
+// The CTA's work, walked in the same order by every role: items, every gridDim.y-th; passes of at most tb row tiles; chunks
+// of K; groups of ts tiles (one stage each).  The row tiles are dealt out in gridDim.x ranges of rt_q or rt_q + 1 tiles; the CTA takes
+// range (blockIdx.x + i) mod gridDim.x of its i-th item, which evens out the one tile by which they differ.  (No divisions: they
 // would be a microsecond in front of the first weight.)
 struct Walk {
     int item, lo, hi, b0, c, ng;  // range [lo, hi), pass at b0, chunk, groups of this pass
@@ -177,7 +187,8 @@ struct Walk {
     }
     template <class P>
     __device__ __forceinline__ void init(const P& p) {
-        item = c = 0;
+        item = P::kRows ? blockIdx.y : 0;
+        c = 0;
         rc = blockIdx.x;
         range(p);
     }
@@ -190,7 +201,7 @@ struct Walk {
             groups(p);
             return true;
         }
-        if (++item >= p.n_items) return false;
+        if ((item += P::kRows ? gridDim.y : 1) >= p.n_items) return false;
         if (++rc == (int)gridDim.x) rc = 0;
         range(p);
         return true;
@@ -246,9 +257,9 @@ __global__ void __launch_bounds__(kThreads, 1) qmv_stream_kernel(const __grid_co
             const uint32_t gpr = (uint32_t)p.K >> p.gshift, half = 16u * gpr, k16 = 16u * (lane % LPR);
             do {
                 const int t_end = wk.tile_end(p), kb0 = wk.c * p.kbc, ops = p.k_tail ? wk.kb_cnt(p) : 1;
-                const CUtensorMap* map = &p.maps[wk.item];
+                const CUtensorMap* map = &p.maps[p.kRows ? 0 : wk.item];
                 const uint32_t g0 = (uint32_t)(wk.c * p.kbc) * KB >> p.gshift, bytes = 2u * min((uint32_t)wk.kb_cnt(p) * KB >> p.gshift, gpr - g0);
-                const char *sc = reinterpret_cast<const char*>(p.items[wk.item].scales), *bi = reinterpret_cast<const char*>(p.items[wk.item].biases);
+                const char *sc = reinterpret_cast<const char*>(p.item(wk.item).scales), *bi = reinterpret_cast<const char*>(p.item(wk.item).biases);
                 const uint32_t need = bytes + (p.k_tail && wk.c + 1 == p.nch ? 2u * SPL : 0u);
                 // where this lane's pieces of the run's first tile begin, as far as there are any, and their bytes of the row
                 uint32_t lo[NB], cnt[NB], some = 0, odd = 0;
@@ -331,8 +342,12 @@ __global__ void __launch_bounds__(kThreads, 1) qmv_stream_kernel(const __grid_co
                 // the sums carried from chunk to chunk change hands (all these warps come here in every run, after an abort too)
                 if (p.nch > 1) asm volatile("bar.sync 2, %0;" ::"r"(p.sum_warps * 32) : "memory");
                 const int kn = wk.kb_cnt(p), t_end = wk.tile_end(p);
-                const int M = p.items[wk.item].M;
-                void* y = p.items[wk.item].y;
+                int M = p.item(wk.item).M;
+                void* y = p.item(wk.item).y;
+                if (p.kRows) {
+                    M = min(M - kItemRows * wk.item, kItemRows);
+                    y = static_cast<char*>(y) + (size_t)wk.item * kItemRows * p.N * (p.y_bf16 ? 2 : 4);
+                }
                 // lane (g, t) of the MMA: rows n = g, g+8 of the tile, rows of x 2t, 2t+1 (and 8 more)
                 const int m0 = 2 * (lane & 3), n0 = lane >> 2;
                 for (int g = 0; g < wk.ng && ok; g++) {
@@ -415,7 +430,8 @@ __global__ void __launch_bounds__(kThreads, 1) qmv_stream_kernel(const __grid_co
         auto pass_x = [&](int row0, bool keep) {
             // lane: a pair of fragments (16 consecutive elements, 32 bytes) of (row, t); PP pairs per t and pass
             constexpr int PP = XP / 2, CPR = 4 * PP, RPI = 32 / CPR, NL = 8 / RPI;
-            const Item& it = p.items[wk.item];
+            const Item& it = p.item(wk.item);
+            const int first = p.kRows ? wk.item * kItemRows : 0;  // row of the matmul that is the item's row 0
             const int pr = lane % PP, tt = lane / PP % 4, row = row0 + lane / CPR, ld = PRO == 0 ? p.K : p.x_ld;
             const int k0 = (wk.c * p.kbc + kq) * KB + tt * KL + pr * 16;
             V8 v[PASS][NL];
@@ -426,8 +442,8 @@ __global__ void __launch_bounds__(kThreads, 1) qmv_stream_kernel(const __grid_co
                     const int k = k0 + h * (KL / PASS);
 #pragma unroll
                     for (int e = 0; e < 8; e++) v[h][i].v[e] = 0;
-                    if (row + i * RPI < it.M && k < p.K) {
-                        const __nv_bfloat16* s = it.x + (size_t)(row + i * RPI) * ld + k;
+                    if (first + row + i * RPI < it.M && k < p.K) {
+                        const __nv_bfloat16* s = it.x + (size_t)(first + row + i * RPI) * ld + k;
                         v[h][i] = p.x32 ? ldg_v8(s) : ldg_2v4(s);
                         if (PRO == 2) {
                             const V8 b = p.x32 ? ldg_v8(s + p.K) : ldg_2v4(s + p.K), d = p.x32 ? ldg_v8(s + 2 * p.K) : ldg_2v4(s + 2 * p.K);
@@ -442,7 +458,7 @@ __global__ void __launch_bounds__(kThreads, 1) qmv_stream_kernel(const __grid_co
 #pragma unroll
                 for (int i = 0; i < NL; i++) {
                     const int slot = (i * RPI + lane / CPR) * 4 + tt, j = h * XP + 2 * pr;
-                    if (row0 + i * RPI >= it.M) break;  // (rows past M: their columns of the result are never stored)
+                    if (first + row0 + i * RPI >= it.M) break;  // (rows past M: their columns of the result are never stored)
                     sts_v4(frag_addr(j, slot), permute_x8<BITS>(make_uint4(v[h][i].v[0], v[h][i].v[1], v[h][i].v[2], v[h][i].v[3])));
                     sts_v4(frag_addr(j + 1, slot), permute_x8<BITS>(make_uint4(v[h][i].v[4], v[h][i].v[5], v[h][i].v[6], v[h][i].v[7])));
                 }
@@ -466,7 +482,7 @@ __global__ void __launch_bounds__(kThreads, 1) qmv_stream_kernel(const __grid_co
             asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
             waited = true;
         };
-        if (NI > 1 || !p.x_early) wait_prev();
+        if (NI != 1 || !p.x_early) wait_prev();
 
         // this lane's place in the stage that comes next: 16-byte pieces 2t and 2t+1 of row g of the k-block
         const uint32_t in_tile = kq * 2048 + g * 128 + (((2 * t) ^ g) << 4), sa0 = ring + tsub * p.tile_bytes + in_tile;
@@ -550,7 +566,7 @@ __global__ void __launch_bounds__(kThreads, 1) qmv_stream_kernel(const __grid_co
 
 // ---- host side ------------------------------------------------------------------------------------------------------
 struct Plan {
-    int gshift, nkb, n_rt, grid, nch, kbc, ts, tb, stages, stage_bytes, tile_bytes, sb_off, xs_off, run_off, bar_off;
+    int gshift, nkb, n_rt, grid, grid_y, nch, kbc, ts, tb, stages, stage_bytes, tile_bytes, sb_off, xs_off, run_off, bar_off;
     size_t smem;
 };
 
@@ -564,6 +580,7 @@ bool make_plan(const QmmArgs& a, int mmax, int sm_count, Plan* pl) {
     pl->n_rt = (a.N + 15) / 16;
     if ((long long)a.N * (a.K / a.group) > (1ll << 30) || (long long)pl->n_rt * pl->nkb > (1ll << 26)) return false;  // 32-bit indices
     pl->grid = std::min(pl->n_rt, sm_count);
+    pl->grid_y = 1;
     const int tiles_max = (pl->n_rt + pl->grid - 1) / pl->grid;
     pl->nch = (pl->nkb + kWarps - 1) / kWarps;
     pl->kbc = (pl->nkb + pl->nch - 1) / pl->nch;
@@ -624,7 +641,7 @@ cudaError_t launch_t(const Params<NI>& p, const Plan& pl, cudaStream_t stream, b
         attr_set[dev & 63].store(true, std::memory_order_relaxed);
     }
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(pl.grid);
+    cfg.gridDim = dim3(pl.grid, pl.grid_y);
     cfg.blockDim = dim3(kThreads);
     cfg.dynamicSmemBytes = pl.smem;
     cfg.stream = stream;
@@ -638,27 +655,23 @@ cudaError_t launch_t(const Params<NI>& p, const Plan& pl, cudaStream_t stream, b
     return cudaLaunchKernelEx(&cfg, kern, p);
 }
 
-template <int BITS, int NI>
-cudaError_t launch_bits(const Params<NI>& p, const Plan& pl, int mmax, int spl, int pro, cudaStream_t stream, bool overlap_prev) {
-    if (mmax > 8) {
-        if (BITS == 4 && spl == 2) return launch_t<BITS, 2, BITS == 4 ? 2 : 1, 0, NI>(p, pl, stream, overlap_prev);
-        return launch_t<BITS, 2, 1, 0, NI>(p, pl, stream, overlap_prev);
+template <int BITS, int SPL, int NI>
+cudaError_t launch_rows(const Params<NI>& p, const Plan& pl, int mmax, int pro, cudaStream_t stream, bool overlap_prev) {
+    if constexpr (NI > 0) {
+        constexpr int P1 = NI == 1 ? 1 : 0, P2 = NI == 1 ? 2 : 0;  // (prologues: single calls only)
+        if (mmax <= 8)
+            return pro == 1   ? launch_t<BITS, 1, SPL, P1, NI>(p, pl, stream, overlap_prev)
+                   : pro == 2 ? launch_t<BITS, 1, SPL, P2, NI>(p, pl, stream, overlap_prev)
+                              : launch_t<BITS, 1, SPL, 0, NI>(p, pl, stream, overlap_prev);
     }
-    constexpr int P1 = NI == 1 ? 1 : 0, P2 = NI == 1 ? 2 : 0;  // (prologues: single calls only)
-    if (BITS == 4 && spl == 2) {
-        constexpr int S = BITS == 4 ? 2 : 1;
-        return pro == 1 ? launch_t<BITS, 1, S, P1, NI>(p, pl, stream, overlap_prev)
-             : pro == 2 ? launch_t<BITS, 1, S, P2, NI>(p, pl, stream, overlap_prev) : launch_t<BITS, 1, S, 0, NI>(p, pl, stream, overlap_prev);
-    }
-    return pro == 1 ? launch_t<BITS, 1, 1, P1, NI>(p, pl, stream, overlap_prev)
-         : pro == 2 ? launch_t<BITS, 1, 1, P2, NI>(p, pl, stream, overlap_prev) : launch_t<BITS, 1, 1, 0, NI>(p, pl, stream, overlap_prev);
+    return launch_t<BITS, 2, SPL, 0, NI>(p, pl, stream, overlap_prev);
 }
 
 template <int NI>
 cudaError_t launch_items(const QmmArgs* items, int n, int mmax, const Plan& pl, cudaStream_t stream, bool overlap_prev, bool x_stable) {
     const QmmArgs& a0 = items[0];
     Params<NI> p;
-    p.n_items = n;
+    p.n_items = p.kRows ? (a0.M + kItemRows - 1) / kItemRows : n;
     p.K = a0.K; p.N = a0.N; p.gshift = pl.gshift; p.y_bf16 = a0.y_dtype == LUX_DTYPE_BFLOAT16;
     p.rt_q = pl.n_rt / pl.grid; p.rt_rem = pl.n_rt % pl.grid;
     p.ts_inv = (65536 + pl.ts - 1) / pl.ts; p.kbc_inv = (65536 + pl.kbc - 1) / pl.kbc;
@@ -676,16 +689,16 @@ cudaError_t launch_items(const QmmArgs* items, int n, int mmax, const Plan& pl, 
         p.items[i] = Item{(const __nv_bfloat16*)items[i].x, (const __nv_bfloat16*)items[i].scales,
                           (const __nv_bfloat16*)items[i].biases, items[i].y, items[i].M};
     }
-    const int spl = a0.bits == 4 && a0.group == 32 ? 2 : 1;
-    return a0.bits == 4 ? launch_bits<4, NI>(p, pl, mmax, spl, a0.pro, stream, overlap_prev)
-                        : launch_bits<8, NI>(p, pl, mmax, spl, a0.pro, stream, overlap_prev);
+    return a0.bits == 8     ? launch_rows<8, 1, NI>(p, pl, mmax, a0.pro, stream, overlap_prev)
+           : a0.group == 32 ? launch_rows<4, 2, NI>(p, pl, mmax, a0.pro, stream, overlap_prev)
+                            : launch_rows<4, 1, NI>(p, pl, mmax, a0.pro, stream, overlap_prev);
 }
 
 }  // namespace
 
 bool qmv_stream_supported(const QmmArgs& a, int sm_count) {
     Plan pl;
-    if (!make_plan(a, a.M, sm_count, &pl)) return false;
+    if (!make_plan(a, std::min(a.M, kItemRows), sm_count, &pl)) return false;
     // the rms-norm prologue needs the whole of x in the first fragments of the CTA's warps
     return !a.pro || (a.M <= 8 && (a.pro == 2 || pl.nch == 1));
 }
@@ -705,10 +718,12 @@ cudaError_t launch_qmv_stream(const QmmArgs* items, int n, int sm_count, cudaStr
         if (((uintptr_t)a.wq | (uintptr_t)a.x | (uintptr_t)a.scales | (uintptr_t)a.biases) & 15) return cudaErrorInvalidValue;
     }
     Plan pl;
-    if (!make_plan(a0, mmax, sm_count, &pl)) return cudaErrorNotSupported;
+    if ((n > 1 && mmax > kItemRows) || !make_plan(a0, std::min(mmax, kItemRows), sm_count, &pl)) return cudaErrorNotSupported;
+    if (mmax > kItemRows) pl.grid_y = std::min((a0.M + kItemRows - 1) / kItemRows, sm_count / pl.grid);
     if (a0.pro && (mmax > 8 || (a0.pro == 1 && pl.nch != 1))) return cudaErrorNotSupported;
-    return n == 1 ? launch_items<1>(items, n, mmax, pl, stream, overlap_prev, x_stable)
-                  : launch_items<kMaxBatch>(items, n, mmax, pl, stream, overlap_prev, x_stable);
+    return mmax > kItemRows ? launch_items<0>(items, n, mmax, pl, stream, overlap_prev, x_stable)
+         : n == 1           ? launch_items<1>(items, n, mmax, pl, stream, overlap_prev, x_stable)
+                            : launch_items<kMaxBatch>(items, n, mmax, pl, stream, overlap_prev, x_stable);
 }
 
 }  // namespace luxcuda

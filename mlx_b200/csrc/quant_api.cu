@@ -132,31 +132,18 @@ LuxBackendError qmatmul_on_stream(Context* c, const QmmArgs& a) {
             LuxBackendError le = ensure_qmm_workspace(c);
             if (le != LUX_BACKEND_OK) return le;
             e = launch_qmm_tc(a, c->qmm_ws->ptr, c->dev->sm_count, c->stream, &name);
-        } else {
-            // decode kernel, 16 rows of x per launch
-            QmmArgs chunk = a;
-            chunk.M = a.M < 16 ? a.M : 16;
-            if (qmv_mma_supported(chunk, c->dev->sm_count) || qmv_stream_supported(chunk, c->dev->sm_count)) {
-                const size_t ws = qmv_mma_workspace_bytes(chunk, c->dev->sm_count);
-                LuxBackendError le = ensure_qmv_workspace(c, ws);
-                if (le != LUX_BACKEND_OK) return le;
-                const size_t ysz = dtype_size(a.y_dtype);
-                launches = 0;
-                for (int m0 = 0; m0 < a.M && e == cudaSuccess; m0 += 16) {
-                    chunk.M = a.M - m0 < 16 ? a.M - m0 : 16;
-                    chunk.x = (const char*)a.x + (size_t)m0 * a.K * 2;
-                    chunk.y = (char*)a.y + (size_t)m0 * a.N * ysz;
-                    overlaps = decode_may_overlap(c, chunk);
-                    e = launch_qmv_mma(chunk, c->qmv_ws ? c->qmv_ws->ptr : nullptr, c->dev->sm_count, c->stream, &name, overlaps,
-                                       nullptr, decode_x_stable(c, chunk));
-                    if (e == cudaSuccess) {
-                        c->launches++;
-                        note_decode_launch(c, chunk);
-                    }
-                }
-            } else {
-                e = launch_qmv_simt(a, c->stream, &name);
+        } else if (qmv_mma_supported(a, c->dev->sm_count) || qmv_stream_supported(a, c->dev->sm_count)) {
+            LuxBackendError le = ensure_qmv_workspace(c, qmv_mma_workspace_bytes(a, c->dev->sm_count));
+            if (le != LUX_BACKEND_OK) return le;
+            launches = 0;
+            overlaps = decode_may_overlap(c, a);
+            e = launch_qmv_mma(a, c->qmv_ws ? c->qmv_ws->ptr : nullptr, c->dev->sm_count, c->stream, &name, overlaps, nullptr, decode_x_stable(c, a));
+            if (e == cudaSuccess) {
+                c->launches++;
+                note_decode_launch(c, a);
             }
+        } else {
+            e = launch_qmv_simt(a, c->stream, &name);
         }
     } else {
         launches = 0;

@@ -195,6 +195,21 @@ def test_fallback_shapes_bf16(ctx, oracle):
         check(oracle, y, x, wq, s, b, bits, group, oracle.BF16)
 
 
+@pytest.mark.parametrize("bits", [4, 8])
+@pytest.mark.parametrize("M,K,N", [(17, 96, 16), (32, 32, 5), (33, 992, 300), (500, 96, 16), (70, 2912, 2500), (2400, 32, 1)])
+def test_many_rows_where_the_prefill_kernel_does_not_apply(ctx, oracle, bits, M, K, N):
+    """K no multiple of 64: any number of rows is one launch, whose items of 16 rows have the bits of calls of their own."""
+    wq, s, b = oracle.make_layer(N, K, bits, 32, oracle.BF16, config_id=16)
+    x = oracle.make_x(M, K, oracle.BF16, config_id=16)
+    for y_dtype in (BF16, F32):
+        n0 = ctx.launch_count()
+        y, _ = run_qmatmul(ctx, x, wq, s, b, bits, 32, y_dtype)
+        assert ctx.launch_count() == n0 + 1
+        check(oracle, y, x, wq, s, b, bits, 32, oracle.BF16)
+        for m in sorted({0, 16, M // 2 // 16 * 16, (M - 1) // 16 * 16}):
+            assert np.array_equal(y[m:m + 16], run_qmatmul(ctx, x[m:m + 16], wq, s, b, bits, 32, y_dtype)[0])
+
+
 @pytest.mark.parametrize("bits,group,K", [(4, 32, 32), (4, 32, 288), (4, 32, 4128), (4, 64, 320), (4, 128, 640), (8, 32, 32), (8, 64, 192), (8, 32, 2080)])
 @pytest.mark.parametrize("M", [1, 9])
 def test_infinite_weights_in_the_last_group(ctx, oracle, bits, group, K, M):
