@@ -111,34 +111,49 @@ __device__ __forceinline__ void task_mma(const uint32_t (&w)[2][8], const uint32
 // ---- x fragments ----------------------------------------------------------------------------------------------------
 // Fragment j of lane (g, t) covers x[row g][kb*KB + t*KL + 8j .. +8), as the unpack orders the weights:
 //   4-bit: (0,4) (1,5) (2,6) (3,7)      8-bit: (0,2) (1,3) (4,6) (5,7)
-__device__ __forceinline__ uint4 ldg_nc_v4(const void* src) {
-    uint4 v;
-    asm volatile("ld.global.nc.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(src));
-    return v;
+struct V8 {
+    uint32_t v[8];
+};
+__device__ __forceinline__ V8 ldg_v8(const void* p) {  // 32 bytes, through L1 as an earlier launch's output (no .nc)
+    V8 r;
+    asm volatile("ld.global.v8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                 : "=r"(r.v[0]), "=r"(r.v[1]), "=r"(r.v[2]), "=r"(r.v[3]), "=r"(r.v[4]), "=r"(r.v[5]), "=r"(r.v[6]), "=r"(r.v[7])
+                 : "l"(p));
+    return r;
 }
+
+__device__ __forceinline__ V8 ldg_2v4(const void* p) {  // the same from a 16-byte boundary
+    V8 r;
+    asm volatile("ld.global.v4.b32 {%0,%1,%2,%3}, [%4];" : "=r"(r.v[0]), "=r"(r.v[1]), "=r"(r.v[2]), "=r"(r.v[3]) : "l"(p));
+    asm volatile("ld.global.v4.b32 {%0,%1,%2,%3}, [%4];" : "=r"(r.v[4]), "=r"(r.v[5]), "=r"(r.v[6]), "=r"(r.v[7]) : "l"((const char*)p + 16));
+    return r;
+}
+__device__ __forceinline__ V8 ldg_32(const void* p, bool aligned) { return aligned ? ldg_v8(p) : ldg_2v4(p); }
 __device__ __forceinline__ uint32_t add3_bf16x2(uint32_t a, uint32_t b, uint32_t c) {
     const float lo = __fadd_rn(__fadd_rn(__uint_as_float(a << 16), __uint_as_float(b << 16)), __uint_as_float(c << 16));
     const float hi = __fadd_rn(__fadd_rn(__uint_as_float(a & 0xFFFF0000u), __uint_as_float(b & 0xFFFF0000u)), __uint_as_float(c & 0xFFFF0000u));
     const __nv_bfloat162 r = __floats2bfloat162_rn(lo, hi);
     return *reinterpret_cast<const uint32_t*>(&r);
 }
-// The fragments of k-block kb of one row of x (row = nullptr: a row past M, zeros), in natural k order; k >= K reads as
-// zero.  PRO 2: bf16(a + b + c) of the column blocks [0,K), [K,2K), [2K,3K) (fp32 adds, left to right, one rounding: the
-// bits of the stand-alone sum3 kernel).
+// The fragments of k-block kb (all of it inside K) of one row of x (row = nullptr: a row past M, zeros), in natural k order;
+// x32: rows start on 32-byte boundaries.  PRO 2: bf16(a + b + c) of the column blocks [0,K), [K,2K), [2K,3K) (fp32 adds, left to
+// right, one rounding: the bits of the stand-alone sum3 kernel).
 template <int BITS, int PRO>
-__device__ __forceinline__ void load_x_row(const __nv_bfloat16* row, int K, int kb, int t, uint4 (&xr)[x_frags(BITS)]) {
+__device__ __forceinline__ void load_x_row(const __nv_bfloat16* row, int K, int kb, int t, bool x32, uint4 (&xr)[x_frags(BITS)]) {
     const int k0 = kb * kb_weights(BITS) + t * lane_weights(BITS);
 #pragma unroll
-    for (int j = 0; j < x_frags(BITS); j++) {
-        xr[j] = make_uint4(0, 0, 0, 0);
-        if (row && k0 + 8 * j < K) {
+    for (int j = 0; j < x_frags(BITS); j += 2) {
+        xr[j] = xr[j + 1] = make_uint4(0, 0, 0, 0);
+        if (row) {
             const __nv_bfloat16* src = row + k0 + 8 * j;
-            xr[j] = ldg_nc_v4(src);
+            V8 v = ldg_32(src, x32);
             if (PRO == 2) {
-                const uint4 b = ldg_nc_v4(src + K), c = ldg_nc_v4(src + 2 * K);
-                xr[j] = make_uint4(add3_bf16x2(xr[j].x, b.x, c.x), add3_bf16x2(xr[j].y, b.y, c.y), add3_bf16x2(xr[j].z, b.z, c.z),
-                                   add3_bf16x2(xr[j].w, b.w, c.w));
+                const V8 b = ldg_32(src + K, x32), c = ldg_32(src + 2 * K, x32);
+#pragma unroll
+                for (int e = 0; e < 8; e++) v.v[e] = add3_bf16x2(v.v[e], b.v[e], c.v[e]);
             }
+            xr[j] = make_uint4(v.v[0], v.v[1], v.v[2], v.v[3]);
+            xr[j + 1] = make_uint4(v.v[4], v.v[5], v.v[6], v.v[7]);
         }
     }
 }

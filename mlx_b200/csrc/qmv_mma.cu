@@ -17,8 +17,9 @@
 //     with 16 rows of x), filled with cp.async (16-byte pieces, L1 bypass): the
 //     tasks ahead of the one being computed (2.5 KiB each) are in flight, with no
 //     registers tied up and no block-wide barrier in the streaming loop;
-//   * lane (g = lane/4, t = lane%4) copies and later reads back exactly its own
-//     pieces: bytes [32t, 32t+32) of rows g and g+8 of the k-block;
+//   * lane (g = lane/4, t = lane%4) copies pieces t and t+4 of rows g and g+8 of the
+//     k-block (64 bytes side by side per quad and instruction) and reads pieces 2t and
+//     2t+1 (piece_slot);
 //   * weights are dequantised in registers and multiplied with mma.sync (qmv_frag.cuh);
 //     the x fragments of the warp's k-block are loaded once, into registers;
 //   * every task leaves a 16 x 8*MT fp32 partial in shared memory; at the end
@@ -62,6 +63,15 @@ __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commi
 template <int N>
 __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
 
+// Where lane (g, t) finds the first of its two pieces of row g in a stage, the second being at the address ^ 16.  (Lane l
+// writes its first piece to slot l and its second to slot l ^ 1 of the next 512 bytes: no bank conflicts either way.
+// Copying the pieces that it reads, 32 bytes of each row per quad and lane, two requests for every sector, cost up to a
+// tenth of a launch whose K is split.)
+__device__ __forceinline__ uint32_t piece_slot(int lane) {
+    const int g = lane >> 2, t = lane & 3;
+    return (t >> 1) * 512 + ((g * 64 + (t & 1) * 32) ^ (t & 2 ? 16 : 0));
+}
+
 struct Params {
     const __nv_bfloat16* x;
     const uint32_t* wq;
@@ -81,6 +91,7 @@ struct Params {
     int sb_bytes;            // bytes of scales per row per k-block: 2, 4, 8 or 16
     int ld, col0;            // y row stride and first column (elements): N and 0 unless the layer is column-sharded
     int x_early;             // x is not written by the previous kernel of the stream: it may be read before the wait for it
+    int x32;                 // every row of x starts on a 32-byte boundary (callers owe 16 bytes only)
     int x_ld;                // row stride of x in elements (K unless a prologue reads column blocks of a wider buffer)
     float eps;               // of the rms-norm prologue
     long long peer_wait_ns;  // limit of a wait for a peer (column-sharded launches)
@@ -318,7 +329,7 @@ __global__ void __launch_bounds__(kThreads, 1) qmv_mma_kernel(const __grid_const
     constexpr int KB = 1024 / BITS;        // weights per k-block (128 bytes per row)
     constexpr int E4 = MT * 32;            // float4 per partial
     constexpr int D = ring_depth(MT);      // ring stages of a warp
-    extern __shared__ __align__(16) unsigned char smem[];
+    extern __shared__ __align__(128) unsigned char smem[];
     float4* part = reinterpret_cast<float4*>(smem + ring_bytes(MT));   // [tb][nkl][MT][32]; ring: [kWarps][D][kStageBytes]
     // after the partials (MT == 2): the x fragments of rows 8..15, [warp][fragment][lane]
     uint4* xs = reinterpret_cast<uint4*>(smem + p.xs_off) + (threadIdx.x >> 5) * (XV * 32) + (threadIdx.x & 31);
@@ -335,7 +346,7 @@ __global__ void __launch_bounds__(kThreads, 1) qmv_mma_kernel(const __grid_const
     const size_t row_bytes = (size_t)p.K * BITS / 8;
     const int gpr = p.K >> p.gshift;   // groups per row
     const int gpk = KB >> p.gshift;    // groups per k-block
-    const unsigned char* wbase = reinterpret_cast<const unsigned char*>(p.wq) + t * 32;
+    const unsigned char* wbase = reinterpret_cast<const unsigned char*>(p.wq) + t * 16;
     const __nv_bfloat16* sb_src = lane < 16 ? p.scales : p.biases;
     const uint32_t ring_lo = smem_u32(smem) + warp * (D * kStageBytes) + lane * 16;  // this lane's slot, stage 0
     const int tail_tile = (p.N & 15) ? p.n_rt - 1 : -1;  // the tile whose rows must be clamped to N-1
@@ -347,7 +358,7 @@ __global__ void __launch_bounds__(kThreads, 1) qmv_mma_kernel(const __grid_const
     const size_t half_tile = 8 * row_bytes, tile_stride = 16 * row_bytes;
     int f_b0 = rt_lo, f_kb = kb_lo + warp, f_rt = rt_lo;  // the task fetched next
     uint32_t f_dst = ring_lo;                             // and the stage it goes to
-    // this lane's sources of that task: rows g and g+8 of the tile (its 32 bytes of the k-block),
+    // this lane's sources of that task: rows g and g+8 of the tile (its two pieces of the k-block),
     // the scales (lanes 0-15) or biases (16-31) of row lane%16.  Inside a run they move by constant strides.
     const unsigned char* f_p0 = nullptr;
     const unsigned char* f_p1 = nullptr;
@@ -368,9 +379,9 @@ __global__ void __launch_bounds__(kThreads, 1) qmv_mma_kernel(const __grid_const
     auto fetch_next = [&]() {
         if (has_work && f_b0 < rt_hi) {
             cp_async16(f_dst, f_p0);
-            cp_async16(f_dst + 512, f_p0 + 16);
+            cp_async16((f_dst ^ 16) + 512, f_p0 + 64);
             cp_async16(f_dst + 1024, f_p1);
-            cp_async16(f_dst + 1536, f_p1 + 16);
+            cp_async16((f_dst ^ 16) + 1536, f_p1 + 64);
             if (p.sb_bytes == 16) cp_async16(f_dst + 2048, f_sb);
             else if (p.sb_bytes == 8) cp_async8(f_dst + 2048, f_sb);
             else cp_async4(f_dst + 2048, reinterpret_cast<const void*>(reinterpret_cast<uintptr_t>(f_sb) & ~uintptr_t(3)));  // a lone scale travels with its neighbour
@@ -406,7 +417,7 @@ __global__ void __launch_bounds__(kThreads, 1) qmv_mma_kernel(const __grid_const
 #pragma unroll
         for (int mt = 0; mt < MT; mt++) {
             const int m = mt * 8 + g;
-            load_x_row<BITS, PRO>(m < p.M ? p.x + (size_t)m * (PRO == 0 ? p.K : p.x_ld) : nullptr, p.K, kb, t, xr[mt]);
+            load_x_row<BITS, PRO>(m < p.M ? p.x + (size_t)m * (PRO == 0 ? p.K : p.x_ld) : nullptr, p.K, kb, t, p.x32, xr[mt]);
         }
     };
     if (kXFirst && p.x_early && has_work) load_x(kb_lo + warp);
@@ -453,7 +464,8 @@ __global__ void __launch_bounds__(kThreads, 1) qmv_mma_kernel(const __grid_const
         rms_scale<XV>(xr[0], rms_inv);
     }
 
-    uint32_t src_c = ring_lo;  // stage of the task computed next (this lane's slot)
+    const uint32_t src_lo = ring_lo - lane * 16 + piece_slot(lane);
+    uint32_t src_c = src_lo;   // stage of the task computed next (this lane's first piece)
     uint32_t sboff[2][SPL];    // byte offsets of this lane's scales inside a stage, by row half r
 #pragma unroll 1
     for (int b0 = rt_lo; b0 < rt_hi; b0 += tb) {
@@ -480,7 +492,7 @@ __global__ void __launch_bounds__(kThreads, 1) qmv_mma_kernel(const __grid_const
                     const int par = p.sb_bytes == 2 ? ((slot * gpr + kb) & 1) : 0;
 #pragma unroll
                     for (int i = 0; i < SPL; i++)
-                        sboff[r][i] = 2048 - lane * 16 + slot * 16 + ((((t * KL + i * 32) >> p.gshift) + par) << 1);
+                        sboff[r][i] = 2048 - piece_slot(lane) + slot * 16 + ((((t * KL + i * 32) >> p.gshift) + par) << 1);
                 }
                 if (p.sp.world > 1 && tid < p.sp.world && tid != p.sp.me)
                     ready_early = ld_relaxed_sys(p.sp.flags[p.sp.me] + kFlagReady + tid);  // used at the first push
@@ -498,7 +510,7 @@ __global__ void __launch_bounds__(kThreads, 1) qmv_mma_kernel(const __grid_const
                         for (int h = 0; h < 2; h++)
                             asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];"
                                          : "=r"(w[r][4 * h]), "=r"(w[r][4 * h + 1]), "=r"(w[r][4 * h + 2]), "=r"(w[r][4 * h + 3])
-                                         : "r"(src_c + (r * 2 + h) * 512));
+                                         : "r"((h ? src_c ^ 16 : src_c) + r * 1024));
 #pragma unroll
                         for (int i = 0; i < SPL; i++) {
                             asm volatile("ld.shared.u16 %0, [%1];" : "=r"(s[r][i]) : "r"(src_c + sboff[r][i]));
@@ -513,7 +525,7 @@ __global__ void __launch_bounds__(kThreads, 1) qmv_mma_kernel(const __grid_const
                     for (int mt = 0; mt < MT; mt++) dstp[mt * 32] = out[mt];
                     dstp += nkl * E4;
                     __syncwarp();  // every lane is done with the stage before it is refilled
-                    src_c = src_c + kStageBytes == ring_lo + D * kStageBytes ? ring_lo : src_c + kStageBytes;
+                    src_c = src_c + kStageBytes == src_lo + D * kStageBytes ? src_lo : src_c + kStageBytes;
                 }
             }
         }
@@ -570,6 +582,7 @@ struct BatchParams {
     int n_items;
     int K, N, gshift, y_bf16;
     int nkb, n_rt, chunks, tb, sb_bytes, xs_off;
+    int x32;  // see Params (K is a multiple of 128 here)
     BatchItem items[kMaxBatch];
     // N is this rank's share of the columns
     int ld, col0, yt_off;
@@ -628,7 +641,7 @@ __global__ void __launch_bounds__(kThreads, 1) qmv_batch_kernel(const __grid_con
     constexpr int D = DEEP ? kDeepDepth : ring_depth(MT);       // ring stages of a warp
     constexpr int kStageBytes = DEEP ? kDeepStageBytes : luxcuda::kStageBytes;
     constexpr int kSlot = DEEP ? 8 : 16;                         // bytes of a row's scales (and of its biases) in a stage
-    extern __shared__ __align__(16) unsigned char smem[];
+    extern __shared__ __align__(128) unsigned char smem[];
     float4* part = reinterpret_cast<float4*>(smem + kWarps * D * kStageBytes);   // [tb][nkl][MT][32]; ring: [kWarps][D][kStageBytes]
     // after the partials (MT == 2): the x fragments of rows 8..15, [warp][fragment][lane]
     uint4* xs = reinterpret_cast<uint4*>(smem + p.xs_off) + (threadIdx.x >> 5) * (XV * 32) + (threadIdx.x & 31);
@@ -668,7 +681,7 @@ __global__ void __launch_bounds__(kThreads, 1) qmv_batch_kernel(const __grid_con
     const int gpk = KB >> p.gshift;    // groups per k-block
     // the matmul whose weights are being fetched (f_pi) runs ahead of the one being computed (pi)
     int f_pi = 0;
-    const unsigned char* wbase = reinterpret_cast<const unsigned char*>(p.items[0].wq) + t * 32;
+    const unsigned char* wbase = reinterpret_cast<const unsigned char*>(p.items[0].wq) + t * 16;
     const __nv_bfloat16* sb_src = lane < 16 ? p.items[0].scales : p.items[0].biases;
     const uint32_t ring_lo = smem_u32(smem) + warp * (D * kStageBytes) + lane * 16;  // this lane's slot, stage 0
     const int tail_tile = (p.N & 15) ? p.n_rt - 1 : -1;  // the tile whose rows must be clamped to N-1
@@ -680,7 +693,7 @@ __global__ void __launch_bounds__(kThreads, 1) qmv_batch_kernel(const __grid_con
     const size_t half_tile = 8 * row_bytes, tile_stride = 16 * row_bytes;
     int f_b0 = rt_lo, f_kb = kb_lo + warp, f_rt = rt_lo;  // the task fetched next
     uint32_t f_dst = ring_lo;                             // and the stage it goes to
-    // this lane's sources of that task: rows g and g+8 of the tile (its 32 bytes of the k-block),
+    // this lane's sources of that task: rows g and g+8 of the tile (its two pieces of the k-block),
     // the scales (lanes 0-15) or biases (16-31) of row lane%16.  Inside a run they move by constant strides.
     const unsigned char* f_p0 = nullptr;
     const unsigned char* f_p1 = nullptr;
@@ -701,9 +714,9 @@ __global__ void __launch_bounds__(kThreads, 1) qmv_batch_kernel(const __grid_con
     auto fetch_next = [&]() {
         if (has_work && f_pi < p.n_items) {
             cp_async16(f_dst, f_p0);
-            cp_async16(f_dst + 512, f_p0 + 16);
+            cp_async16((f_dst ^ 16) + 512, f_p0 + 64);
             cp_async16(f_dst + 1024, f_p1);
-            cp_async16(f_dst + 1536, f_p1 + 16);
+            cp_async16((f_dst ^ 16) + 1536, f_p1 + 64);
             const uint32_t sb_dst = f_dst + 2048 - lane * (16 - kSlot);  // (f_dst is this lane's 16-byte slot of the stage)
             if (!DEEP && p.sb_bytes == 16) cp_async16(sb_dst, f_sb);
             else if (p.sb_bytes == 8) cp_async8(sb_dst, f_sb);
@@ -719,7 +732,7 @@ __global__ void __launch_bounds__(kThreads, 1) qmv_batch_kernel(const __grid_con
                 if (f_b0 >= f_hi && ++f_pi < p.n_items) {  // on to the next matmul: the next range of tiles, its weights
                     next_range(f_c, f_lo, f_hi, f_acc);
                     f_b0 = f_lo;
-                    wbase = reinterpret_cast<const unsigned char*>(p.items[f_pi].wq) + t * 32;
+                    wbase = reinterpret_cast<const unsigned char*>(p.items[f_pi].wq) + t * 16;
                     sb_src = lane < 16 ? p.items[f_pi].scales : p.items[f_pi].biases;
                 }
                 f_rt = f_b0;
@@ -741,7 +754,7 @@ __global__ void __launch_bounds__(kThreads, 1) qmv_batch_kernel(const __grid_con
 #pragma unroll
         for (int mt = 0; mt < MT; mt++) {
             const int m = mt * 8 + g;
-            load_x_row<BITS, 0>(m < M ? x + (size_t)m * p.K : nullptr, p.K, kb, t, xr[mt]);
+            load_x_row<BITS, 0>(m < M ? x + (size_t)m * p.K : nullptr, p.K, kb, t, p.x32, xr[mt]);
         }
     };
 #pragma unroll
@@ -756,7 +769,8 @@ __global__ void __launch_bounds__(kThreads, 1) qmv_batch_kernel(const __grid_con
     }
     unsigned char* const ytiles = smem + p.yt_off;
     const int yt_bytes = p.y_bf16 ? 512 : 1024;  // of a staged tile
-    uint32_t src_c = ring_lo;  // stage of the task computed next (this lane's slot)
+    const uint32_t src_lo = ring_lo - lane * 16 + piece_slot(lane);
+    uint32_t src_c = src_lo;   // stage of the task computed next (this lane's first piece)
     uint32_t sboff[2][SPL];    // byte offsets of this lane's scales inside a stage, by row half r
 #pragma unroll 1
     for (int pi = 0; pi < p.n_items; pi++) {
@@ -786,7 +800,7 @@ __global__ void __launch_bounds__(kThreads, 1) qmv_batch_kernel(const __grid_con
                     const int par = p.sb_bytes == 2 ? ((slot * gpr + kb) & 1) : 0;
 #pragma unroll
                     for (int i = 0; i < SPL; i++)
-                        sboff[r][i] = 2048 - lane * 16 + slot * kSlot + ((((t * KL + i * 32) >> p.gshift) + par) << 1);
+                        sboff[r][i] = 2048 - piece_slot(lane) + slot * kSlot + ((((t * KL + i * 32) >> p.gshift) + par) << 1);
                 }
                 float4* dstp = part + (kb - kb_lo) * E4 + lane;
 #pragma unroll 1
@@ -802,7 +816,7 @@ __global__ void __launch_bounds__(kThreads, 1) qmv_batch_kernel(const __grid_con
                         for (int h = 0; h < 2; h++)
                             asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];"
                                          : "=r"(w[r][4 * h]), "=r"(w[r][4 * h + 1]), "=r"(w[r][4 * h + 2]), "=r"(w[r][4 * h + 3])
-                                         : "r"(src_c + (r * 2 + h) * 512));
+                                         : "r"((h ? src_c ^ 16 : src_c) + r * 1024));
 #pragma unroll
                         for (int i = 0; i < SPL; i++) {
                             asm volatile("ld.shared.u16 %0, [%1];" : "=r"(s[r][i]) : "r"(src_c + sboff[r][i]));
@@ -817,7 +831,7 @@ __global__ void __launch_bounds__(kThreads, 1) qmv_batch_kernel(const __grid_con
                     for (int mt = 0; mt < MT; mt++) dstp[mt * 32] = out[mt];
                     dstp += nkl * E4;
                     __syncwarp();  // every lane is done with the stage before it is refilled
-                    src_c = src_c + kStageBytes == ring_lo + D * kStageBytes ? ring_lo : src_c + kStageBytes;
+                    src_c = src_c + kStageBytes == src_lo + D * kStageBytes ? src_lo : src_c + kStageBytes;
                 }
             }
         }
@@ -1043,6 +1057,7 @@ cudaError_t launch_qmv_mma(const QmmArgs& a, void* workspace, int sm_count, cuda
     p.ld = a.N; p.col0 = 0;
     p.x_early = (!overlap_prev || x_stable) ? 1 : 0;
     p.x_ld = a.pro ? a.x_ld : a.K;
+    p.x32 = ((uintptr_t)a.x & 31) == 0 && p.x_ld % 16 == 0;
     p.eps = a.eps;
     if (a.pro) {
         // prologues: M <= 8; the rms-norm needs the whole of x in the first fragments of the CTA's warps
@@ -1122,8 +1137,10 @@ cudaError_t launch_qmv_batch(const QmmArgs* items, int n, int sm_count, cudaStre
     p.K = a0.K; p.N = a0.N; p.gshift = pl.gshift;
     p.y_bf16 = a0.y_dtype == LUX_DTYPE_BFLOAT16;
     p.nkb = pl.nkb; p.n_rt = pl.n_rt; p.chunks = pl.chunks; p.tb = pl.tb; p.sb_bytes = pl.sb_bytes; p.xs_off = pl.xs_off;
+    p.x32 = 1;
     for (int i = 0; i < n; i++) {
         const QmmArgs& a = items[i];
+        if ((uintptr_t)a.x & 31) p.x32 = 0;
         if (a.K != a0.K || a.N != a0.N || a.bits != a0.bits || a.group != a0.group || a.y_dtype != a0.y_dtype ||
             a.x_dtype != LUX_DTYPE_BFLOAT16 || a.sb_dtype != LUX_DTYPE_BFLOAT16 || a.M < 1 || (a.M <= 8) != (mmax <= 8) || a.pro)
             return cudaErrorNotSupported;

@@ -120,24 +120,6 @@ __device__ __forceinline__ void add_f32x4(uint4& s, const uint4& v) {
         "  add.rn.f32x2 a, a, c; add.rn.f32x2 b, b, d; mov.b64 {%0, %1}, a; mov.b64 {%2, %3}, b; }"
         : "+r"(s.x), "+r"(s.y), "+r"(s.z), "+r"(s.w) : "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w));
 }
-struct V8 {
-    uint32_t v[8];
-};
-__device__ __forceinline__ V8 ldg_v8(const void* p) {  // 32 bytes, through L1 as an earlier launch's output (no .nc)
-    V8 r;
-    asm volatile("ld.global.v8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
-                 : "=r"(r.v[0]), "=r"(r.v[1]), "=r"(r.v[2]), "=r"(r.v[3]), "=r"(r.v[4]), "=r"(r.v[5]), "=r"(r.v[6]), "=r"(r.v[7])
-                 : "l"(p));
-    return r;
-}
-
-__device__ __forceinline__ V8 ldg_2v4(const void* p) {  // the same from a 16-byte boundary
-    V8 r;
-    asm volatile("ld.global.v4.b32 {%0,%1,%2,%3}, [%4];" : "=r"(r.v[0]), "=r"(r.v[1]), "=r"(r.v[2]), "=r"(r.v[3]) : "l"(p));
-    asm volatile("ld.global.v4.b32 {%0,%1,%2,%3}, [%4];" : "=r"(r.v[4]), "=r"(r.v[5]), "=r"(r.v[6]), "=r"(r.v[7]) : "l"((const char*)p + 16));
-    return r;
-}
-
 constexpr int kItemRows = 16;  // rows of x of an item, at most (more of one matmul: several items, see Params)
 struct Item {
     const __nv_bfloat16* x;
@@ -444,9 +426,9 @@ __global__ void __launch_bounds__(kThreads, 1) qmv_stream_kernel(const __grid_co
                     for (int e = 0; e < 8; e++) v[h][i].v[e] = 0;
                     if (first + row + i * RPI < it.M && k < p.K) {
                         const __nv_bfloat16* s = it.x + (size_t)(first + row + i * RPI) * ld + k;
-                        v[h][i] = p.x32 ? ldg_v8(s) : ldg_2v4(s);
+                        v[h][i] = ldg_32(s, p.x32);
                         if (PRO == 2) {
-                            const V8 b = p.x32 ? ldg_v8(s + p.K) : ldg_2v4(s + p.K), d = p.x32 ? ldg_v8(s + 2 * p.K) : ldg_2v4(s + 2 * p.K);
+                            const V8 b = ldg_32(s + p.K, p.x32), d = ldg_32(s + 2 * p.K, p.x32);
 #pragma unroll
                             for (int e = 0; e < 8; e++) v[h][i].v[e] = add3_bf16x2(v[h][i].v[e], b.v[e], d.v[e]);
                         }
