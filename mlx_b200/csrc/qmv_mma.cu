@@ -906,6 +906,7 @@ __global__ void __launch_bounds__(kThreads, 1) qmv_batch_kernel(const __grid_con
 
 struct Plan {
     int nkb, n_rt, mt, chunks, ks, tb, gshift, sb_bytes, xs_off, yt_off;
+    bool ks_forced;  // by LUXCUDA_QMV_KSPLIT
     size_t smem, scratch_bytes;
 };
 
@@ -936,8 +937,9 @@ bool make_plan(const QmmArgs& a, int sm_count, Plan* pl, bool sharded = false, s
     // CTA's 16 warps would each still own more than one k-block
     int ks = 1;
     if (pl->n_rt * 2 <= sm_count) ks = std::max(1, std::min((pl->nkb + kWarps - 1) / kWarps, sm_count / pl->n_rt));
+    pl->ks_forced = false;
     if (const char* env = getenv("LUXCUDA_QMV_KSPLIT"))
-        if (pl->n_rt <= kMaxSplitTiles) ks = std::max(1, std::min(atoi(env), pl->nkb));
+        if (pl->n_rt <= kMaxSplitTiles) pl->ks_forced = true, ks = std::max(1, std::min(atoi(env), pl->nkb));
     if (pl->n_rt > kMaxSplitTiles) ks = 1;
     pl->ks = ks;
     pl->chunks = std::max(1, std::min(pl->n_rt, sm_count / ks));
@@ -1024,7 +1026,13 @@ static const char* variant_name(int bits, int mt, int pro) {
 }
 
 // Launches of their own CTAs' whole K on one GPU go to qmv_stream.cu; this file's kernel takes the launches whose K is
-// split over CTAs and those that deliver y to peers.
+// split over CTAs and those that deliver y to peers.  Of the splits, one in two (37 to 74 row tiles, or K of 17 to 32 k-blocks)
+// is mostly better off there, too: a CTA then reads twice as much, but nothing has to travel through scratch.  Measured, us,
+// split here / whole there, 1024 rows of W, 4 bit: 1 row of x, 17 and 64 k-blocks 6.6/3.2 and 9.3/7.5; 8 rows, 64, 96, 128
+// k-blocks 10.5/10.2, 13.3/14.5, 16.2/19.3; 16 rows, 32 and 128 k-blocks 9.9/6.8 and 30.0/26.1.  (Split in three, 512 rows of W:
+// 33 k-blocks 6.1/4.9 with 1 row of x, but 48 with 8 rows 6.8/7.6: the line is drawn at two.)
+static bool split_pays(const Plan& pl) { return pl.ks > 2 || (pl.ks == 2 && (pl.ks_forced || (pl.mt == 1 && pl.nkb > 64))); }
+
 // workspace layout: [counters: kCounterBytes][partials]; the counters must be zero before the
 // first launch and are left zero by every launch.
 cudaError_t launch_qmv_mma(const QmmArgs& a, void* workspace, int sm_count, cudaStream_t stream, const char** name,
@@ -1032,7 +1040,7 @@ cudaError_t launch_qmv_mma(const QmmArgs& a, void* workspace, int sm_count, cuda
     Plan pl;
     const bool sharded = push && push->world > 1;
     const bool on_grid = make_plan(a, sm_count, &pl, sharded);
-    if (!sharded && (!on_grid || pl.ks == 1)) {
+    if (!sharded && (!on_grid || !split_pays(pl))) {
         // (the name: a K off the k-block grid belongs to the family that callers know for such shapes)
         if (name) *name = on_grid ? variant_name(a.bits, a.M <= 8 ? 1 : 2, a.pro) : a.bits == 4 ? "qmv_simt<4,bf16,mma>" : "qmv_simt<8,bf16,mma>";
         return launch_qmv_stream(&a, 1, sm_count, stream, overlap_prev, x_stable);

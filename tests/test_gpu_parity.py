@@ -115,7 +115,8 @@ def test_decode_sweep_shape(ctx, oracle, M):
 def test_decode_workspace_shared_between_split_shapes(ctx, oracle):
     """Two K-split shapes with different tile counts, one after the other on one context: the second must not
     read the first one's partials as arrival counters (the counters sit in a region of fixed size)."""
-    for (M, K, N, bits, group) in ((8, 8192, 64, 4, 64), (1, 8192, 1120, 4, 64), (8, 16384, 1024, 4, 64), (1, 8192, 1120, 4, 64)):
+    for (M, K, N, bits, group) in ((8, 8192, 64, 4, 64), (1, 8192, 1120, 4, 64), (8, 16384, 1024, 4, 64), (1, 8192, 1120, 4, 64),
+                                   (8, 16384, 64, 4, 64), (1, 16640, 1120, 4, 64), (8, 12288, 752, 4, 64), (16, 16384, 64, 4, 64), (1, 16640, 1120, 4, 64)):
         wq, s, b = oracle.make_layer(N, K, bits, group, oracle.BF16, config_id=2, layer=K, proj=N)
         x = oracle.make_x(M, K, oracle.BF16, config_id=2, layer=K, tag=M)
         y, kern = run_qmatmul(ctx, x, wq, s, b, bits, group, BF16)
@@ -431,6 +432,24 @@ def test_dispatch_rereads_its_parameter_buffer_only_when_it_changed(ctx, plugin,
     v.kernel_destroy(ctx.handle, k)
     for h in (bx, bw, bs, bb, y, want8):
         h.free()
+
+
+@pytest.mark.parametrize("M", [1, 8, 9, 16])
+@pytest.mark.parametrize("K,N,bits,group", [(16384, 592, 4, 64), (16384, 608, 4, 64), (16640, 1184, 4, 128), (12288, 784, 4, 32), (8192, 16, 8, 128), (4224, 1184, 8, 64)])
+def test_k_split_gives_the_bits_of_whole_k(ctx, oracle, M, K, N, bits, group):
+    """On both sides of the rules for splitting K over CTAs (rows of W, k-blocks, rows of x): the bits of a launch that has too
+    many rows of W for a split, and those of x off the 32-byte grid."""
+    wq, s, b = oracle.make_layer(N, K, bits, group, oracle.BF16, config_id=17, layer=K)
+    x = oracle.make_x(M, K, oracle.BF16, config_id=17, tag=M)
+    y, _ = run_qmatmul(ctx, x, wq, s, b, bits, group, F32)
+    check(oracle, y, x, wq, s, b, bits, group, oracle.BF16)
+    rep = -(-1300 // N)
+    whole, _ = run_qmatmul(ctx, x, *(np.tile(a, (rep, 1)) for a in (wq, s, b)), bits, group, F32)
+    assert np.array_equal(whole[:, :N], y) and np.array_equal(whole[:, -N:], y)
+    keep, bx = _off(ctx, x, 16)
+    bw, bs, bb, by = ctx.upload(wq), ctx.upload(s), ctx.upload(b), ctx.empty((M, N), np.float32)
+    ctx.qmatmul(bx, bw, bs, bb, by, M, K, N, bits, group, BF16, BF16, F32)
+    assert np.array_equal(by.to_host(), y)
 
 
 def test_more_rows_than_one_pass_of_the_decode_kernel(ctx, oracle):

@@ -28,6 +28,7 @@ SHAPES = [
     (8, 8192, 64, 4, 64),       # few rows, long K: K is split, partials travel through the scratch
     (16, 4096, 96, 8, 128),     # 8-bit, split
     (3, 1024, 100, 4, 32),
+    (8, 16384, 64, 4, 64),      # split in four
 ]
 
 
@@ -91,7 +92,8 @@ def test_noalloc_scratch_shared_between_split_shapes(plugin, ctx, oracle):
     the first again.  Each must give the bits of the ordinary qmatmul on a fresh context."""
     fresh = plugin.context(0)
     try:
-        for (M, K, N, bits, group) in ((8, 8192, 64, 4, 64), (1, 8192, 1120, 4, 64), (8, 8192, 64, 4, 64), (1, 8192, 1120, 4, 64)):
+        for (M, K, N, bits, group) in ((8, 8192, 64, 4, 64), (1, 8192, 1120, 4, 64), (8, 8192, 64, 4, 64), (1, 8192, 1120, 4, 64),
+                                       (8, 16384, 64, 4, 64), (1, 16640, 1120, 4, 64), (8, 16384, 64, 4, 64), (1, 16640, 1120, 4, 64)):
             wq, s, b = oracle.make_layer(N, K, bits, group, oracle.BF16, config_id=13, layer=K, proj=N)
             x = oracle.make_x(M, K, oracle.BF16, config_id=13, tag=M)
             fx, fw, fs, fb = fresh.upload(x), fresh.upload(wq), fresh.upload(s), fresh.upload(b)
