@@ -44,15 +44,13 @@ struct GemmPlan {
 // Tile height: the matrix instruction's N.  One CTA's (M = 128) takes multiples of 16.  The pair's (M = 256, A in tensor
 // memory) is documented for multiples of 32 only, so a pair's tiles are that high whatever is left of M.
 //
-// Schedule and height go by a rough estimate of the time in microseconds, not a fit: the order of the three kernels on
-// the shapes that were timed (32 to 512 tiles), with errors of up to a third for low tiles (48 rows: 0.64 us a stage
-// measured, 0.50 here).  A k-stage of a tile costs about 0.45 + 0.001 * bm whatever the kernel (dequantisation, then the
+// Schedule and height go by a rough estimate of the time in microseconds, not a fit: on 392 shapes (32 to 2048 rows, K 512 to
+// 8192, N 256 to 11008) it takes the fastest of the three kernels or one within 4 % of it on 377, within 20 % at worst, but
+// the times themselves are off by up to a third for low tiles (48 rows: 0.64 us a stage measured, 0.50 here).  A k-stage of a tile costs about 0.45 + 0.001 * bm whatever the kernel (dequantisation, then the
 // MMAs), so a lower tile pays where it saves no round of tiles: 777 x 2880 x 5003 took 35.6 us in 208-row tiles and
 // 30.8 in 112-row ones, two rounds either way.
 //   whole tiles: ceil(T/G) rounds, each with an epilogue of 3 * bm/256 that nothing else overlaps;
-//   CTA pairs:   rounds of pair tiles; the epilogue overlaps where y leaves by TMA; 3 to set up; 0.1 more per stage for
-//                groups of 32, whose scales outgrow the L1 that this kernel leaves (from one shape, 777 rows: 35.4
-//                against 30.8 us);
+//   CTA pairs:   rounds of pair tiles; the epilogue overlaps where y leaves by TMA; 3 to set up;
 //   stream-K:    T*nst/G stages of up to 1.6 times the cost, an epilogue more, and the exchange of partials.
 inline bool choose_gemm_plan(const GemmShape& a, int sm_count, const GemmForce& force, bool no_ytma, GemmPlan* pl) {
     pl->n_tiles = (a.N + kTileN - 1) / kTileN;
@@ -74,7 +72,7 @@ inline bool choose_gemm_plan(const GemmShape& a, int sm_count, const GemmForce& 
             } else if (k == 1) {
                 if (sm_count & 1) continue;
                 const double prounds = std::ceil((pl->n_tiles + 1) / 2 * (double)mt / (sm_count / 2));
-                cost = 3.0 + prounds * (nst * (stage + (a.group == 32 ? 0.1 : 0.0)) + (y_fast ? 0.5 : e));
+                cost = 3.0 + prounds * (nst * stage + (y_fast ? 0.5 : e));
             } else {
                 if (T * nst < G && !(force.streamk == 1 && mt == m0)) continue;
                 cost = 2.0 + (1.1 + 0.5 * h) * T * nst / G * stage + (rounds + 1.0) * e + 4.0 * h * (T < G ? std::ceil(G / T) : 1.0);

@@ -58,3 +58,11 @@ def test_every_plan_can_be_launched(plan):
 def test_an_odd_number_of_sms_has_no_pairs(plan):
     assert plan(2048, 4096, 4096, sms=147, streamk=0, pair=1) is None
     assert plan(2048, 4096, 4096, sms=147)["pair"] == 0
+
+
+@pytest.mark.parametrize("group", [32, 64, 128])
+def test_many_rows_take_pairs_whatever_the_group(plan, group):
+    """2048 x 2880 x 11008 and 2048 x 1024 x 4096 in groups of 32: 100 and 21 us by pairs, 108 and 23 by single CTAs."""
+    for K, N in ((2880, 11008), (1024, 4096)):
+        if K % group == 0:
+            assert plan(2048, K, N, group=group)["pair"] == 1
