@@ -236,7 +236,7 @@ void note_chain_launch(Context* c, const void* out, size_t out_bytes);  // right
 void note_decode_launch(Context* c, const QmmArgs& a);  // call right after a decode launch, before counting it
 // decode / small-M, any supported dtype combination: CUDA cores + warp shuffles
 // overlap_prev (fp32 only): as above
-cudaError_t launch_qmv_simt(const QmmArgs& a, cudaStream_t stream, const char** name, bool overlap_prev = false);
+cudaError_t launch_qmv_simt(const QmmArgs& a, int sm_count, cudaStream_t stream, const char** name, bool overlap_prev = false);
 // several decode matmuls of one shape (M on one side of 8) as one persistent launch; at most qmv_batch_max() items
 int qmv_batch_max();
 // push (column-sharded layer, world > 1): every item's y lies inside this rank's symmetric buffer and the launch

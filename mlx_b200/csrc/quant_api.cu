@@ -143,12 +143,12 @@ LuxBackendError qmatmul_on_stream(Context* c, const QmmArgs& a) {
                 note_decode_launch(c, a);
             }
         } else {
-            e = launch_qmv_simt(a, c->stream, &name);
+            e = launch_qmv_simt(a, c->dev->sm_count, c->stream, &name);
         }
     } else {
         launches = 0;
         overlaps = decode_may_overlap(c, a);
-        e = launch_qmv_simt(a, c->stream, &name, overlaps);
+        e = launch_qmv_simt(a, c->dev->sm_count, c->stream, &name, overlaps);
         if (e == cudaSuccess) {
             c->launches++;
             note_decode_launch(c, a);

@@ -161,6 +161,25 @@ def test_fp32_edges(ctx, oracle, bits, group, M):
             assert (np.abs(y - t) <= K * 2.0 ** -24 * mag + 1e-30).all()
 
 
+@pytest.mark.parametrize("bits", [4, 8])
+@pytest.mark.parametrize("K", [256, 512, 1024, 2048, 4128, 8192])
+def test_fp32_rows_and_columns_are_independent(ctx, oracle, bits, K):
+    """One row of x and one row of W have the same bits whatever the other rows are: 1 to 40 rows of x, few and many rows of W
+    (also x off the 32-byte grid)."""
+    N, group = 6000, 32
+    wq, s, b = oracle.make_layer(N, K, bits, group, oracle.F32, config_id=18, layer=K)
+    x = oracle.make_x(40, K, oracle.F32, config_id=18)
+    full, _ = run_qmatmul(ctx, x, wq, s, b, bits, group, F32)
+    for m0, M in ((0, 1), (39, 1), (7, 2), (1, 3), (4, 4), (30, 8), (11, 17)):
+        for n0, n in ((0, N), (0, 300), (1500, 1500), (N - 5, 5)):
+            y, _ = run_qmatmul(ctx, x[m0:m0 + M], wq[n0:n0 + n], s[n0:n0 + n], b[n0:n0 + n], bits, group, F32)
+            assert np.array_equal(y, full[m0:m0 + M, n0:n0 + n]), (m0, M, n0, n)
+    keep, bx = _off(ctx, x[:2], 16)
+    bw, bs, bb, by = ctx.upload(wq), ctx.upload(s), ctx.upload(b), ctx.empty((2, N), np.float32)
+    ctx.qmatmul(bx, bw, bs, bb, by, 2, K, N, bits, group, F32, F32, F32)
+    assert np.array_equal(by.to_host(), full[:2])
+
+
 def test_fp32_launches_back_to_back(ctx, oracle):
     """fp32 matmuls fed by one another without a synchronisation (each fetches its weights while the one before it runs):
     the bits of the same calls one at a time."""
