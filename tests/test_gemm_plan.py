@@ -66,3 +66,10 @@ def test_many_rows_take_pairs_whatever_the_group(plan, group):
     for K, N in ((2880, 11008), (1024, 4096)):
         if K % group == 0:
             assert plan(2048, K, N, group=group)["pair"] == 1
+
+
+def test_smoke_runs_each_of_the_three_kernels(plan):
+    import __graft_entry__
+    for name, (M, K, N) in __graft_entry__.SMOKE_PREFILL.items():
+        p = plan(M, K, N)
+        assert name == ("qmm_tc<4,stream-k>" if p["streamk"] else "qmm_tc<4,pairs>" if p["pair"] else "qmm_tc<4>")
