@@ -54,7 +54,8 @@ static_assert(kDqGroups == kStagesB, "a group always owns the same slot (and its
 constexpr int kTmaWarp = kEpiWarps + kDqWarps, kMmaWarp = kTmaWarp + 1, kWWarp = kMmaWarp + 1;
 constexpr int kNumThreads = (kWWarp + 1) * 32;
 constexpr uint32_t kTmemCols = 512, kAColBase = 256, kAColsPerSub = kBK / 2, kAColsPerSlot = kSub * kAColsPerSub;
-constexpr uint32_t kSpinLimit = 1u << 20;
+constexpr uint32_t kWaitClocks = 4000000000u;
+constexpr uint32_t kSpinLimit = 1u << 22;  // polls of a flag in global memory, 100 ns and more apart
 constexpr size_t kWsFlagBytes = 1024;  // flag words of the stream-K workspace (one per CTA), ahead of the partials
 
 __device__ __forceinline__ uint32_t s32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
@@ -74,14 +75,19 @@ __device__ __forceinline__ bool mbar_try(uint64_t* b, uint32_t parity) {
                  : "=r"(ok) : "r"(s32(b)), "r"(parity), "r"(20000u) : "memory");
     return ok != 0;
 }
-// Bounded wait.  Returns false (and raises *abort_flag) when the barrier does not
-// flip within the limit or another role has already given up.
+// Bounded wait, about two seconds of SM clock (a poll may itself last 20 us: counting polls would not bound it).  Returns
+// false (and raises *abort_flag) when the barrier does not flip within the limit or another role has already given up.
 __device__ __forceinline__ bool mbar_wait(uint64_t* b, uint32_t parity, volatile int* abort_flag) {
-    for (uint32_t i = 0; i < kSpinLimit; i++) {
-        if (mbar_try(b, parity)) return true;
-        if (i > 4) __nanosleep(40);  // waiting roles must not steal issue slots from the working ones
-        if ((i & 1023u) == 1023u && *abort_flag) return false;
-    }
+    if (mbar_try(b, parity)) return true;
+    const uint32_t t0 = clock();
+    uint32_t i = 0;
+    do {
+#pragma unroll 1
+        for (uint32_t end = i + 64; i < end; i++) {
+            if (i > 4) __nanosleep(40);  // waiting roles must not steal issue slots from the working ones
+            if (mbar_try(b, parity)) return true;
+        }
+    } while (!*abort_flag && (uint32_t)clock() - t0 < kWaitClocks);
     *abort_flag = 1;
     return false;
 }
@@ -89,12 +95,22 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* b, uint32_t parity, volatile
 // Same bound, no back-off, for the warp whose wake-up latency is on the tensor pipe's critical path.  Whole warp; the vote
 // makes the answer, and with it the control flow behind it, uniform for the compiler.
 __device__ __forceinline__ bool mbar_wait_warp(uint64_t* b, uint32_t parity, volatile int* abort_flag) {
-    for (uint32_t i = 0; i < kSpinLimit * 8; i++) {
-        if (__all_sync(0xffffffffu, mbar_try(b, parity))) return true;
-        if ((i & 4095u) == 4095u && __any_sync(0xffffffffu, *abort_flag != 0)) return false;
-    }
+    if (__all_sync(0xffffffffu, mbar_try(b, parity))) return true;
+    const uint32_t t0 = clock();
+    do {
+#pragma unroll 1
+        for (uint32_t i = 0; i < 64; i++)
+            if (__all_sync(0xffffffffu, mbar_try(b, parity))) return true;
+    } while (__all_sync(0xffffffffu, !*abort_flag && (uint32_t)clock() - t0 < kWaitClocks));
     *abort_flag = 1;
     return false;
+}
+// After an abort nobody waits for the copies and MMAs in flight any more; before the CTA frees its tensor memory and ends
+// they get two milliseconds, far more than they take.  Every thread, behind the barrier at which all roles have returned.
+__device__ __forceinline__ void settle_after_abort(volatile int* abort_flag) {
+    if (!*abort_flag) return;
+    const uint32_t t0 = clock();
+    while ((uint32_t)clock() - t0 < 4000000u) __nanosleep(1000);
 }
 __device__ __forceinline__ bool elect_one() {  // whole warp: true in one lane, always the same
     uint32_t r;
@@ -631,7 +647,7 @@ qmm_tc_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant_
                     if (et < parts) {
                         const uint32_t* f = p.ws_flags + blockIdx.x + 1 + et;
                         uint32_t v = 0;
-                        for (uint32_t i = 0; i < kSpinLimit * 4; i++) {
+                        for (uint32_t i = 0; i < kSpinLimit; i++) {
                             asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(f) : "memory");
                             if (v || ((i & 1023u) == 1023u && *abort_flag)) break;
                             __nanosleep(100);
@@ -757,6 +773,7 @@ qmm_tc_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant_
     // ---------------- teardown ----------------
     tc_fence_before();
     __syncthreads();
+    settle_after_abort(abort_flag);
     if (tid == 0 && sl->abort_flag) *p.error = 1;
     if (warp == kMmaWarp) {
         tc_fence_after();
@@ -918,6 +935,7 @@ qmm_tc_tiles_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_con
     // ---------------- teardown ----------------
     tc_fence_before();
     __syncthreads();
+    settle_after_abort(abort_flag);
     if (tid == 0 && sl->abort_flag) *p.error = 1;
     if (warp == kMmaWarp) {
         tc_fence_after();
@@ -1194,6 +1212,7 @@ qmm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_cons
     if (tid == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");  // the last tile has left
     tc_fence_before();
     __syncthreads();
+    settle_after_abort(abort_flag);
     cluster_sync();  // neither CTA leaves (or frees tensor memory) while the other may still reach into it
     if (tid == 0 && sl->abort_flag) *p.error = 1;
     if (warp == kMmaWarp) {
