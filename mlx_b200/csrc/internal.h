@@ -183,6 +183,19 @@ struct DeviceGuard {
     }
 };
 
+// Lets the kernel be launched with up to `bytes` of dynamic shared memory, the most that any plan asks for: set once per
+// device, to the same value by whichever thread comes first.  (To each launch's own size, two threads could end with the
+// smaller one set.)
+template <class K>
+cudaError_t allow_smem(K kern, int bytes, std::atomic<bool> (&set)[64]) {
+    int dev = 0;
+    cudaGetDevice(&dev);
+    if (set[dev & 63].load(std::memory_order_relaxed)) return cudaSuccess;
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+    if (e == cudaSuccess) set[dev & 63].store(true, std::memory_order_relaxed);
+    return e;
+}
+
 // ---------------------------------------------------------------------------
 // kernel launchers (each enqueues on `stream`, returns the launch status)
 // ---------------------------------------------------------------------------

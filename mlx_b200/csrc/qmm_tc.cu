@@ -1274,14 +1274,8 @@ bool make_gemm_plan(const QmmArgs& a, int sm_count, const ShardPush* push, GemmP
 template <int BITS>
 cudaError_t launch_gemm_pair_t(const CUtensorMap& tmap, const CUtensorMap& tmap_w, const CUtensorMap& tmap_y, const GemmParams& p, const GemmPlan& pl, int sm_count, cudaStream_t stream) {
     auto kern = qmm_tc_pair_kernel<BITS>;
-    static std::atomic<size_t> attr_smem[64];
-    int dev = 0;
-    cudaGetDevice(&dev);
-    if (attr_smem[dev & 63].load() < pl.smem) {
-        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pl.smem);
-        if (e != cudaSuccess) return e;
-        attr_smem[dev & 63].store(pl.smem);
-    }
+    static std::atomic<bool> attr_set[64];
+    if (cudaError_t e = allow_smem(kern, kGemmSmemLimit, attr_set)) return e;
     // one pair of CTAs per pair of SMs (the kernel carries its cluster shape), unless there are fewer pair tiles
     const int pairs = ((pl.n_tiles + 1) / 2) * pl.m_tiles;
     const int grid = 2 * std::min(sm_count / 2, pairs);
@@ -1292,14 +1286,8 @@ cudaError_t launch_gemm_pair_t(const CUtensorMap& tmap, const CUtensorMap& tmap_
 template <int BITS, bool SK>
 cudaError_t launch_gemm_t(const CUtensorMap& tmap, const CUtensorMap& tmap_w, const GemmParams& p, const GemmPlan& pl, int sm_count, cudaStream_t stream) {
     auto kern = SK ? qmm_tc_kernel<BITS, true> : qmm_tc_tiles_kernel<BITS>;
-    static std::atomic<size_t> attr_smem[64];
-    int dev = 0;
-    cudaGetDevice(&dev);
-    if (attr_smem[dev & 63].load() < pl.smem) {
-        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pl.smem);
-        if (e != cudaSuccess) return e;
-        attr_smem[dev & 63].store(pl.smem);
-    }
+    static std::atomic<bool> attr_set[64];
+    if (cudaError_t e = allow_smem(kern, kGemmSmemLimit, attr_set)) return e;
     // one CTA per SM, unless the launch has fewer units of work (tiles, or k-stages under stream-K) than that
     const long long units = (long long)pl.m_tiles * pl.n_tiles * (SK ? (p.K / kBK + kSub - 1) / kSub : 1);
     const int grid = (int)std::min<long long>(sm_count, units);

@@ -46,7 +46,7 @@ constexpr int kThreads = kWarps * 32;
 constexpr int ring_depth(int mt) { return mt == 1 ? 4 : 2; }
 constexpr int kStageBytes = 2048 + 512;    // 4 x 32 x 16 B of weights + 32 x 16 B of scales/biases
 constexpr int ring_bytes(int mt) { return kWarps * ring_depth(mt) * kStageBytes; }
-constexpr int kSmemLimit = 227 * 1024 - 256;
+constexpr int kSmemLimit = 227 * 1024 - 1024;  // dynamic; the rest is for the static part (up to 640 bytes)
 constexpr int kMaxTb = 32;                 // tiles per reduction batch (flags array)
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
@@ -964,15 +964,8 @@ bool make_plan(const QmmArgs& a, int sm_count, Plan* pl, bool sharded = false, s
 template <int BITS, int MT, int PRO>
 cudaError_t launch_t(const Params& p, const Plan& pl, cudaStream_t stream, bool overlap_prev) {
     auto kern = qmv_mma_kernel<BITS, MT, PRO>;
-    // opt in to large dynamic shared memory (static + dynamic stay within the 227 KiB per-block limit)
-    static std::atomic<size_t> attr_smem[64];
-    int dev = 0;
-    cudaGetDevice(&dev);
-    if (attr_smem[dev & 63].load() < pl.smem) {
-        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pl.smem);
-        if (e != cudaSuccess) return e;
-        attr_smem[dev & 63].store(pl.smem);
-    }
+    static std::atomic<bool> attr_set[64];
+    if (cudaError_t e = allow_smem(kern, kSmemLimit, attr_set)) return e;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(pl.chunks * pl.ks);
     cfg.blockDim = dim3(kThreads);
@@ -1097,14 +1090,8 @@ cudaError_t launch_qmv_mma(const QmmArgs& a, void* workspace, int sm_count, cuda
 template <int BITS, int MT, bool DEEP>
 cudaError_t launch_batch_t(const BatchParams& p, const Plan& pl, cudaStream_t stream) {
     auto kern = qmv_batch_kernel<BITS, MT, DEEP>;
-    static std::atomic<size_t> attr_smem[64];
-    int dev = 0;
-    cudaGetDevice(&dev);
-    if (attr_smem[dev & 63].load() < pl.smem) {
-        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pl.smem);
-        if (e != cudaSuccess) return e;
-        attr_smem[dev & 63].store(pl.smem);
-    }
+    static std::atomic<bool> attr_set[64];
+    if (cudaError_t e = allow_smem(kern, kSmemLimit, attr_set)) return e;
     kern<<<pl.chunks, kThreads, pl.smem, stream>>>(p);
     return cudaGetLastError();
 }

@@ -615,13 +615,7 @@ template <int BITS, int MT, int SPL, int PRO, int NI>
 cudaError_t launch_t(const Params<NI>& p, const Plan& pl, cudaStream_t stream, bool overlap_prev) {
     auto kern = qmv_stream_kernel<BITS, MT, SPL, PRO, NI>;
     static std::atomic<bool> attr_set[64];
-    int dev = 0;
-    cudaGetDevice(&dev);
-    if (!attr_set[dev & 63].load(std::memory_order_relaxed)) {
-        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemLimit);
-        if (e != cudaSuccess) return e;
-        attr_set[dev & 63].store(true, std::memory_order_relaxed);
-    }
+    if (cudaError_t e = allow_smem(kern, kSmemLimit, attr_set)) return e;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(pl.grid, pl.grid_y);
     cfg.blockDim = dim3(kThreads);

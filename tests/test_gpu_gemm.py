@@ -1,6 +1,10 @@
 """Prefill-regime GEMM (tcgen05 + TMEM) against the oracle, through the C ABI.
 Same bars as the decode tests: outputs within 1e-2 (bf16 compute) of the
 fp64-accumulated truth over the same bf16 dequantised weights."""
+import os
+import subprocess
+import sys
+
 import numpy as np
 import pytest
 
@@ -162,3 +166,44 @@ def test_odd_stage_counts_on_every_schedule(ctx, oracle, monkeypatch, schedule, 
     y, kern = run_qmatmul(ctx, x, wq, s, b, bits, group, BF16)
     assert kern.startswith("qmm_tc"), kern
     check(oracle, y, x, wq, s, b, bits, group, oracle.BF16)
+
+
+THREADS = r"""
+import sys, threading
+sys.path.insert(0, %r)
+import numpy as np
+import mlx_b200
+import oracle as O
+from mlx_b200 import BF16
+plugin = mlx_b200.Plugin(require_gpu=True)
+K, N = 512, 512
+wq, s, b = O.make_layer(N, K, 4, 64, O.BF16, config_id=3)
+gate, failed = threading.Barrier(12), []
+
+def work(i):
+    ctx = plugin.context(0)
+    M = (4, 12, 32, 64, 128, 256)[i %% 6] if i < 6 else 20 + 18 * i
+    x = O.make_x(M, K, O.BF16, config_id=3, tag=M)
+    bx, bw, bs, bb, by = ctx.upload(x), ctx.upload(wq), ctx.upload(s), ctx.upload(b), ctx.empty((M, N), np.uint16)
+    gate.wait()
+    try:
+        for _ in range(20):
+            ctx.qmatmul(bx, bw, bs, bb, by, M, K, N, 4, 64, BF16, BF16, BF16)
+        err, _ = O.rel_err(by.to_host(), O.qmatmul_truth(x, wq, s, b, 4, 64))
+        assert err <= O.TOL[O.BF16], err
+    except Exception as e:
+        failed.append((M, repr(e)))
+
+ts = [threading.Thread(target=work, args=(i,)) for i in range(12)]
+[t.start() for t in ts]
+[t.join() for t in ts]
+print("FAILED", failed)
+"""
+
+
+@pytest.mark.parametrize("run", range(3))
+def test_first_launches_from_many_threads(run):
+    """Twelve threads, a context each, whose first launches of a kernel ask for different amounts of shared memory."""
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    r = subprocess.run([sys.executable, "-c", THREADS % root], capture_output=True, text=True, timeout=120, cwd=root)
+    assert r.returncode == 0 and "FAILED []" in r.stdout, (r.stdout[-800:], r.stderr[-800:])
