@@ -1170,7 +1170,7 @@ def run_ours(args, rank, world):
                          "each launch reads a set last touched 11 launches earlier"},
         "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
                      "peak_source": which, "frac_of_nominal_8TBps": achieved / NOMINAL_HBM_GBS,
-                     "kernel": ("qmv_batch<4,m8|m16>" if world == 1 else "qmv_batch<4,m8|m16,push>") if use_batch else "qmv_mma<4,m8|m16>",
+                     "kernel": ("qmv_batch<4,m8|m16>" if world == 1 else "qmv_batch<4,m8|m16,push>") if use_batch else "qmv_mma<4,m8|m16,stream>" if world == 1 else "qmv_mma<4,m8|m16>",
                      ("avg_us_per_matmul" if use_batch else "avg_us_per_launch"): avg_us,
                      "alg_bytes_per_launch": {str(M): alg_bytes(M) for M in M_SWEEP},
                      **({"traffic": NCU_TRAFFIC_BYTES_BATCH, "alg_bytes_of_that_launch": R_SETS * sum(alg_bytes(M) for M in M_SWEEP if M <= 8),

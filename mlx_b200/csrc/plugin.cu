@@ -486,14 +486,24 @@ void fill_vtbl() {
 // Directory of the kernels compiled into the library, in the format of the reference's kernel registry
 // (include/lux/gpu/kernel_loader.h:70-90).  name = kernel family, entry_point = variant.
 const LuxEmbeddedKernel g_kernels[] = {
-    {LUX_CUDA_QMM_KERNEL_NAME, "qmv_mma<4,m8>", LUX_KERNEL_LANG_CUDA, nullptr, 0, nullptr, 0},   // decode GEMV, 4-bit, M <= 8
-    {LUX_CUDA_QMM_KERNEL_NAME, "qmv_mma<4,m16>", LUX_KERNEL_LANG_CUDA, nullptr, 0, nullptr, 0},  // decode GEMV, 4-bit, M <= 16
-    {LUX_CUDA_QMM_KERNEL_NAME, "qmv_mma<4,m8,rms>", LUX_KERNEL_LANG_CUDA, nullptr, 0, nullptr, 0},   // x = rms-norm of the buffer, applied as it is loaded
-    {LUX_CUDA_QMM_KERNEL_NAME, "qmv_mma<4,m8,sum3>", LUX_KERNEL_LANG_CUDA, nullptr, 0, nullptr, 0},  // x = sum of three column blocks
+    {LUX_CUDA_QMM_KERNEL_NAME, "qmv_mma<4,m8,stream>", LUX_KERNEL_LANG_CUDA, nullptr, 0, nullptr, 0},  // decode, M <= 8: weights through the copy engine
+    {LUX_CUDA_QMM_KERNEL_NAME, "qmv_mma<4,m8,stream,rms>", LUX_KERNEL_LANG_CUDA, nullptr, 0, nullptr, 0},  // x = rms-norm of the buffer, applied as it is loaded
+    {LUX_CUDA_QMM_KERNEL_NAME, "qmv_mma<4,m8,stream,sum3>", LUX_KERNEL_LANG_CUDA, nullptr, 0, nullptr, 0},  // x = sum of three column blocks
+    {LUX_CUDA_QMM_KERNEL_NAME, "qmv_mma<4,m16,stream>", LUX_KERNEL_LANG_CUDA, nullptr, 0, nullptr, 0},  // M <= 16
+    {LUX_CUDA_QMM_KERNEL_NAME, "qmv_mma<4,rows,stream>", LUX_KERNEL_LANG_CUDA, nullptr, 0, nullptr, 0},  // any M, where the prefill GEMM does not apply
+    {LUX_CUDA_QMM_KERNEL_NAME, "qmv_mma<8,m8,stream>", LUX_KERNEL_LANG_CUDA, nullptr, 0, nullptr, 0},
+    {LUX_CUDA_QMM_KERNEL_NAME, "qmv_mma<8,m8,stream,rms>", LUX_KERNEL_LANG_CUDA, nullptr, 0, nullptr, 0},
+    {LUX_CUDA_QMM_KERNEL_NAME, "qmv_mma<8,m8,stream,sum3>", LUX_KERNEL_LANG_CUDA, nullptr, 0, nullptr, 0},
+    {LUX_CUDA_QMM_KERNEL_NAME, "qmv_mma<8,m16,stream>", LUX_KERNEL_LANG_CUDA, nullptr, 0, nullptr, 0},
+    {LUX_CUDA_QMM_KERNEL_NAME, "qmv_mma<8,rows,stream>", LUX_KERNEL_LANG_CUDA, nullptr, 0, nullptr, 0},
+    {LUX_CUDA_QMM_KERNEL_NAME, "qmv_mma<4,m8>", LUX_KERNEL_LANG_CUDA, nullptr, 0, nullptr, 0},  // the decode kernel for K split over CTAs and for column-sharded layers
+    {LUX_CUDA_QMM_KERNEL_NAME, "qmv_mma<4,m16>", LUX_KERNEL_LANG_CUDA, nullptr, 0, nullptr, 0},
+    {LUX_CUDA_QMM_KERNEL_NAME, "qmv_mma<4,m8,rms>", LUX_KERNEL_LANG_CUDA, nullptr, 0, nullptr, 0},
+    {LUX_CUDA_QMM_KERNEL_NAME, "qmv_mma<4,m8,sum3>", LUX_KERNEL_LANG_CUDA, nullptr, 0, nullptr, 0},
     {LUX_CUDA_QMM_KERNEL_NAME, "qmv_mma<8,m8>", LUX_KERNEL_LANG_CUDA, nullptr, 0, nullptr, 0},
+    {LUX_CUDA_QMM_KERNEL_NAME, "qmv_mma<8,m16>", LUX_KERNEL_LANG_CUDA, nullptr, 0, nullptr, 0},
     {LUX_CUDA_QMM_KERNEL_NAME, "qmv_mma<8,m8,rms>", LUX_KERNEL_LANG_CUDA, nullptr, 0, nullptr, 0},
     {LUX_CUDA_QMM_KERNEL_NAME, "qmv_mma<8,m8,sum3>", LUX_KERNEL_LANG_CUDA, nullptr, 0, nullptr, 0},
-    {LUX_CUDA_QMM_KERNEL_NAME, "qmv_mma<8,m16>", LUX_KERNEL_LANG_CUDA, nullptr, 0, nullptr, 0},
     {LUX_CUDA_QMM_KERNEL_NAME, "qmv_batch<4,m8>", LUX_KERNEL_LANG_CUDA, nullptr, 0, nullptr, 0},  // several decode matmuls of one shape per launch
     {LUX_CUDA_QMM_KERNEL_NAME, "qmv_batch<4,m16>", LUX_KERNEL_LANG_CUDA, nullptr, 0, nullptr, 0},
     {LUX_CUDA_QMM_KERNEL_NAME, "qmv_batch<8,m8>", LUX_KERNEL_LANG_CUDA, nullptr, 0, nullptr, 0},
@@ -508,7 +518,7 @@ const LuxEmbeddedKernel g_kernels[] = {
     {LUX_CUDA_QMM_KERNEL_NAME, "qmm_tc<8,stream-k>", LUX_KERNEL_LANG_CUDA, nullptr, 0, nullptr, 0},
     {LUX_CUDA_QMM_KERNEL_NAME, "qmm_tc<4,pairs>", LUX_KERNEL_LANG_CUDA, nullptr, 0, nullptr, 0},     // the same on pairs of CTAs (cta_group::2)
     {LUX_CUDA_QMM_KERNEL_NAME, "qmm_tc<8,pairs>", LUX_KERNEL_LANG_CUDA, nullptr, 0, nullptr, 0},
-    {LUX_CUDA_QMM_KERNEL_NAME, "qmv_simt", LUX_KERNEL_LANG_CUDA, nullptr, 0, nullptr, 0},        // fp32 activations, odd K
+    {LUX_CUDA_QMM_KERNEL_NAME, "qmv_simt", LUX_KERNEL_LANG_CUDA, nullptr, 0, nullptr, 0},        // fp32 activations; bf16 past the index ranges of the others
     {"lux.qmm.dequantize", "dequantize", LUX_KERNEL_LANG_CUDA, nullptr, 0, nullptr, 0},
     {"lux.qmm.unpack", "unpack", LUX_KERNEL_LANG_CUDA, nullptr, 0, nullptr, 0},
     {"lux.qmm.quantize", "quantize", LUX_KERNEL_LANG_CUDA, nullptr, 0, nullptr, 0},

@@ -1018,6 +1018,13 @@ static const char* variant_name(int bits, int mt, int pro) {
     return mt == 2 ? "qmv_mma<8,m16>" : pro == 1 ? "qmv_mma<8,m8,rms>" : pro == 2 ? "qmv_mma<8,m8,sum3>" : "qmv_mma<8,m8>";
 }
 
+static const char* stream_name(int bits, int M, int pro) {
+    if (bits == 4) return M > 16 ? "qmv_mma<4,rows,stream>" : M > 8 ? "qmv_mma<4,m16,stream>" : pro == 1 ? "qmv_mma<4,m8,stream,rms>"
+                        : pro == 2 ? "qmv_mma<4,m8,stream,sum3>" : "qmv_mma<4,m8,stream>";
+    return M > 16 ? "qmv_mma<8,rows,stream>" : M > 8 ? "qmv_mma<8,m16,stream>" : pro == 1 ? "qmv_mma<8,m8,stream,rms>"
+         : pro == 2 ? "qmv_mma<8,m8,stream,sum3>" : "qmv_mma<8,m8,stream>";
+}
+
 // Launches of their own CTAs' whole K on one GPU go to qmv_stream.cu; this file's kernel takes the launches whose K is
 // split over CTAs and those that deliver y to peers.  Of the splits, one in two (37 to 74 row tiles, or K of 17 to 32 k-blocks)
 // is mostly better off there, too: a CTA then reads twice as much, but nothing has to travel through scratch.  Measured, us,
@@ -1034,8 +1041,7 @@ cudaError_t launch_qmv_mma(const QmmArgs& a, void* workspace, int sm_count, cuda
     const bool sharded = push && push->world > 1;
     const bool on_grid = make_plan(a, sm_count, &pl, sharded);
     if (!sharded && (!on_grid || !split_pays(pl))) {
-        // (the name: a K off the k-block grid belongs to the family that callers know for such shapes)
-        if (name) *name = on_grid ? variant_name(a.bits, a.M <= 8 ? 1 : 2, a.pro) : a.bits == 4 ? "qmv_simt<4,bf16,mma>" : "qmv_simt<8,bf16,mma>";
+        if (name) *name = stream_name(a.bits, a.M, a.pro);
         return launch_qmv_stream(&a, 1, sm_count, stream, overlap_prev, x_stable);
     }
     if (!on_grid) return cudaErrorInvalidValue;

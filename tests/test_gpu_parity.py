@@ -206,13 +206,37 @@ def test_fp32_launches_back_to_back(ctx, oracle):
 
 
 def test_fallback_shapes_bf16(ctx, oracle):
-    """K not a multiple of the tensor-core k-blocks: the CUDA-core kernel takes over."""
+    """K not a multiple of the tensor-core k-blocks: the streaming decode kernel takes them, whose last k-block is cut off."""
     for (M, K, N, bits, group) in ((3, 192, 20, 4, 64), (2, 64, 7, 8, 64), (20, 96, 33, 4, 32)):
         wq, s, b = oracle.make_layer(N, K, bits, group, oracle.BF16, config_id=5)
         x = oracle.make_x(M, K, oracle.BF16, config_id=5)
         y, kern = run_qmatmul(ctx, x, wq, s, b, bits, group, BF16)
-        assert kern.startswith("qmv_simt"), kern
+        assert kern.startswith("qmv_mma") and kern.endswith("stream>"), kern
         check(oracle, y, x, wq, s, b, bits, group, oracle.BF16)
+
+
+@pytest.mark.parametrize("bits", [4, 8])
+def test_index_ranges_past_the_tensor_core_kernels(ctx, oracle, bits):
+    """More than 2^30 groups: the CUDA-core kernel, the only one with 64-bit indices throughout (W is one block of rows over
+    and over, so that the oracle has to do the block alone)."""
+    torch = pytest.importorskip("torch")
+    K, group, rows, reps = 1024, 32, 1031, 32546   # rows * reps * K / group = 2^30 + some
+    N = rows * reps
+    assert 2 ** 30 < N * (K // group) < 2 ** 31
+    wq, s, b = oracle.make_layer(rows, K, bits, group, oracle.BF16, config_id=19)
+    big = [torch.from_numpy(a.view(np.int32 if a.dtype == np.uint32 else np.int16)).cuda().repeat(reps, 1) for a in (wq, s, b)]
+    torch.cuda.synchronize()
+    h = [ctx.wrap(t.data_ptr(), t.numel() * t.element_size()) for t in big]
+    for M in (1, 2, 5):
+        x = oracle.make_x(M, K, oracle.BF16, config_id=19, tag=M)
+        bx, y = ctx.upload(x), torch.empty((M, reps, rows), dtype=torch.float32, device="cuda")
+        ctx.qmatmul(bx, *h, ctx.wrap(y.data_ptr(), y.numel() * 4), M, K, N, bits, group, BF16, BF16, F32)
+        assert ctx.last_kernel() == f"qmv_simt<{bits},bf16>"
+        ctx.sync()
+        assert bool((y == y[:, :1]).all())
+        check(oracle, y[:, 0].cpu().numpy(), x, wq, s, b, bits, group, oracle.BF16)
+    del big, y
+    torch.cuda.empty_cache()
 
 
 @pytest.mark.parametrize("bits", [4, 8])
