@@ -231,17 +231,38 @@ struct ShardPush {
     uint32_t* flags[kMaxShardWorld] = {};   // every rank's flag words (see qmv_mma.cu)
 };
 
-// decode GEMV, bf16 activations: mma.sync m16n8k16 with in-register dequant
+// Decode matmul, bf16 activations: mma.sync m16n8k16 with in-register dequant.  Two kernels: qmv_stream.cu (any K that is a
+// multiple of the group, weights by bulk copies; several matmuls of one shape and one side of M = 8 in one launch, or one of
+// any number of rows) and qmv_mma.cu (K split over CTAs, and column-sharded layers; M <= 16).
+struct QmvSplitPlan {
+    int nkb, n_rt, mt, chunks, ks, tb, gshift, sb_bytes, xs_off, yt_off;
+    bool ks_forced;  // by LUXCUDA_QMV_KSPLIT
+    size_t smem, scratch_bytes;
+};
+struct QmvStreamPlan {
+    int gshift, nkb, n_rt, grid, grid_y, nch, kbc, ts, tb, stages, stage_bytes, tile_bytes, sb_off, xs_off, run_off, bar_off;
+    size_t smem;
+};
+struct DecodePlan {
+    bool on_grid;            // K on the k-blocks of the split kernel: the shapes that prologues and the fixed scratch are for
+    bool split;              // which of the two plans holds
+    size_t workspace_bytes;  // counters and partials (for every shape on the grid)
+    QmvSplitPlan s;
+    QmvStreamPlan st;
+};
+bool plan_decode(const QmmArgs& a, int sm_count, DecodePlan* pl);  // false: for neither kernel
+// the same for a column-sharded layer (a: this rank's columns): always the split kernel's
 bool qmv_mma_supported(const QmmArgs& a, int sm_count);
-// the same without K split or peers, any K (a multiple of the group): weights through bulk copies (qmv_stream.cu);
-// n items of one shape and one side of M = 8 in one launch, or one matmul of any number of rows
-bool qmv_stream_supported(const QmmArgs& a, int sm_count);
-cudaError_t launch_qmv_stream(const QmmArgs* items, int n, int sm_count, cudaStream_t stream, bool overlap_prev, bool x_stable);
 size_t qmv_mma_workspace_bytes(const QmmArgs& a, int sm_count);
+bool plan_qmv_stream(const QmmArgs& a, int sm_count, QmvStreamPlan* pl);
+cudaError_t launch_qmv_stream(const QmmArgs& a, const QmvStreamPlan& pl, cudaStream_t stream, bool overlap_prev, bool x_stable);
+cudaError_t launch_qmv_stream_batch(const QmmArgs* items, int n, int sm_count, cudaStream_t stream);
 // overlap_prev: launch as a programmatic dependent of the previous kernel in the stream (see Context);
 // x_stable: that previous kernel does not write x, which may then be read before the wait for it
-cudaError_t launch_qmv_mma(const QmmArgs& a, void* workspace, int sm_count, cudaStream_t stream, const char** name,
-                           bool overlap_prev = false, const ShardPush* push = nullptr, bool x_stable = false);
+cudaError_t launch_decode(const QmmArgs& a, const DecodePlan& pl, void* workspace, cudaStream_t stream, const char** name,
+                          bool overlap_prev, bool x_stable);
+cudaError_t launch_qmv_push(const QmmArgs& a, void* workspace, int sm_count, cudaStream_t stream, const char** name,
+                            bool overlap_prev, const ShardPush& push);
 bool decode_may_overlap(const Context* c, const QmmArgs& a);
 bool decode_x_stable(const Context* c, const QmmArgs& a);  // the last chain kernel's output does not overlap x
 bool chain_is_open(const Context* c);  // the last thing the context enqueued is a chain kernel (decode matmul, rms-norm)

@@ -904,11 +904,7 @@ __global__ void __launch_bounds__(kThreads, 1) qmv_batch_kernel(const __grid_con
     }
 }
 
-struct Plan {
-    int nkb, n_rt, mt, chunks, ks, tb, gshift, sb_bytes, xs_off, yt_off;
-    bool ks_forced;  // by LUXCUDA_QMV_KSPLIT
-    size_t smem, scratch_bytes;
-};
+using Plan = QmvSplitPlan;
 
 // Arrival counters of k-split tiles live at the head of the workspace in a region of fixed size, so that
 // launches of different shapes that share a workspace agree on where the counters end and the partials begin.
@@ -937,9 +933,12 @@ bool make_plan(const QmmArgs& a, int sm_count, Plan* pl, bool sharded = false, s
     // CTA's 16 warps would each still own more than one k-block
     int ks = 1;
     if (pl->n_rt * 2 <= sm_count) ks = std::max(1, std::min((pl->nkb + kWarps - 1) / kWarps, sm_count / pl->n_rt));
-    pl->ks_forced = false;
-    if (const char* env = getenv("LUXCUDA_QMV_KSPLIT"))
-        if (pl->n_rt <= kMaxSplitTiles) pl->ks_forced = true, ks = std::max(1, std::min(atoi(env), pl->nkb));
+    static const int forced = [] {  // (an experiment: read once)
+        const char* env = getenv("LUXCUDA_QMV_KSPLIT");
+        return env ? std::max(1, atoi(env)) : 0;
+    }();
+    pl->ks_forced = forced && pl->n_rt <= kMaxSplitTiles;
+    if (pl->ks_forced) ks = std::min(forced, pl->nkb);
     if (pl->n_rt > kMaxSplitTiles) ks = 1;
     pl->ks = ks;
     pl->chunks = std::max(1, std::min(pl->n_rt, sm_count / ks));
@@ -1033,18 +1032,18 @@ static const char* stream_name(int bits, int M, int pro) {
 // 33 k-blocks 6.1/4.9 with 1 row of x, but 48 with 8 rows 6.8/7.6: the line is drawn at two.)
 static bool split_pays(const Plan& pl) { return pl.ks > 2 || (pl.ks == 2 && (pl.ks_forced || (pl.mt == 1 && pl.nkb > 64))); }
 
+// One pass over a call's shape: what takes it, and with what.
+bool plan_decode(const QmmArgs& a, int sm_count, DecodePlan* pl) {
+    pl->on_grid = make_plan(a, sm_count, &pl->s);
+    pl->split = pl->on_grid && split_pays(pl->s);
+    pl->workspace_bytes = pl->on_grid ? kCounterBytes + pl->s.scratch_bytes : 0;
+    return pl->split || plan_qmv_stream(a, sm_count, &pl->st);
+}
+
 // workspace layout: [counters: kCounterBytes][partials]; the counters must be zero before the
 // first launch and are left zero by every launch.
-cudaError_t launch_qmv_mma(const QmmArgs& a, void* workspace, int sm_count, cudaStream_t stream, const char** name,
-                           bool overlap_prev, const ShardPush* push, bool x_stable) {
-    Plan pl;
-    const bool sharded = push && push->world > 1;
-    const bool on_grid = make_plan(a, sm_count, &pl, sharded);
-    if (!sharded && (!on_grid || !split_pays(pl))) {
-        if (name) *name = stream_name(a.bits, a.M, a.pro);
-        return launch_qmv_stream(&a, 1, sm_count, stream, overlap_prev, x_stable);
-    }
-    if (!on_grid) return cudaErrorInvalidValue;
+static cudaError_t launch_split(const QmmArgs& a, const Plan& pl, void* workspace, cudaStream_t stream, const char** name,
+                                bool overlap_prev, const ShardPush* push, bool x_stable) {
     Params p;
     p.x = (const __nv_bfloat16*)a.x;
     p.wq = a.wq;
@@ -1091,6 +1090,23 @@ cudaError_t launch_qmv_mma(const QmmArgs& a, void* workspace, int sm_count, cuda
          : a.pro == 2 ? launch_t<8, 1, 2>(p, pl, stream, overlap_prev) : launch_t<8, 1, 0>(p, pl, stream, overlap_prev);
 }
 
+cudaError_t launch_decode(const QmmArgs& a, const DecodePlan& pl, void* workspace, cudaStream_t stream, const char** name,
+                          bool overlap_prev, bool x_stable) {
+    if (pl.split) return launch_split(a, pl.s, workspace, stream, name, overlap_prev, nullptr, x_stable);
+    if (name) *name = stream_name(a.bits, a.M, a.pro);
+    return launch_qmv_stream(a, pl.st, stream, overlap_prev, x_stable);
+}
+cudaError_t launch_qmv_push(const QmmArgs& a, void* workspace, int sm_count, cudaStream_t stream, const char** name,
+                            bool overlap_prev, const ShardPush& push) {
+    if (push.world <= 1) {
+        DecodePlan pl;
+        return plan_decode(a, sm_count, &pl) ? launch_decode(a, pl, workspace, stream, name, overlap_prev, false) : cudaErrorNotSupported;
+    }
+    Plan pl;
+    if (!make_plan(a, sm_count, &pl, true)) return cudaErrorInvalidValue;
+    return launch_split(a, pl, workspace, stream, name, overlap_prev, &push, false);
+}
+
 // Several matmuls of one shape in one launch (qmv_batch_kernel).  All items: the shape of items[0] but for M, with
 // M on the same side of 8; bf16; no K split for that shape.  cudaErrorNotSupported otherwise.
 template <int BITS, int MT, bool DEEP>
@@ -1114,7 +1130,7 @@ cudaError_t launch_qmv_batch(const QmmArgs* items, int n, int sm_count, cudaStre
     if (on_grid && pl.ks != 1) return cudaErrorNotSupported;
     if (!sh) {
         if (name) *name = a0.bits == 4 ? (mmax <= 8 ? "qmv_batch<4,m8>" : "qmv_batch<4,m16>") : (mmax <= 8 ? "qmv_batch<8,m8>" : "qmv_batch<8,m16>");
-        return launch_qmv_stream(items, n, sm_count, stream, false, false);
+        return launch_qmv_stream_batch(items, n, sm_count, stream);
     }
     if (!on_grid) return cudaErrorNotSupported;
     // The deep ring (see the kernel) when a CTA's tiles of a matmul still fit into one batch beside it
@@ -1213,8 +1229,10 @@ extern "C" LUX_GPU_BACKEND_EXPORT LuxBackendError lux_gpu_cuda_qmatmul_decode_no
     a.error = c->err_dev;  // (without it the first launch of a process would allocate the word that processes share)
     std::lock_guard<std::mutex> lk(c->mu);
     DeviceGuard g(c->dev->device());
-    const size_t need = qmv_mma_workspace_bytes(a, c->dev->sm_count);
-    if (need == 0) {
+    DecodePlan pl;
+    const bool taken = plan_decode(a, c->dev->sm_count, &pl);
+    const size_t need = pl.workspace_bytes;
+    if (!taken || !pl.on_grid) {
         set_last_error("qmatmul_decode_noalloc: shape not taken by the decode kernel (K must be a multiple of %d)", 1024 / bits);
         return LUX_BACKEND_ERROR_NOT_SUPPORTED;
     }
@@ -1227,7 +1245,7 @@ extern "C" LUX_GPU_BACKEND_EXPORT LuxBackendError lux_gpu_cuda_qmatmul_decode_no
     cudaError_t e = static_scratch_ptr(c->dev->device(), &scratch);
     if (e != cudaSuccess) return map_cuda_error(e, "cudaGetSymbolAddress(static scratch)");
     const char* name = "";
-    e = launch_qmv_mma(a, scratch, c->dev->sm_count, c->stream, &name, decode_may_overlap(c, a), nullptr, decode_x_stable(c, a));
+    e = launch_decode(a, pl, scratch, c->stream, &name, decode_may_overlap(c, a), decode_x_stable(c, a));
     if (e != cudaSuccess) return map_cuda_error(e, name);
     c->last_kernel = name;
     c->launches++;

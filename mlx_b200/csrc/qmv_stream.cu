@@ -143,7 +143,7 @@ struct Params {
     int k_tail;             // K is no multiple of the k-block: the last one is cut off at K
     int stages, sum_warps, stage_bytes, tile_bytes, sb_off;  // bytes of weights per tile; offset of the scales in a stage
     int xs_off, run_off, bar_off;                 // offsets in shared memory
-    int x_early, x_ld;      // see launch_qmv_mma
+    int x_early, x_ld;      // see launch_decode
     int x32;                // every row of every x starts on a 32-byte boundary (callers owe 16 bytes only)
     float eps;              // of the rms-norm prologue
     int* error;             // host-visible error word of the bounded waits
@@ -547,10 +547,7 @@ __global__ void __launch_bounds__(kThreads, 1) qmv_stream_kernel(const __grid_co
 }
 
 // ---- host side ------------------------------------------------------------------------------------------------------
-struct Plan {
-    int gshift, nkb, n_rt, grid, grid_y, nch, kbc, ts, tb, stages, stage_bytes, tile_bytes, sb_off, xs_off, run_off, bar_off;
-    size_t smem;
-};
+using Plan = QmvStreamPlan;
 
 bool make_plan(const QmmArgs& a, int mmax, int sm_count, Plan* pl) {
     if (a.x_dtype != LUX_DTYPE_BFLOAT16 || a.sb_dtype != LUX_DTYPE_BFLOAT16 || (a.bits != 4 && a.bits != 8)) return false;
@@ -672,34 +669,36 @@ cudaError_t launch_items(const QmmArgs* items, int n, int mmax, const Plan& pl, 
 
 }  // namespace
 
-bool qmv_stream_supported(const QmmArgs& a, int sm_count) {
-    Plan pl;
-    if (!make_plan(a, std::min(a.M, kItemRows), sm_count, &pl)) return false;
-    // the rms-norm prologue needs the whole of x in the first fragments of the CTA's warps
-    return !a.pro || (a.M <= 8 && (a.pro == 2 || pl.nch == 1));
+bool plan_qmv_stream(const QmmArgs& a, int sm_count, QmvStreamPlan* pl) {
+    if (!make_plan(a, std::min(a.M, kItemRows), sm_count, pl)) return false;
+    if (a.M > kItemRows) pl->grid_y = std::min((a.M + kItemRows - 1) / kItemRows, sm_count / pl->grid);
+    return true;
 }
 
 int qmv_batch_max() { return kMaxBatch; }
 
-cudaError_t launch_qmv_stream(const QmmArgs* items, int n, int sm_count, cudaStream_t stream, bool overlap_prev, bool x_stable) {
+cudaError_t launch_qmv_stream(const QmmArgs& a, const QmvStreamPlan& pl, cudaStream_t stream, bool overlap_prev, bool x_stable) {
+    // the rms-norm prologue needs the whole of x in the first fragments of the CTA's warps
+    if (a.pro && (a.M > 8 || (a.pro == 1 && pl.nch != 1))) return cudaErrorNotSupported;
+    return a.M > kItemRows ? launch_items<0>(&a, 1, a.M, pl, stream, overlap_prev, x_stable)
+                           : launch_items<1>(&a, 1, a.M, pl, stream, overlap_prev, x_stable);
+}
+
+cudaError_t launch_qmv_stream_batch(const QmmArgs* items, int n, int sm_count, cudaStream_t stream) {
     if (n < 1 || n > kMaxBatch) return cudaErrorInvalidValue;
     const QmmArgs& a0 = items[0];
     int mmax = 0;
     for (int i = 0; i < n; i++) {
         const QmmArgs& a = items[i];
         mmax = std::max(mmax, a.M);
-        if (a.K != a0.K || a.N != a0.N || a.bits != a0.bits || a.group != a0.group || a.y_dtype != a0.y_dtype || a.M < 1 ||
-            (n > 1 && (a.pro || a.x_dtype != LUX_DTYPE_BFLOAT16 || a.sb_dtype != LUX_DTYPE_BFLOAT16)))
+        if (a.K != a0.K || a.N != a0.N || a.bits != a0.bits || a.group != a0.group || a.y_dtype != a0.y_dtype || a.M < 1 || a.pro ||
+            a.x_dtype != LUX_DTYPE_BFLOAT16 || a.sb_dtype != LUX_DTYPE_BFLOAT16)
             return cudaErrorNotSupported;
         if (((uintptr_t)a.wq | (uintptr_t)a.x | (uintptr_t)a.scales | (uintptr_t)a.biases) & 15) return cudaErrorInvalidValue;
     }
     Plan pl;
-    if ((n > 1 && mmax > kItemRows) || !make_plan(a0, std::min(mmax, kItemRows), sm_count, &pl)) return cudaErrorNotSupported;
-    if (mmax > kItemRows) pl.grid_y = std::min((a0.M + kItemRows - 1) / kItemRows, sm_count / pl.grid);
-    if (a0.pro && (mmax > 8 || (a0.pro == 1 && pl.nch != 1))) return cudaErrorNotSupported;
-    return mmax > kItemRows ? launch_items<0>(items, n, mmax, pl, stream, overlap_prev, x_stable)
-         : n == 1           ? launch_items<1>(items, n, mmax, pl, stream, overlap_prev, x_stable)
-                            : launch_items<kMaxBatch>(items, n, mmax, pl, stream, overlap_prev, x_stable);
+    if (mmax > kItemRows || !make_plan(a0, mmax, sm_count, &pl)) return cudaErrorNotSupported;
+    return n == 1 ? launch_items<1>(items, n, mmax, pl, stream, false, false) : launch_items<kMaxBatch>(items, n, mmax, pl, stream, false, false);
 }
 
 }  // namespace luxcuda

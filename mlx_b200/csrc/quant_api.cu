@@ -132,12 +132,12 @@ LuxBackendError qmatmul_on_stream(Context* c, const QmmArgs& a) {
             LuxBackendError le = ensure_qmm_workspace(c);
             if (le != LUX_BACKEND_OK) return le;
             e = launch_qmm_tc(a, c->qmm_ws->ptr, c->dev->sm_count, c->stream, &name);
-        } else if (qmv_mma_supported(a, c->dev->sm_count) || qmv_stream_supported(a, c->dev->sm_count)) {
-            LuxBackendError le = ensure_qmv_workspace(c, qmv_mma_workspace_bytes(a, c->dev->sm_count));
+        } else if (DecodePlan pl; plan_decode(a, c->dev->sm_count, &pl)) {
+            LuxBackendError le = ensure_qmv_workspace(c, pl.workspace_bytes);
             if (le != LUX_BACKEND_OK) return le;
             launches = 0;
             overlaps = decode_may_overlap(c, a);
-            e = launch_qmv_mma(a, c->qmv_ws ? c->qmv_ws->ptr : nullptr, c->dev->sm_count, c->stream, &name, overlaps, nullptr, decode_x_stable(c, a));
+            e = launch_decode(a, pl, c->qmv_ws ? c->qmv_ws->ptr : nullptr, c->stream, &name, overlaps, decode_x_stable(c, a));
             if (e == cudaSuccess) {
                 c->launches++;
                 note_decode_launch(c, a);
@@ -343,15 +343,16 @@ LuxBackendError qmatmul_pro(LuxBackendContext* ctx, LuxBackendBuffer* x, LuxBack
     a.error = c->err_dev;
     a.x_ld = (int)x_ld;
     a.eps = eps;
-    if (M > 8 || !qmv_mma_supported(a, c->dev->sm_count)) {
+    DecodePlan pl;
+    if (M > 8 || !plan_decode(a, c->dev->sm_count, &pl) || !pl.on_grid) {
         set_last_error("qmatmul_pro: shape not taken by the decode kernel with a prologue (M <= 8, K as qmatmul's decode path)");
         return LUX_BACKEND_ERROR_NOT_SUPPORTED;
     }
-    LuxBackendError le = ensure_qmv_workspace(c, qmv_mma_workspace_bytes(a, c->dev->sm_count));
+    LuxBackendError le = ensure_qmv_workspace(c, pl.workspace_bytes);
     if (le != LUX_BACKEND_OK) return le;
     const char* name = "";
     // (x is the output of the launch before: never read ahead of the wait for it)
-    cudaError_t e = launch_qmv_mma(a, c->qmv_ws->ptr, c->dev->sm_count, c->stream, &name, decode_may_overlap(c, a), nullptr, false);
+    cudaError_t e = launch_decode(a, pl, c->qmv_ws->ptr, c->stream, &name, decode_may_overlap(c, a), false);
     if (e == cudaErrorNotSupported) {
         cudaGetLastError();
         set_last_error("qmatmul_pro: the rms-norm prologue needs K within 16 k-blocks of 128 packed bytes and no K split");

@@ -205,7 +205,7 @@ LuxBackendError push_decode_at(LuxCudaSymmBuffer* sb, const QmmArgs& a, size_t y
     QmmArgs whole = local;  // what the launch writes, for the chain bookkeeping: every column of the local copy
     whole.N = sp.ld;
     const char* name = "";
-    cudaError_t e = launch_qmv_mma(local, c->qmv_ws->ptr, c->dev->sm_count, c->stream, &name, decode_may_overlap(c, local), &sp);
+    cudaError_t e = launch_qmv_push(local, c->qmv_ws->ptr, c->dev->sm_count, c->stream, &name, decode_may_overlap(c, local), sp);
     if (e == cudaErrorNotSupported && a.pro) {
         cudaGetLastError();
         set_last_error("qmatmul_sharded_push_pro: the prologue needs M <= 8, no K split, and for the rms-norm K within 16 k-blocks of 128 packed bytes");
