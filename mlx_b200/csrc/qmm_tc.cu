@@ -220,10 +220,7 @@ struct GemmParams {
 // (c+1 .. the owner of the tile's last stage) in its epilogue and writes y.  Those partials are produced
 // either at the start of the neighbour's range or, when a range is shorter than a tile, at the same time
 // as the head: the head's wait for them is short, and bounded.
-template <bool SK>
-struct SegIter;
-template <>
-struct SegIter<true> {  // stream-K: the CTA's range of units, segment by segment
+struct SegIter {  // stream-K: the CTA's range of units, segment by segment
     long long u, u_hi;
     int nst;
     __device__ __forceinline__ void init(long long total_units, int nst_) {
@@ -488,7 +485,7 @@ __device__ __forceinline__ void dequant_role(const GemmParams& p, Seg seg, int g
     }
 }
 
-template <int BITS, bool SK>
+template <int BITS>
 __global__ void __launch_bounds__(kNumThreads, 1)
 qmm_tc_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ CUtensorMap tmap_w,
               const __grid_constant__ GemmParams p) {
@@ -535,7 +532,7 @@ qmm_tc_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant_
             asm volatile("prefetch.tensormap [%0];" ::"l"(&tmap_w) : "memory");
             uint32_t it = 0;
             bool ok = true;
-            SegIter<SK> seg;
+            SegIter seg;
             for (seg.init(total_units, nst); seg.valid() && ok; seg.next()) {
                 const int tile = seg.tile(), s_hi = seg.s_hi();
                 const int m0 = (tile % p.m_tiles) * p.bm;
@@ -560,7 +557,7 @@ qmm_tc_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant_
             uint32_t tile_i = 0, slot = 0, phase = 0;
             const uint64_t db0 = umma_desc_sw128(s32(sB));
             bool ok = true;
-            SegIter<SK> seg;
+            SegIter seg;
             for (seg.init(total_units, nst); seg.valid() && ok; seg.next(), tile_i++) {
                 const int s_lo = seg.s_lo(), s_hi = seg.s_hi();
                 if (!mbar_wait_warp(&sl->tmem_empty, (tile_i & 1) ^ 1, abort_flag)) break;
@@ -590,13 +587,13 @@ qmm_tc_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant_
         }
     } else if (warp == kWWarp) {
         // ---------------- TMA producer: packed weights ----------------
-        SegIter<SK> seg;
+        SegIter seg;
         seg.init(total_units, nst);
         if (lane == 0) weight_producer<BITS>(p, &tmap_w, seg, nks, sW, sl->wfull, sl->wempty, abort_flag, [&](int tile) { return (tile / p.m_tiles) * kTileN; });
     } else if (warp >= kEpiWarps) {
         // ---------------- dequantisers ----------------
         const int q = warp & 3, grp = (warp - kEpiWarps) >> 2;
-        SegIter<SK> seg;
+        SegIter seg;
         seg.init(total_units, nst);
         dequant_role<BITS>(p, seg, grp, q * 32 + lane, nks, sW + (size_t)grp * p.w_slots * kWUnitBytes, &sl->wfull[grp * kMaxWSlots],
                            &sl->wempty[grp * kMaxWSlots], &sl->empty[grp],
@@ -611,7 +608,7 @@ qmm_tc_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant_
         constexpr int kEpiBar = 1 + kDqGroups;    // named barrier of the epilogue warps
         uint32_t tile_i = 0;
         bool ok = true;
-        SegIter<SK> seg;
+        SegIter seg;
         for (seg.init(total_units, nst); seg.valid() && ok; seg.next(), tile_i++) {
             const int tile = seg.tile(), s_lo = seg.s_lo(), s_hi = seg.s_hi();
             const int n = (tile / p.m_tiles) * kTileN + nl;
@@ -672,34 +669,31 @@ qmm_tc_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant_
                 unsigned char* stg = sEpi + (size_t)warp * kEpiStageBytes;
                 const int ncol0 = (tile / p.m_tiles) * kTileN + q * 32 + (lane & 3) * 8;  // first of this thread's 8 columns on the way out
                 auto store_rows = [&](const uint32_t* v, int c0, int cnt) {
-                    if (y_vec) {
-                        {
-                            constexpr int h = 0;  // (callers on this path pass sixteen rows)
-                            __syncwarp();  // the previous sixteen rows have been read
+                    if (y_vec) {  // (callers on this path pass sixteen rows)
+                        __syncwarp();  // the previous sixteen rows have been read
 #pragma unroll
-                            for (int j = 0; j < 16; j += 2) {
-                                const __nv_bfloat162 pr = __floats2bfloat162_rn(__uint_as_float(v[h + j]), __uint_as_float(v[h + j + 1]));
-                                *reinterpret_cast<__nv_bfloat16*>(stg + j * 64 + lane * 2) = pr.x;
-                                *reinterpret_cast<__nv_bfloat16*>(stg + (j + 1) * 64 + lane * 2) = pr.y;
-                            }
-                            __syncwarp();
+                        for (int j = 0; j < 16; j += 2) {
+                            const __nv_bfloat162 pr = __floats2bfloat162_rn(__uint_as_float(v[j]), __uint_as_float(v[j + 1]));
+                            *reinterpret_cast<__nv_bfloat16*>(stg + j * 64 + lane * 2) = pr.x;
+                            *reinterpret_cast<__nv_bfloat16*>(stg + (j + 1) * 64 + lane * 2) = pr.y;
+                        }
+                        __syncwarp();
 #pragma unroll
-                            for (int i = 0; i < 2; i++) {
-                                const int row = i * 8 + (lane >> 2), m = c0 + h + row;
-                                const uint4 val = *reinterpret_cast<const uint4*>(stg + row * 64 + (lane & 3) * 16);
-                                if (m >= m_end || ncol0 >= p.N) continue;
-                                const size_t idx = (size_t)(m0 + m) * p.ld + p.col0 + ncol0;
-                                if (ncol0 + 8 <= p.N) {
-                                    for (int dst = 0; dst < p.world; dst++)
-                                        *reinterpret_cast<uint4*>(reinterpret_cast<__nv_bfloat16*>(p.y_all[dst]) + idx) = val;
-                                } else {  // the last columns of y: one by one
-                                    const uint32_t w4[4] = {val.x, val.y, val.z, val.w};
-                                    for (int dst = 0; dst < p.world; dst++) {
-                                        uint16_t* yp = reinterpret_cast<uint16_t*>(p.y_all[dst]) + idx;
+                        for (int i = 0; i < 2; i++) {
+                            const int row = i * 8 + (lane >> 2), m = c0 + row;
+                            const uint4 val = *reinterpret_cast<const uint4*>(stg + row * 64 + (lane & 3) * 16);
+                            if (m >= m_end || ncol0 >= p.N) continue;
+                            const size_t idx = (size_t)(m0 + m) * p.ld + p.col0 + ncol0;
+                            if (ncol0 + 8 <= p.N) {
+                                for (int dst = 0; dst < p.world; dst++)
+                                    *reinterpret_cast<uint4*>(reinterpret_cast<__nv_bfloat16*>(p.y_all[dst]) + idx) = val;
+                            } else {  // the last columns of y: one by one
+                                const uint32_t w4[4] = {val.x, val.y, val.z, val.w};
+                                for (int dst = 0; dst < p.world; dst++) {
+                                    uint16_t* yp = reinterpret_cast<uint16_t*>(p.y_all[dst]) + idx;
 #pragma unroll
-                                        for (int e = 0; e < 8; e++)
-                                            if (ncol0 + e < p.N) yp[e] = (uint16_t)(w4[e >> 1] >> ((e & 1) * 16));
-                                    }
+                                    for (int e = 0; e < 8; e++)
+                                        if (ncol0 + e < p.N) yp[e] = (uint16_t)(w4[e >> 1] >> ((e & 1) * 16));
                                 }
                             }
                         }
@@ -1283,9 +1277,10 @@ cudaError_t launch_gemm_pair_t(const CUtensorMap& tmap, const CUtensorMap& tmap_
     return cudaGetLastError();
 }
 
+// SK: stream-K, else whole tiles
 template <int BITS, bool SK>
 cudaError_t launch_gemm_t(const CUtensorMap& tmap, const CUtensorMap& tmap_w, const GemmParams& p, const GemmPlan& pl, int sm_count, cudaStream_t stream) {
-    auto kern = SK ? qmm_tc_kernel<BITS, true> : qmm_tc_tiles_kernel<BITS>;
+    auto kern = SK ? qmm_tc_kernel<BITS> : qmm_tc_tiles_kernel<BITS>;
     static std::atomic<bool> attr_set[64];
     if (cudaError_t e = allow_smem(kern, kGemmSmemLimit, attr_set)) return e;
     // one CTA per SM, unless the launch has fewer units of work (tiles, or k-stages under stream-K) than that

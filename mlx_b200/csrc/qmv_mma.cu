@@ -84,7 +84,6 @@ struct Params {
     int M, K, N, gshift, y_bf16;
     int nkb, n_rt;
     int chunks, ks;          // grid = chunks (tile ranges) x ks (k-block ranges)
-    int chained;             // launched as a programmatic dependent of the previous kernel
     int xs_off;              // byte offset in shared memory of the x fragments kept there (16-row variant)
     int yt_off;              // byte offset in shared memory of the tiles staged for the peers (0: not sharded)
     int tb;                  // tiles per reduction batch
@@ -536,19 +535,8 @@ __global__ void __launch_bounds__(kThreads, 1) qmv_mma_kernel(const __grid_const
                 ok = (int32_t)(ready_early - epoch) >= 0 || wait_flag(p.sp.flags[p.sp.me] + kFlagReady + tid, epoch, p.peer_wait_ns);
             peers_ready = __syncthreads_and(ok);
         }
-        // End of the batch: sum the per-k-block partials of every tile in k-block order and write y.  The
-        // common case stays in line (reads of the parameter block from a function out of line are slow).
-        if (p.ks == 1 && p.sp.world <= 1) {
-            constexpr int E = 128 * MT;
-            __syncthreads();
-            for (int ti = tid / E; ti < nt; ti += kThreads / E)
-                store_tile<MT>(p, b0 + ti, tid % E,
-                               ordered_sum<false>(reinterpret_cast<const float*>(part) + ti * nkl * E + tid % E, nkl, E, 0.0f), nullptr);
-            if (b0 + tb < rt_hi) __syncthreads();  // the partial buffer is reused by the next batch
-        } else {
-            batch_end<MT>(p, reinterpret_cast<const float*>(part), b0, nt, kb_lo, nkl, s_flags, b0 + tb < rt_hi, peers_ready, epoch,
-                          p.yt_off ? smem + p.yt_off : nullptr);
-        }
+        batch_end<MT>(p, reinterpret_cast<const float*>(part), b0, nt, kb_lo, nkl, s_flags, b0 + tb < rt_hi, peers_ready, epoch,
+                      p.yt_off ? smem + p.yt_off : nullptr);
     }
     cp_async_wait<0>();
     if (p.sp.world > 1) {
@@ -1057,7 +1045,6 @@ static cudaError_t launch_split(const QmmArgs& a, const Plan& pl, void* workspac
     p.y_bf16 = a.y_dtype == LUX_DTYPE_BFLOAT16;
     p.nkb = pl.nkb; p.n_rt = pl.n_rt;
     p.chunks = pl.chunks; p.ks = pl.ks; p.tb = pl.tb; p.sb_bytes = pl.sb_bytes;
-    p.chained = overlap_prev ? 1 : 0;
     p.xs_off = pl.xs_off;
     p.yt_off = pl.yt_off;
     p.ld = a.N; p.col0 = 0;
