@@ -25,10 +25,10 @@ pytestmark = pytest.mark.gpu
 SHAPES = [
     # M, K, N, bits, group
     (1, 4096, 11008, 4, 64),    # the benchmark's decode layer: counters only
-    (8, 8192, 64, 4, 64),       # few rows, long K: K is split, partials travel through the scratch
-    (16, 4096, 96, 8, 128),     # 8-bit, split
+    (8, 8192, 64, 4, 64),       # few rows, long K: K may be split in two, the scratch is asked for
+    (16, 4096, 96, 8, 128),     # 8-bit, the same
     (3, 1024, 100, 4, 32),
-    (8, 16384, 64, 4, 64),      # split in four
+    (8, 16384, 64, 4, 64),      # split in four, partials travel through the scratch
 ]
 
 
